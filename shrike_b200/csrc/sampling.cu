@@ -10,6 +10,8 @@
 //   g_i = -log(-log(u_i)) and u_i a hash of (seed, i): the same seed gives the same
 //   token whatever else is in the batch (the reference's torch.multinomial on the
 //   global generator, sampler.py:29, does not have that property).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 constexpr int SAMPLE_THREADS = 1024;
@@ -107,8 +109,8 @@ sample_slices_kernel(const float* __restrict__ logits, const float* __restrict__
   }
 }
 
-// Stage 2: one block per row.  Rows handled by stage 1 only pick the best slice result;
-// rows with top_p < 1 run the whole nucleus procedure here.
+// Stage 2 for vocabularies whose rows do not fit a cluster's shared memory (above some 400,000 tokens): one block per row,
+// the row read from memory at every step of the bisection.
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
               const float* __restrict__ top_p, const long long* __restrict__ seeds, int* __restrict__ out,
@@ -168,11 +170,190 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
   if (threadIdx.x == 0) out[row] = valid_token(top.index, vocab, status);
 }
 
+// Stage 2: a cluster of eight CTAs per row.  Rows handled by stage 1 only pick the best slice result (the first CTA
+// does); rows with top_p < 1 run the whole nucleus procedure here.
+//
+// The procedure is a bisection of some thirty steps, each a sum over the row, so the row's probabilities stay in the
+// cluster's shared memory, and two steps cost a scan of a thread's own entries and one cluster barrier.  An entry at or below
+// the bisection's lower end can never count again and is dropped from its thread's list, in place, now and then.  The sums are those of one block of 1,024 threads that walk the row with a
+// stride of 1,024, to the bit: thread t of CTA r is that block's thread 128 r + t, dropped entries add nothing, and the 32
+// warps' sums meet in one warp in the same order.
+// Measured (one B200): 64 rows of 152,064 logits with top_p 0.95: 221 us, and 1,391 with a block a row that reads the row
+// from memory thirty times.
+constexpr int ROW_CTAS = 8, ROW_THREADS = SAMPLE_THREADS / ROW_CTAS;
+
+struct RowShare {
+  float warps[2][4][32];   // up to four values per warp of the cluster, two buffers: one barrier a sum
+  Best best[ROW_CTAS];
+};
+
+__device__ __forceinline__ void row_publish(float4 mine, RowShare& share, int buffer, cooperative_groups::cluster_group& cluster) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane < ROW_CTAS) {
+    RowShare* to = cluster.map_shared_rank(&share, lane);
+    const int at = cluster.block_rank() * (ROW_THREADS / 32) + warp;
+    to->warps[buffer][0][at] = mine.x;
+    to->warps[buffer][1][at] = mine.y;
+    to->warps[buffer][2][at] = mine.z;
+    to->warps[buffer][3][at] = mine.w;
+  }
+  cluster.sync();
+}
+
+__global__ void __launch_bounds__(ROW_THREADS)
+sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
+                      const float* __restrict__ top_p, const long long* __restrict__ seeds, int* __restrict__ out,
+                      const float* __restrict__ partial_value, const int* __restrict__ partial_index, int vocab,
+                      int chunks, int* __restrict__ status) {
+  extern __shared__ float held[];   // [entries of a thread][ROW_THREADS]
+  __shared__ RowShare share;
+  __shared__ Best best_scratch[33];
+  let_dependents_start();
+  wait_for_previous();
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int row = blockIdx.x / ROW_CTAS, rank = blockIdx.x % ROW_CTAS, lane = threadIdx.x & 31;
+  const float temp = temperature[row];
+  const float nucleus = top_p[row];
+  if (temp == 0.f || nucleus >= 1.0f) {
+    if (rank != 0) return;
+    Best mine{-INFINITY, 0x7fffffff};
+    for (int i = threadIdx.x; i < chunks; i += ROW_THREADS)
+      mine = better(mine, Best{partial_value[static_cast<size_t>(row) * chunks + i],
+                               partial_index[static_cast<size_t>(row) * chunks + i]});
+    const Best top = block_best(mine, best_scratch);
+    if (threadIdx.x == 0) out[row] = valid_token(top.index, vocab, status);
+    return;
+  }
+  cluster.sync();   // every CTA of the cluster runs: its shared memory may be written from the others
+  const float* x = logits + static_cast<size_t>(row) * vocab;
+  float* own = held + threadIdx.x;
+  const int first = rank * ROW_THREADS + threadIdx.x;
+  int count = first < vocab ? (vocab - first + SAMPLE_THREADS - 1) / SAMPLE_THREADS : 0;
+  const float inv_temp = 1.0f / temp;
+  float local_max = -INFINITY;
+#pragma unroll 8
+  for (int j = 0; j < count; ++j) {
+    const float v = x[first + j * SAMPLE_THREADS];
+    own[j * ROW_THREADS] = v;
+    local_max = fmaxf(local_max, v);
+  }
+  row_publish(make_float4(warp_max(local_max), 0.f, 0.f, 0.f), share, 0, cluster);
+  const float row_max = warp_max(share.warps[0][0][lane]);
+  float local_sum = 0.f;
+#pragma unroll 4
+  for (int j = 0; j < count; ++j) {
+    const float e = expf((own[j * ROW_THREADS] - row_max) * inv_temp);
+    own[j * ROW_THREADS] = e;
+    local_sum += e;
+  }
+  row_publish(make_float4(warp_sum(local_sum), 0.f, 0.f, 0.f), share, 1, cluster);
+  const float total = warp_sum(share.warps[1][0][lane]);
+  const float inv_total = 1.0f / total;
+#pragma unroll 4
+  for (int j = 0; j < count; ++j) own[j * ROW_THREADS] *= inv_total;
+  // Bisection on the bit pattern of a positive float: mass_above(lo) >= top_p and
+  // mass_above(hi) < top_p hold throughout; at the end no probability lies
+  // strictly between lo and hi, and the kept set is {p > lo}.
+  unsigned lo = 0u, hi = __float_as_uint(1.0f);  // mass_above(0) = 1 >= top_p; mass_above(1) = 0
+  // Two levels of it a pass: the middle and the middles of both halves, a sum each.
+  int buffer = 0, passes = 0;
+  while (hi - lo > 1u) {
+    const unsigned mid = lo + (hi - lo) / 2u, low = lo + (mid - lo) / 2u, high = mid + (hi - mid) / 2u;
+    const float cut = __uint_as_float(mid), cut_low = __uint_as_float(low), cut_high = __uint_as_float(high);
+    const float floor = __uint_as_float(lo), ceiling = __uint_as_float(hi);
+    float above = 0.f, above_low = 0.f, above_high = 0.f;
+    bool between = false;
+#pragma unroll 8
+    for (int j = 0; j < count; ++j) {
+      const float p = own[j * ROW_THREADS];
+      if (p > cut_low) above_low += p;
+      if (p > cut) above += p;
+      if (p > cut_high) above_high += p;
+      between = between || (p > floor && p < ceiling);
+    }
+    above = warp_sum(above), above_low = warp_sum(above_low), above_high = warp_sum(above_high);
+    row_publish(make_float4(above, above_low, above_high, __any_sync(0xffffffffu, between) ? 1.f : 0.f), share, buffer, cluster);
+    // no probability lies strictly between the ends: wherever between them the search ended, {p > lo} would be kept
+    if (warp_max(share.warps[buffer][3][lane]) == 0.f) break;
+    const bool upper = !(warp_sum(share.warps[buffer][0][lane]) < nucleus);
+    const bool again = !(warp_sum(share.warps[buffer][upper ? 2 : 1][lane]) < nucleus);
+    buffer ^= 1;
+    if (upper) lo = mid;
+    else hi = mid;
+    if (hi - lo > 1u) {
+      if (again) lo = upper ? high : low;
+      else hi = upper ? high : low;
+    }
+    if ((++passes & 3) == 3) {   // drop what cannot count any more; eight entries are read before the first is written
+      const float drop = __uint_as_float(lo);
+      int kept = 0;
+      for (int j = 0; j < count; j += 8) {
+        float p[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) p[e] = j + e < count ? own[(j + e) * ROW_THREADS] : 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (p[e] > drop) own[kept++ * ROW_THREADS] = p[e];
+      }
+      count = kept;
+    }
+  }
+  const float threshold = lo == 0u ? -1.f : __uint_as_float(lo);
+  Best mine{-INFINITY, 0x7fffffff};
+  const unsigned long long seed = static_cast<unsigned long long>(seeds[row]);
+  for (int i0 = first; i0 < vocab; i0 += 8 * SAMPLE_THREADS) {
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = i0 + e * SAMPLE_THREADS < vocab ? x[i0 + e * SAMPLE_THREADS] : -INFINITY;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int i = i0 + e * SAMPLE_THREADS;
+      const float p = expf((v[e] - row_max) * inv_temp) * inv_total;
+      if (i < vocab && p > threshold) mine = better(mine, Best{v[e] * inv_temp + gumbel(seed, i), i});
+    }
+  }
+  const Best top = block_best(mine, best_scratch);
+  if (threadIdx.x == 0) cluster.map_shared_rank(&share, 0)->best[rank] = top;
+  cluster.sync();
+  if (rank == 0 && threadIdx.x == 0) {
+    Best winner = share.best[0];
+    for (int r = 1; r < ROW_CTAS; ++r) winner = better(winner, share.best[r]);
+    out[row] = valid_token(winner.index, vocab, status);
+  }
+}
+
 // How many slices stage 1 cuts a row into; scratch must hold rows * slices floats and ints.
 SHRIKE_API int shrike_sample_slices(int vocab) {
   const int slices = (vocab + 2047) / 2048;
   return slices < 1 ? 1 : (slices > 128 ? 128 : slices);
 }
+
+namespace {
+// Both stages; rows that fit a cluster's shared memory take the cluster form of stage 2.
+int launch_sample(const float* logits, const float* temperature, const float* top_p, const long long* seeds, int* out,
+                  float* scratch_value, int* scratch_index, int rows, int vocab, int chunks, int* status, cudaStream_t stream) {
+  cudaError_t err = launch_dependent(sample_slices_kernel, dim3(chunks, rows), SLICE_THREADS, 0, stream, logits, temperature, top_p,
+                                     seeds, scratch_value, scratch_index, vocab, chunks);
+  if (err != cudaSuccess) return static_cast<int>(err);
+  const size_t smem = static_cast<size_t>((vocab + SAMPLE_THREADS - 1) / SAMPLE_THREADS) * ROW_THREADS * sizeof(float);
+  constexpr size_t MOST = 200 * 1024;
+  if (smem <= MOST) {
+    static bool configured = false;
+    if (!configured) {
+      err = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(MOST));
+      if (err != cudaSuccess) return static_cast<int>(err);
+      configured = true;
+    }
+    err = launch_dependent_clusters(sample_cluster_kernel, dim3(rows * ROW_CTAS), dim3(ROW_THREADS), smem, stream, ROW_CTAS, logits,
+                                    temperature, top_p, seeds, out, static_cast<const float*>(scratch_value),
+                                    static_cast<const int*>(scratch_index), vocab, chunks, status);
+  } else {
+    err = launch_dependent(sample_kernel, rows, SAMPLE_THREADS, 0, stream, logits, temperature, top_p, seeds, out,
+                           static_cast<const float*>(scratch_value), static_cast<const int*>(scratch_index), vocab, chunks, status);
+  }
+  return err == cudaSuccess ? shrike_launch_status() : static_cast<int>(err);
+}
+}  // namespace
 
 SHRIKE_API int shrike_sample(const float* logits, const float* temperature, const float* top_p,
                              const long long* seeds, int* out, float* scratch_value, int* scratch_index,
@@ -180,12 +361,7 @@ SHRIKE_API int shrike_sample(const float* logits, const float* temperature, cons
   if (rows <= 0) return SHRIKE_OK;
   if (vocab <= 0 || rows > 65535 || scratch_value == nullptr || scratch_index == nullptr) return SHRIKE_BAD_ARGUMENT;
   const int chunks = shrike_sample_slices(vocab);
-  launch_dependent(sample_slices_kernel, dim3(chunks, rows), SLICE_THREADS, 0, stream, logits, temperature, top_p, seeds,
-                   scratch_value, scratch_index, vocab, chunks);
-  launch_dependent(sample_kernel, rows, SAMPLE_THREADS, 0, stream, logits, temperature, top_p, seeds, out,
-                   static_cast<const float*>(scratch_value), static_cast<const int*>(scratch_index), vocab, chunks,
-                   status);
-  return shrike_launch_status();
+  return launch_sample(logits, temperature, top_p, seeds, out, scratch_value, scratch_index, rows, vocab, chunks, status, stream);
 }
 
 // ------------------------------------------------------------------------------------
@@ -233,11 +409,7 @@ SHRIKE_API int shrike_sample_no_alloc(const float* logits, const float* temperat
   if (status != SHRIKE_OK) return status;
   float* values = static_cast<float*>(base);
   int* indices = reinterpret_cast<int*>(static_cast<unsigned char*>(base) + SHRIKE_SAMPLE_NO_ALLOC_BYTES / 2);
-  sample_slices_kernel<<<dim3(chunks, rows), SLICE_THREADS, 0, stream>>>(logits, temperature, top_p, seeds,
-                                                                         values, indices, vocab, chunks);
-  sample_kernel<<<rows, SAMPLE_THREADS, 0, stream>>>(logits, temperature, top_p, seeds, out, values, indices,
-                                                     vocab, chunks, nullptr);
-  return shrike_launch_status();
+  return launch_sample(logits, temperature, top_p, seeds, out, values, indices, rows, vocab, chunks, nullptr, stream);
 }
 
 SHRIKE_API const char* shrike_sample_no_alloc_message(int code) {

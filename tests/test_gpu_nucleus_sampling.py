@@ -1,0 +1,40 @@
+"""Nucleus sampling over a cluster of CTAs: the token that the definition gives, at the sizes where a row is cut differently."""
+
+import math
+
+import pytest
+import torch
+
+from shrike_b200.sampling.rng import gumbel_noise_host
+from tests.gpu_common import cuda_ops
+from tests.plain import plain_model as pm
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def rnd(*shape, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+# rows of fewer entries than a cluster's threads, exactly as many, one more; a real vocabulary; more than fits a cluster
+@pytest.mark.parametrize("vocab", [1, 5, 127, 1023, 1024, 1025, 9000, 152064, 420000])
+def test_nucleus_sampling_draws_the_token_the_definition_gives(vocab):
+    ops = cuda_ops(torch.float32)
+    rows = 6
+    logits = rnd(rows, vocab, seed=vocab) * 2.0
+    temperature = [0.8, 1.0, 0.5, 2.0, 0.8, 0.0]
+    top_p = [0.95, 0.5, 0.9, 0.99, 1e-6, 0.5]
+    seeds = [11 + 1000003 * r for r in range(rows)]
+    out = torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+    ops.sample(logits, torch.tensor(temperature, device=DEV), torch.tensor(top_p, device=DEV), torch.tensor(seeds, dtype=torch.int64, device=DEV), out)
+    ops.check_status()
+    host = logits.cpu()
+    assert int(out[5]) == int(host[5].argmax())
+    for r in range(rows - 1):
+        probs = pm.softmax_with_temperature(host[r], temperature[r])
+        score = host[r].double() / temperature[r] + torch.from_numpy(gumbel_noise_host(seeds[r], vocab)).double()
+        # a float32 sum of the mass is good to about 1e-5: the kept set lies between the sets of top_p -+ that
+        sets = [pm.top_p_keep(probs, min(max(top_p[r] + d, 1e-9), 1.0)) for d in (-1e-5, 1e-5)]
+        allowed = {int(torch.where(kept, score, torch.tensor(-math.inf, dtype=torch.float64)).argmax()) for kept in sets}
+        assert int(out[r]) in allowed, (r, int(out[r]), allowed)
