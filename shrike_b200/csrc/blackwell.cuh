@@ -150,24 +150,26 @@ static inline EncodeTiled encode_tiled() {
 struct MapKey {
   const void* base;
   long long rows;
-  int cols, box_rows;
-  bool operator==(const MapKey& o) const { return base == o.base && rows == o.rows && cols == o.cols && box_rows == o.box_rows; }
+  int cols, box_rows, element;
+  bool operator==(const MapKey& o) const {
+    return base == o.base && rows == o.rows && cols == o.cols && box_rows == o.box_rows && element == o.element;
+  }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     size_t h = reinterpret_cast<size_t>(k.base);
     h = h * 1000003u ^ static_cast<size_t>(k.rows);
     h = h * 1000003u ^ static_cast<size_t>(k.cols);
-    return h * 1000003u ^ static_cast<size_t>(k.box_rows);
+    return (h * 1000003u ^ static_cast<size_t>(k.box_rows)) * 31u + static_cast<size_t>(k.element);
   }
 };
 
-// A row-major [rows, cols] bfloat16 matrix seen as boxes of box_rows x 64 elements in the
-// 128-byte swizzle; out-of-range parts of a box read as zero.  cols must be a multiple of 8.
-static inline int tensor_map_bf16(const void* base, long long rows, int cols, int box_rows, CUtensorMap* out) {
+// A row-major [rows, cols] matrix of bfloat16 or float32 seen as boxes of box_rows rows of 128 bytes in the 128-byte
+// swizzle; out-of-range parts of a box read as zero.  A row's bytes must be a multiple of 16.
+static inline int tensor_map_rows(const void* base, long long rows, int cols, int box_rows, int element, CUtensorMap* out) {
   static std::mutex mutex;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-  const MapKey key{base, rows, cols, box_rows};
+  const MapKey key{base, rows, cols, box_rows, element};
   std::lock_guard<std::mutex> guard(mutex);
   auto found = cache.find(key);
   if (found != cache.end()) {
@@ -175,20 +177,27 @@ static inline int tensor_map_bf16(const void* base, long long rows, int cols, in
     return SHRIKE_OK;
   }
   EncodeTiled encode = encode_tiled();
-  if (encode == nullptr || cols % 8 || box_rows < 1 || box_rows > 256) return SHRIKE_BAD_ARGUMENT;
+  const int bytes = element == SHRIKE_F32 ? 4 : 2;
+  if (encode == nullptr || (static_cast<long long>(cols) * bytes) % 16 || box_rows < 1 || box_rows > 256) return SHRIKE_BAD_ARGUMENT;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
-  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * bytes};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / bytes), static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t element_strides[2] = {1, 1};
   CUtensorMap map;
-  const CUresult rc = encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box,
-                             element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult rc = encode(&map, element == SHRIKE_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                             const_cast<void*>(base), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) return 1000 + static_cast<int>(rc);
   if (cache.size() > 4096) cache.clear();
   cache.emplace(key, map);
   *out = map;
   return SHRIKE_OK;
+}
+static inline int tensor_map_bf16(const void* base, long long rows, int cols, int box_rows, CUtensorMap* out) {
+  return tensor_map_rows(base, rows, cols, box_rows, SHRIKE_BF16, out);
+}
+static inline int tensor_map_f32(const void* base, long long rows, int cols, int box_rows, CUtensorMap* out) {
+  return tensor_map_rows(base, rows, cols, box_rows, SHRIKE_F32, out);
 }
 
 }  // namespace bw

@@ -156,7 +156,8 @@ class CudaOps:
         lib.shrike_silu_mul.argtypes = [_P, _P, _I, _I, _I, _I, _P]
         lib.shrike_rope_kv_write.argtypes = [_P] * 10 + [_I] * 5 + [_LL, _I, _LL, _P]
         lib.shrike_kv_write.argtypes = [_P] * 5 + [_I, _I, _I, _LL, _P]
-        lib.shrike_gemm_fp32.argtypes = [_P, _P, _P, _P, _I, _I, _I, _P]
+        lib.shrike_gemm_fp32.argtypes = [_P, _P, _P, _P, _I, _I, _I, _I, _P, _P]
+        lib.shrike_gemm_fp32_stack.argtypes = [_I, _I, _I]
         lib.shrike_sample.argtypes = [_P, _P, _P, _P, _P, _P, _P, _I, _I, _P, _P]
         lib.shrike_embed_positions.argtypes = [_P, _P, _I, _P, _I, _I, _I, _P, _I, _P, _P, _I, _P]
         lib.shrike_act_mul.argtypes = [_P, _P, _I, _I, _I, _I, _I, _P]
@@ -222,7 +223,7 @@ class CudaOps:
         lib.shrike_sample_slices.argtypes = [_I]
         lib.shrike_sample_slices.restype = _I
         for name in ("shrike_embed", "shrike_add_rmsnorm", "shrike_silu_mul", "shrike_rope_kv_write",
-                     "shrike_kv_write", "shrike_gemm_fp32", "shrike_sample", "shrike_embed_positions", "shrike_act_mul",
+                     "shrike_kv_write", "shrike_gemm_fp32", "shrike_gemm_fp32_stack", "shrike_sample", "shrike_embed_positions", "shrike_act_mul",
                      "shrike_norm_rows", "shrike_qk_norm_store", "shrike_latent_store", "shrike_head_scale"):
             getattr(lib, name).restype = _I
 
@@ -539,9 +540,14 @@ class CudaOps:
             _dense(x, torch.float32, "linear input")
             _dense(w, torch.float32, "linear weight")
             _dense(out, torch.float32, "linear output")
-            _check(self.core.shrike_gemm_fp32(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), n, o, k, self._stream()),
-                   "gemm_fp32")
-            return out
+            # K is cut into the same runs, added in the same order, whether they leave as a stack or summed
+            stack = self.core.shrike_gemm_fp32_stack(n, o, k) if allow_partials and bias is None else 1
+            if stack > 1 and (x.data_ptr() | w.data_ptr()) % 16:
+                stack = 1
+            target = self._partial_stack(out, stack) if stack > 1 else out
+            _check(self.core.shrike_gemm_fp32(_ptr(x), _ptr(w), _ptr(bias), _ptr(target), n, o, k, stack, _ptr(self.status),
+                                              self._stream()), "gemm_fp32")
+            return target
         _dense(x, torch.bfloat16, "linear input")
         _dense(w, torch.bfloat16, "linear weight")
         if self.gemm_tc is not None and n <= self.tensor_core_gemm_max_tokens and k % 8 == 0:
@@ -602,6 +608,10 @@ class CudaOps:
             15: "attention_tcgen05 (portions): shared memory was not aligned as the tiles need",
             21: "attention_bf16 (single tokens, by pages): the wait for a page's tile ran out",
             22: "attention_bf16 (single tokens, by pages): shared memory was not aligned as the tiles need",
+            41: "gemm_fp32 (few rows): the wait for a loaded stage ran out",
+            42: "gemm_fp32 (tiles): the wait for a free stage ran out",
+            43: "gemm_fp32 (tiles): the wait for a loaded stage ran out",
+            44: "gemm_fp32: copies still in flight after an aborted wait",
             31: "sampling: a row of logits had no finite element (NaN logits); token 0 was returned for it",
         }
         return roles.get(code, f"unknown status code {code}")

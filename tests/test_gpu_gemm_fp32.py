@@ -1,0 +1,46 @@
+"""The 32-bit product at the sizes where its work is cut differently: against float64, and bit for bit against the same
+row in other batches."""
+
+import math
+
+import pytest
+import torch
+
+from tests.gpu_common import cuda_ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def rnd(*shape, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+# k below and above the sizes from which it is cut into runs, ragged last runs and boxes; n around the row counts of a
+# warp, a tile, and the matrix size from which a row is one chain
+@pytest.mark.parametrize("n,k", [(7, 4), (129, 508), (130, 512), (96, 900), (1000, 4092), (257, 4100), (8, 9000), (9472, 516), (18943, 516), (18945, 516), (300, 1001)])
+def test_gemm_fp32_gives_a_row_the_same_bits_in_every_batch(n, k):
+    ops = cuda_ops(torch.float32)
+    rows = 200
+    x, w, bias = rnd(rows, k, seed=1), rnd(n, k, seed=2), rnd(n, seed=3)
+    want = x.double() @ w.double().T
+    # sums of k terms in float32: sqrt(k) u sum |a b| (Higham & Mary 2019), u = 2^-24
+    bound = math.sqrt(k) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    first = None
+    for m in (1, 2, 3, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128, 200):
+        whole = torch.empty(m, n, device=DEV)
+        ops.linear(x[:m].contiguous(), w, whole)
+        assert ((whole.double() - want[:m]).abs() <= bound[:m]).all(), m
+        first = whole[0].clone() if first is None else first
+        assert torch.equal(first, whole[0]), m
+        got = ops.linear(x[:m].contiguous(), w, torch.empty(m, n, device=DEV), allow_partials=True)
+        if got.dim() == 3:   # the consumer's sum
+            total = got[0].clone()
+            for part in got[1:]:
+                total += part
+            got = total
+        assert torch.equal(got, whole), m
+        with_bias = torch.empty(m, n, device=DEV)
+        ops.linear(x[:m].contiguous(), w, with_bias, bias=bias, allow_partials=True)
+        assert torch.equal(with_bias, whole + bias), m
+    ops.check_status()
