@@ -11,8 +11,9 @@
 // Two optional changes to a score s = scale * q.k, in this order: a soft cap, s <- cap * tanh(s / cap)
 // (softcap > 0), and a distance bias, s <- s - slopes[head] * (p - j) for key j (slopes != null).
 //
-// Built once per head size: -DSHRIKE_HEAD_DIM=<multiple of 16, at most 1024>.  Head sizes above 256 (a wide
-// cached latent) have this kernel alone, in bfloat16 too.
+// Built once per head size: -DSHRIKE_HEAD_DIM=<multiple of 16, at most 1024>.  It serves head sizes above 256 (a wide
+// cached latent), in float32 and in bfloat16; narrower heads have attention_fp32.cu, attention_bf16.cu and
+// attention_tcgen05.cu.
 #include "common.cuh"
 
 #ifndef SHRIKE_HEAD_DIM
@@ -183,27 +184,4 @@ SHRIKE_API int shrike_paged_attention_generic_kept(const void* q, const void* k_
   else return SHRIKE_BAD_ARGUMENT;
 #undef SHRIKE_ATTN_CASE
   return shrike_launch_status();
-}
-
-SHRIKE_API int shrike_paged_attention_generic_sinks(const void* q, const void* k_cache, const void* v_cache,
-                                                    const int* block_table, int max_blocks, const int* q_start,
-                                                    const int* ctx_len, const int* seq_of_token, int dtype,
-                                                    int num_tokens, int num_heads, int num_kv_heads,
-                                                    int page_size, int num_pages, float scale, int window,
-                                                    float softcap, const float* slopes, const float* sinks, void* out,
-                                                    cudaStream_t stream) {
-  return shrike_paged_attention_generic_kept(q, k_cache, v_cache, block_table, max_blocks, q_start, ctx_len, seq_of_token,
-                                             dtype, num_tokens, num_heads, num_kv_heads, page_size, num_pages, scale, window,
-                                             softcap, slopes, sinks, 0, out, stream);
-}
-
-SHRIKE_API int shrike_paged_attention_generic(const void* q, const void* k_cache, const void* v_cache,
-                                              const int* block_table, int max_blocks, const int* q_start,
-                                              const int* ctx_len, const int* seq_of_token, int dtype,
-                                              int num_tokens, int num_heads, int num_kv_heads,
-                                              int page_size, int num_pages, float scale, int window,
-                                              float softcap, const float* slopes, void* out, cudaStream_t stream) {
-  return shrike_paged_attention_generic_sinks(q, k_cache, v_cache, block_table, max_blocks, q_start, ctx_len, seq_of_token,
-                                              dtype, num_tokens, num_heads, num_kv_heads, page_size, num_pages, scale, window,
-                                              softcap, slopes, nullptr, out, stream);
 }

@@ -164,14 +164,14 @@ def load_library(name: str, sources, defines=None, extra_flags=()) -> ctypes.CDL
 
 # The libraries of this package.
 CORE_SOURCES = ["elementwise.cu", "branch_ops.cu", "parallel_ops.cu", "decay_ops.cu", "stream_ops.cu", "delta_ops.cu", "gemm_fp32.cu", "sampling.cu"]
-ATTENTION_SOURCES = ["attention_generic.cu", "attention_bf16.cu", "attention_tcgen05.cu"]
+ATTENTION_SOURCES = ["attention_fp32.cu", "attention_bf16.cu", "attention_tcgen05.cu"]
 
 
 def core_library() -> ctypes.CDLL:
     return load_library("shrike_core", CORE_SOURCES)
 
 
-TENSOR_CORE_HEAD_DIM = 256   # the widest head the mma.sync and tcgen05 attention kernels are built for
+TENSOR_CORE_HEAD_DIM = 256   # the widest head that the tiled attention kernels are built for
 
 
 def attention_library(head_dim: int) -> ctypes.CDLL:

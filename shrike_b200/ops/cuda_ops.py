@@ -232,18 +232,17 @@ class CudaOps:
         if lib is None:
             self.check_head_dim(head_dim)
             lib = build.attention_library(head_dim)
-            lib.shrike_paged_attention_generic.argtypes = (
-                [_P, _P, _P, _P, _I, _P, _P, _P] + [_I] * 6 + [_F, _I, _F, _P, _P, _P]
-            )
-            lib.shrike_paged_attention_generic.restype = _I
-            lib.shrike_paged_attention_generic_sinks.argtypes = (
-                [_P, _P, _P, _P, _I, _P, _P, _P] + [_I] * 6 + [_F, _I, _F, _P, _P, _P, _P]
-            )
-            lib.shrike_paged_attention_generic_sinks.restype = _I
-            lib.shrike_paged_attention_generic_kept.argtypes = (
-                [_P, _P, _P, _P, _I, _P, _P, _P] + [_I] * 6 + [_F, _I, _F, _P, _P, _I, _P, _P]
-            )
-            lib.shrike_paged_attention_generic_kept.restype = _I
+            if head_dim > build.TENSOR_CORE_HEAD_DIM:
+                lib.shrike_paged_attention_generic_kept.argtypes = (
+                    [_P, _P, _P, _P, _I, _P, _P, _P] + [_I] * 6 + [_F, _I, _F, _P, _P, _I, _P, _P]
+                )
+                lib.shrike_paged_attention_generic_kept.restype = _I
+            else:
+                lib.shrike_paged_attention_fp32.argtypes = (
+                    [_P, _P, _P, _P, _I, _P, _P, _P] + [_I] * 6 + [_F, _I, _F, _P, _P] + [_I] * 4 + [_P, _P, _P]
+                )
+                lib.shrike_paged_attention_fp32.restype = _I
+                lib.shrike_attention_fp32_chunk.restype = _I
             if head_dim <= build.TENSOR_CORE_HEAD_DIM:
                 self._declare_tensor_core_attention(lib)
             self._attention[head_dim] = lib
@@ -691,13 +690,24 @@ class CudaOps:
                 raise KernelError("attention takes a window or a chunk, not both")
             window = -int(chunk)   # the kernels' one number: > 0 a window, < 0 runs of that many positions
         keep_first = int(keep_first) if window and window > 0 else 0
-        if self.dtype == torch.float32 or head_dim > build.TENSOR_CORE_HEAD_DIM:
+        if head_dim > build.TENSOR_CORE_HEAD_DIM:
             self.launches += 1
             _check(lib.shrike_paged_attention_generic_kept(
                 _ptr(q), _ptr(keys), _ptr(values), _ptr(block_table), max_blocks, _ptr(q_start),
                 _ptr(ctx_len), _ptr(seq_of_token), self.code, q.shape[0], num_heads, num_kv_heads,
                 page_size, num_pages, scale, window or 0, softcap or 0.0, _ptr(slopes), _ptr(sinks), keep_first, _ptr(out),
                 self._stream()), "paged_attention")
+            return
+        if self.dtype == torch.float32:
+            has_single = max_q_len == 1 or (max_q_len > 1 and min_q_len == 1)
+            has_portions = max_q_len != 1   # lengths that are not known among them: that kernel takes entries of any length
+            chunks, scratch = self.fp32_chunks(lib, num_seqs, num_heads, num_kv_heads, head_dim, max_blocks * page_size) if has_single else (1, None)
+            self.launches += has_portions + has_single + (chunks > 1)
+            _check(lib.shrike_paged_attention_fp32(
+                _ptr(q), _ptr(keys), _ptr(values), _ptr(block_table), max_blocks, _ptr(q_start), _ptr(ctx_len), _ptr(seq_of_token),
+                q.shape[0], num_seqs, num_heads, num_kv_heads, page_size, num_pages, scale, window or 0, softcap or 0.0,
+                _ptr(slopes), _ptr(sinks), keep_first, has_single, has_portions, chunks, _ptr(scratch), _ptr(out),
+                self._stream()), "paged_attention_fp32")
             return
         if slopes is not None:
             _dense(slopes, torch.float32, "distance slopes")
@@ -723,6 +733,23 @@ class CudaOps:
             plan.has_single, has_portions, max_q_len, plan.splits, plan.cluster, _ptr(plan.scratch), _ptr(plan.arrivals),
             _ptr(self.status), softcap or 0.0, _ptr(slopes), _ptr(sinks), keep_first, self._stream()),
             "paged_attention_bf16")
+
+    FP32_SCRATCH_FLOATS = 64 << 20   # at most 256 MiB of partial rows for the 32-bit path's single tokens
+
+    def fp32_chunks(self, lib, num_seqs, num_heads, num_kv_heads, head_dim, keys):
+        """(chunks of keys that run on CTAs of their own, their scratch) for single tokens in float32: all of them where
+        the kv heads of the batch alone would leave SMs idle, else one CTA walks a row's chunks itself; the bits are the
+        same.  `keys`: what the block tables can hold."""
+        chunks = -(-keys // lib.shrike_attention_fp32_chunk())
+        need = num_seqs * num_heads * chunks * (head_dim + 2)
+        if num_seqs * num_kv_heads >= 4 * 148 or need > self.FP32_SCRATCH_FLOATS:
+            chunks = 1
+        if chunks == 1:
+            return 1, None
+        if self._scratch is None or self._scratch.numel() < need:
+            self._scratch = torch.empty(max(need, 1 << 20), dtype=torch.float32, device=self.device)
+            self.generation += 1
+        return chunks, self._scratch
 
     def portion_tiles(self, q_lens, skip_single, rows) -> int:
         """Query tiles of `rows` rows that the batch's portions make; 0 when the lengths are not known."""

@@ -1,0 +1,76 @@
+"""The 32-bit path's attention: a token's bits are the same in a prompt, alone and beside a portion, and close to float64."""
+
+import numpy as np
+import pytest
+import torch
+
+from tests.gpu_common import cuda_ops
+from tests.plain import plain_model as pm
+from tests.test_gpu_kernels import paged_case
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def rnd(*shape, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+def attention(ops, case, rows, q_start, ctx_len, seq_of, table, heads, kv_heads, dim, q_lens, **options):
+    out = torch.full((rows.shape[0], heads * dim), float("nan"), device=DEV)
+    ops.paged_attention(rows, case["keys"], case["values"], table, q_start, ctx_len, seq_of, heads, kv_heads, dim, dim ** -0.5,
+                        options.pop("window", None), out, max_q_len=max(q_lens), max_ctx_len=int(ctx_len.max()), min_q_len=min(q_lens),
+                        q_lens=list(q_lens), **options)
+    return out
+
+
+# contexts around a tile of 32 and a chunk of 128 keys; shared heads below, at and above the 16 and 64 rows of a CTA
+@pytest.mark.parametrize("heads,kv_heads,dim,page", [(7, 1, 128, 16), (16, 1, 64, 16), (17, 1, 48, 5), (66, 1, 16, 8), (4, 2, 256, 16)])
+@pytest.mark.parametrize("options", [{}, {"window": 40}, {"window": 40, "keep_first": 5}, {"chunk": 48}, {"softcap": 3.0, "sinks": True}])
+def test_fp32_attention_gives_a_token_the_same_bits_in_a_prompt_and_alone(heads, kv_heads, dim, page, options):
+    ops = cuda_ops(torch.float32)
+    options = dict(options)
+    if options.pop("sinks", False):
+        options["sinks"] = rnd(heads, seed=9)
+    ctx_lens = [1, 31, 33, 127, 128, 129, 300, 517]
+    case = paged_case(torch.float32, heads, kv_heads, dim, page, ctx_lens, ctx_lens, seed=heads)
+    whole = attention(ops, case, case["q"], case["q_start"], case["ctx_len"], case["seq_of"], case["table"], heads, kv_heads, dim, ctx_lens, **options)
+    assert torch.isfinite(whole).all()
+    # the last token of every sequence alone, in a batch of single tokens (keys on CTAs of their own) and beside a portion
+    last = (case["q_start"][1:] - 1).long()
+    count = len(ctx_lens)
+    index = torch.arange(count + 1, dtype=torch.int32, device=DEV)
+    alone = attention(ops, case, case["q"][last].contiguous(), index, case["ctx_len"], index[:count], case["table"], heads, kv_heads, dim,
+                      [1] * count, **options)
+    assert torch.equal(alone, whole[last])
+    # lengths that the caller does not know: the shortest alone, or none at all; and rows that do not lie on 16 bytes
+    for known in ({"max_q_len": 1}, {}):
+        shifted = torch.empty(count * heads * dim + 1, device=DEV)
+        rows = shifted[1:].view(count, heads * dim)
+        rows.copy_(case["q"][last])
+        out = torch.empty(count * heads * dim + 1, device=DEV)[1:].view(count, heads * dim)
+        given = dict(options)
+        ops.paged_attention(rows, case["keys"], case["values"], case["table"], index, case["ctx_len"], index[:count], heads, kv_heads, dim,
+                            dim ** -0.5, given.pop("window", None), out, **known, **given)
+        assert torch.equal(out, alone)
+    rows = torch.cat([case["q"][last[:-1]], case["q"][last[-1] - 9:]]).contiguous()
+    q_lens = [1] * (count - 1) + [10]
+    starts = torch.tensor(np.cumsum([0] + q_lens), dtype=torch.int32, device=DEV)
+    seq_of = torch.repeat_interleave(torch.arange(count), torch.tensor(q_lens)).to(torch.int32).to(DEV)
+    mixed = attention(ops, case, rows, starts, case["ctx_len"], seq_of, case["table"], heads, kv_heads, dim, q_lens, **options)
+    assert torch.equal(mixed[: count - 1], whole[last[:-1]]) and torch.equal(mixed[count - 1:], whole[last[-1] - 9: last[-1] + 1])
+    if set(options) <= {"window"}:
+        want = torch.cat([pm.causal_attention(q.double().to(DEV), k.double().to(DEV), v.double().to(DEV), options.get("window"))
+                          for q, k, v in case["seqs"]]).reshape(whole.shape)
+        assert (whole.double() - want).abs().max() < 2e-5
+
+
+def test_fp32_attention_keeps_a_later_tokens_values_out():
+    ops = cuda_ops(torch.float32)
+    case = paged_case(torch.float32, 2, 1, 64, 16, [40], [40], seed=3)
+    args = (case["q_start"], case["ctx_len"], case["seq_of"], case["table"], 2, 1, 64, [40])
+    want = attention(ops, case, case["q"], *args)
+    page = int(case["table"][0, 2])
+    case["values"][page, 7] = float("inf")   # the value of position 39
+    got = attention(ops, case, case["q"], *args)
+    assert torch.equal(got[:39], want[:39]) and not torch.isfinite(got[39]).all()
