@@ -939,10 +939,20 @@ SHRIKE_API long long shrike_attention_bf16_scratch_floats(int num_seqs, int num_
 // How many single-token CTAs the GPU holds at once; the host picks
 // splits = min(tiles, this / (seqs * kv heads * row tiles)).
 SHRIKE_API int shrike_attention_bf16_resident_ctas() {
-  const size_t smem = bf16attn::SINGLE_SMEM + 1024;
-  const ShrikeDevice& device = shrike_device();
-  const int per_sm = static_cast<int>(static_cast<size_t>(device.max_smem) / smem);
-  return device.sm_count * (per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm));
+  using namespace bf16attn;
+  // by registers and shared memory alike: heads of 64 have shared memory for four CTAs an SM but registers for two (40
+  // requests of 500 tokens, 14 heads over 2: 13.2 us with the 320 CTAs that four an SM suggest, 8.0 with 240)
+  static const int per_sm = [] {
+    int found = 0;
+    const size_t smem = SINGLE_PAGES_SMEM > SINGLE_SMEM ? SINGLE_PAGES_SMEM : SINGLE_SMEM;
+    if (cudaFuncSetAttribute(single_token_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&found, single_token_kernel<true>, PAGES_THREADS, smem) != cudaSuccess || found < 1) {
+      cudaGetLastError();
+      found = 1;
+    }
+    return found > 4 ? 4 : found;
+  }();
+  return shrike_device().sm_count * per_sm;
 }
 
 // has_single / has_portions: whether the batch holds rows with q_len == 1 / q_len > 1
