@@ -48,14 +48,20 @@
 // Tensor memory is allocated BEFORE dependents are allowed to start, so that a dependent
 // kernel that also wants tensor memory cannot starve a CTA of this one it is waiting for.
 //
-// Built once per head size; serves head sizes 64 and 128 and page sizes 8, 16, 32, 64.
+// Built once per head size; serves head sizes 64, 128 and 256 and page sizes 8, 16, 32, 64.
+// Head size 256 is served where the keys are their own values (a cached latent: one plane of pages), in a form of its own:
+// one chain of 128 rows (64 + 2 x 32 + 256 columns of tensor memory), and one tile of keys that both products read, so that
+// two stages of 128 keys and the query tile fill shared memory.  A stage is free after its last PV; the 32 boxes of a tile of
+// 16-token pages are shared by the warps that bring keys and values otherwise.
+// Measured (2,048 tokens, 12 heads over one row of 256 a token): 50 us a layer, and 172 on the mma.sync kernel, which reads
+// every key fragment from shared memory for 16 rows only and is bound by that.
 #include "blackwell.cuh"
 
 #ifndef SHRIKE_HEAD_DIM
 #error "compile with -DSHRIKE_HEAD_DIM=<head size>"
 #endif
 
-#if SHRIKE_HEAD_DIM == 64 || SHRIKE_HEAD_DIM == 128
+#if SHRIKE_HEAD_DIM == 64 || SHRIKE_HEAD_DIM == 128 || SHRIKE_HEAD_DIM == 256
 #define SHRIKE_TC_ATTENTION 1
 
 namespace tcattn {
@@ -173,10 +179,12 @@ __device__ __forceinline__ void find_work(const Args& args, int work, int rows, 
 }
 
 namespace pair {
-constexpr int ROWS = 2 * BM;                  // query rows per CTA
+constexpr bool OWN_VALUES = D == 256;         // the keys are their own values: one tile for both products
+constexpr int CHAINS = OWN_VALUES ? 1 : 2;
+constexpr int ROWS = CHAINS * BM;             // query rows per CTA
 constexpr int KEYS = 128;                     // keys per step
 constexpr int PSTAGES = 2;
-constexpr int PTHREADS = 128 + 2 * 128;   // producer, two issuers, tensor-memory owner; four softmax warps per chain
+constexpr int PTHREADS = 128 + CHAINS * 128;   // producer, two issuers, tensor-memory owner; four softmax warps per chain
 constexpr int KV_TILE_HALF = KEYS * 128;      // bytes of one 64-element-wide sub-tile of a key (or value) tile
 constexpr int KV_TILE = HALVES * KV_TILE_HALF;
 constexpr int HALF_KEYS = KEYS / 2;           // keys per softmax step
@@ -191,7 +199,7 @@ struct PairShared {
   unsigned tmem_base;
   volatile int abort;
 };
-constexpr size_t PAIR_SMEM = 2 * Q_BYTES + PSTAGES * 2 * KV_TILE + sizeof(PairShared);
+constexpr size_t PAIR_SMEM = CHAINS * Q_BYTES + PSTAGES * (OWN_VALUES ? 1 : 2) * KV_TILE + sizeof(PairShared);
 
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand (probabilities, bfloat16 packed two to a column, one
 // row per lane) comes from tensor memory.
@@ -240,8 +248,8 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   const int start = args.q_start[seq];
   const int q_len = args.q_start[seq + 1] - start;
   unsigned char* q_tiles = smem_raw;                             // [2 chains][Q_BYTES]
-  unsigned char* k_tiles = q_tiles + 2 * Q_BYTES;                // [PSTAGES][KV_TILE]
-  unsigned char* v_tiles = k_tiles + PSTAGES * KV_TILE;          // [PSTAGES][KV_TILE]
+  unsigned char* k_tiles = q_tiles + CHAINS * Q_BYTES;           // [PSTAGES][KV_TILE]
+  unsigned char* v_tiles = OWN_VALUES ? k_tiles : k_tiles + PSTAGES * KV_TILE;   // [PSTAGES][KV_TILE]
   PairShared* sh = reinterpret_cast<PairShared*>(v_tiles + PSTAGES * KV_TILE);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -249,7 +257,7 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   const int pos0 = args.ctx_len[seq] - q_len;                   // position of the first new token
   const int kv_head = head / (args.num_heads / args.num_kv_heads);
   // chain c owns rows tile_start + 128 c ...; rows_c <= 0: the chain has none
-  const int rows_0 = min(BM, q_len - tile_start), rows_1 = min(BM, q_len - tile_start - BM);
+  const int rows_0 = min(BM, q_len - tile_start), rows_1 = CHAINS > 1 ? min(BM, q_len - tile_start - BM) : 0;
   const int lo = first_visible_key(pos0 + tile_start, args.window);   // first key any row sees
   const int hi_0 = pos0 + tile_start + rows_0 - 1;              // last key chain 0 sees
   const int hi_1 = rows_1 > 0 ? hi_0 + rows_1 : -1;
@@ -307,13 +315,16 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     // a box to the copy engine costs the issuing warp about 50 ns, and a tile of 16-token pages is 16
     // boxes of keys and 16 of values: one warp for both would need longer per tile than the tensor
     // pipe does.
-    const bool for_keys = warp == 0;
+    // With one tile for both products, warp 0 and warp 3 bring half of the head's groups each and warp 0 arms the barrier
+    // (bytes that land before it is armed are counted all the same: its phase waits for the arming).
+    const bool for_keys = warp == 0 || OWN_VALUES;
+    const int first_half = OWN_VALUES && warp == 3 ? HALVES / 2 : 0, end_half = OWN_VALUES && warp == 0 ? HALVES / 2 : HALVES;
     const int* table = args.block_table + static_cast<size_t>(seq) * args.max_blocks;
     const int pages_per_tile = KEYS / args.page_size;
     const int nowhere = args.num_pages * args.page_size;      // a row coordinate outside the cache: reads zeros
-    if (for_keys && lane == 0 && num_tiles > 0) {
-      mbar_expect_tx(&sh->q_full, 2 * Q_BYTES);
-      for (int c = 0; c < 2; ++c)
+    if (warp == 0 && lane == 0 && num_tiles > 0) {
+      mbar_expect_tx(&sh->q_full, CHAINS * Q_BYTES);
+      for (int c = 0; c < CHAINS; ++c)
         for (int h = 0; h < HALVES; ++h)
           tma_load_2d(q_tiles + c * Q_BYTES + h * Q_HALF, &map_q, &sh->q_full, head * D + h * 64, start + tile_start + c * BM);
     }
@@ -348,12 +359,12 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       int ok = 1;
       if (lane == 0) {
         ok = mbar_wait(&free_again[s], phase ^ 1, &sh->abort, args.status, ERR_PRODUCER) ? 1 : 0;
-        if (ok) mbar_expect_tx(&full[s], KV_TILE);
+        if (ok && (!OWN_VALUES || warp == 0)) mbar_expect_tx(&full[s], KV_TILE);
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
       if (lane < pages_per_tile)
-        for (int h = 0; h < HALVES; ++h) tma_load_2d(tile + h * KV_TILE_HALF + at, map, &full[s], kv_head * D + h * 64, y);
+        for (int h = first_half; h < end_half; ++h) tma_load_2d(tile + h * KV_TILE_HALF + at, map, &full[s], kv_head * D + h * 64, y);
       issued = i + 1;
     }
     if (lane == 0 && sh->abort) {   // copies may still be in flight: wait for the stages armed last
@@ -362,7 +373,7 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         for (unsigned tries = 0; tries < WAIT_LIMIT && !landed; ++tries) landed = mbar_try_wait(&full[i % PSTAGES], (i / PSTAGES) & 1);
         if (!landed && args.status != nullptr) *args.status = ERR_DRAIN;
       }
-      bool landed = !for_keys || num_tiles <= 0;
+      bool landed = warp != 0 || num_tiles <= 0;
       for (unsigned tries = 0; tries < WAIT_LIMIT && !landed; ++tries) landed = mbar_try_wait(&sh->q_full, 0);
     }
   } else if (warp == 1 || warp == 2) {
@@ -399,7 +410,7 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           umma(tmem_chain, q_base + (((kk / 4) * Q_HALF + (kk % 4) * 32) >> 4), k_base + (((kk / 4) * KV_TILE_HALF + (kk % 4) * 32) >> 4), idesc_s,
                kk > 0 ? 1u : 0u);
         umma_commit(&sh->s_full[c]);
-        if ((h & 1) || h + 1 == steps) umma_commit(&sh->k_free[st]);
+        if (!OWN_VALUES && ((h & 1) || h + 1 == steps)) umma_commit(&sh->k_free[st]);
       };
       // The two chains' softmax warps share the sub-partitions; started together they stay in step and
       // do their arithmetic at the same time and their waiting at the same time.  The later chain
@@ -414,7 +425,7 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           if (!ok) break;
         }
         const int i = h >> 1, st = i % PSTAGES;
-        if (values_ready < i) {
+        if (!OWN_VALUES && values_ready < i) {
           ok = mbar_wait(&sh->v_full[st], (i / PSTAGES) & 1, &sh->abort, args.status, ERR_MMA);
           values_ready = i;
         }
@@ -429,7 +440,7 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           umma_a_in_tmem(tmem_o, tmem_p + kk * 8, v_base + ((kk * 16 * 128) >> 4), idesc_o, (h > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&sh->pv_done[c][h & 1]);
         if (h + 1 == steps) umma_commit(&sh->pv_last[c]);
-        if ((h & 1) || h + 1 == steps) umma_commit(&sh->v_free[st]);
+        if ((h & 1) || h + 1 == steps) umma_commit(OWN_VALUES ? &sh->k_free[st] : &sh->v_free[st]);
       }
     }
   } else if (warp >= 4) {
@@ -540,7 +551,7 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       // any), at the tile's first step, before either of its PV
       if ((h & 1) == 0 && tile_lo + (h >> 1) == tile_hi && (hi + 1) % KEYS != 0) {
         const int s = (h >> 1) % PSTAGES;
-        ok = mbar_wait(&sh->v_full[s], ((h >> 1) / PSTAGES) & 1, &sh->abort, args.status, ERR_SOFTMAX);
+        ok = mbar_wait(OWN_VALUES ? &sh->k_full[s] : &sh->v_full[s], ((h >> 1) / PSTAGES) & 1, &sh->abort, args.status, ERR_SOFTMAX);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         zero_value_rows(v_tiles + s * KV_TILE, hi + 1 - key_base, row);
@@ -662,6 +673,8 @@ combine_portions_kernel(const Args args) {
 }  // namespace tcattn
 
 SHRIKE_API int shrike_attention_tc_available() { return 1; }
+// Whether this head size is served only where the keys are their own values.
+SHRIKE_API int shrike_attention_tc_own_values() { return tcattn::pair::OWN_VALUES ? 1 : 0; }
 
 // Query rows a CTA owns: what the caller counts the portions' query tiles in.
 SHRIKE_API int shrike_attention_tc_portions_rows() { return tcattn::pair::ROWS; }
@@ -718,6 +731,7 @@ SHRIKE_API int shrike_paged_attention_tc_portions_kept(const void* q, const void
   using namespace tcattn;
   if (num_seqs <= 0 || num_tokens <= 0) return SHRIKE_OK;
   if (keep_first < 0 || (keep_first > 0 && window > 0 && splits < 2)) return SHRIKE_BAD_ARGUMENT;
+  if (pair::OWN_VALUES && k_cache != v_cache) return SHRIKE_BAD_ARGUMENT;
   if (splits < 1 || splits > 32 || (splits > 1 && (scratch == nullptr || seq_of_token == nullptr))) return SHRIKE_BAD_ARGUMENT;
   // query tiles of the batch's portions: the caller's count, or what `num_tokens` tokens in
   // `num_seqs` sequences can make at most
@@ -820,6 +834,7 @@ SHRIKE_API int shrike_paged_attention_tc_portions(const void* q, const void* k_c
 #else  // other head sizes: the mma.sync kernel serves them
 
 SHRIKE_API int shrike_attention_tc_available() { return 0; }
+SHRIKE_API int shrike_attention_tc_own_values() { return 0; }
 SHRIKE_API int shrike_attention_tc_portions_rows() { return 128; }
 SHRIKE_API int shrike_attention_tc_portions_splits(int, int, int, int, int) { return 1; }
 SHRIKE_API long long shrike_attention_tc_portions_scratch_floats(int, int, int) { return 0; }

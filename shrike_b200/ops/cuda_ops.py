@@ -714,7 +714,7 @@ class CudaOps:
             if slopes.numel() != num_heads:
                 raise KernelError("one distance slope per query head")
         plan = self.attention_plan(num_heads, num_kv_heads, head_dim, num_seqs, max_blocks, page_size, max_q_len, min_q_len,
-                                   q.shape[0], q_lens, keep_first=keep_first)
+                                   q.shape[0], q_lens, keep_first=keep_first, own_values=keys.data_ptr() == values.data_ptr())
         self.launches += plan.has_single + plan.has_portions + (1 if plan.portion_splits > 1 else 0)
         has_portions = plan.has_portions
         if plan.tc_portions:
@@ -763,7 +763,7 @@ class CudaOps:
         return tiles
 
     def attention_plan(self, num_heads, num_kv_heads, head_dim, num_seqs, max_blocks, page_size, max_q_len, min_q_len,
-                       num_tokens=0, q_lens=None, keep_first=0):
+                       num_tokens=0, q_lens=None, keep_first=0, own_values=False):
         """How a bfloat16 batch's attention is cut: which kernels run (single tokens, portions, the
         tensor-core form of the latter), the key splits and clusters of the single-token kernel, the
         key splits of the portions kernel, and their scratch.  A function of the batch's shape alone."""
@@ -787,8 +787,11 @@ class CudaOps:
                 self._arrivals = torch.zeros(max(groups, 4096), dtype=torch.int32, device=self.device)
                 self.generation += 1
             scratch, arrivals = self._scratch, self._arrivals
-        tc_portions = bool(has_portions and self.tensor_core_attention and lib.shrike_attention_tc_available()
-                           and page_size in (8, 16, 32, 64))
+        # the tensor-core form walks long contexts several times faster, but starts slower: a prompt of 43 tokens takes 5.6 us
+        # with it and 4.4 with the mma.sync kernel (14 heads of 64), one of 100 the same with both
+        short = max_q_len <= 64 and max_blocks * page_size <= 128
+        tc_portions = bool(has_portions and self.tensor_core_attention and lib.shrike_attention_tc_available() and not short
+                           and page_size in (8, 16, 32, 64) and (own_values or not lib.shrike_attention_tc_own_values()))
         portion_splits, portion_scratch = 1, None
         if tc_portions and num_tokens > 0:
             tiles = self.portion_tiles(q_lens, has_single, lib.shrike_attention_tc_portions_rows())

@@ -1,0 +1,34 @@
+"""Portions whose keys are their own values, rows of 256, on the tcgen05 kernel: against float64."""
+
+import pytest
+import torch
+
+from tests.gpu_common import cuda_ops
+from tests.plain import plain_model as pm
+from tests.test_gpu_kernels import paged_case
+
+pytestmark = pytest.mark.gpu
+
+
+# query tiles of 128 rows and key tiles of 128 in steps of 64: lengths and contexts around both, with and without several
+# CTAs that share a tile's keys; tokens beside portions
+@pytest.mark.parametrize("heads,page,window,splits", [(3, 16, None, 0), (12, 16, None, 2), (2, 8, 100, 0), (1, 64, 300, 3), (5, 32, None, 0)])
+@pytest.mark.parametrize("ctx_lens,q_lens", [([2, 63, 64, 65], [2, 63, 64, 65]), ([127, 128, 129], [127, 128, 129]), ([257, 400, 1, 700], [256, 129, 1, 66]),
+                                             ([1000], [900])])
+def test_own_values_on_the_tensor_core_portions_kernel(heads, page, window, splits, ctx_lens, q_lens):
+    ops = cuda_ops(torch.bfloat16)
+    dim = 256
+    case = paged_case(torch.bfloat16, heads, 1, dim, page, ctx_lens, q_lens, seed=heads)
+    wide = torch.full((len(ctx_lens), max(case["table"].shape[1], 160 // page + 1)), -1, dtype=torch.int32, device="cuda")   # no short table
+    wide[:, : case["table"].shape[1]] = case["table"]
+    ops.portion_splits = splits
+    out = torch.full_like(case["q"], float("nan"))
+    plan = ops.attention_plan(heads, 1, dim, len(ctx_lens), wide.shape[1], page, max(q_lens), min(q_lens), sum(q_lens), list(q_lens), own_values=True)
+    assert plan.tc_portions, "the case is meant for the tensor-core kernel"
+    ops.paged_attention(case["q"], case["keys"], case["keys"], wide, case["q_start"], case["ctx_len"], case["seq_of"], heads, 1, dim,
+                        dim ** -0.5, window, out, max_q_len=max(q_lens), max_ctx_len=max(ctx_lens), min_q_len=min(q_lens), q_lens=list(q_lens))
+    ops.check_status()
+    want = torch.cat([pm.causal_attention(q[len(q) - n:].double().cuda(), k.double().cuda(), k.double().cuda(), window)
+                      for (q, k, _), n in zip(case["seqs"], q_lens)]).reshape(out.shape)
+    # probabilities rounded to bfloat16 (2^-9 each, relative) and one rounding of outputs of order one: as for the other heads
+    assert torch.isfinite(out).all() and (out.double() - want).abs().max() < 2e-2
