@@ -154,19 +154,15 @@ rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
   const int k_begin = segment * segment_length, k_end = min(K, k_begin + segment_length);
   const int steps = n0 < N && k_end > k_begin ? (k_end - k_begin + 31) / 32 : 0;
   unsigned char* mine = tiles + static_cast<size_t>(warp) * stages * STAGE;
-  int issued = 0;
-  if (lane == 0) {
-    const int early = min(steps, stages);
-    for (int i = 0; i < early; ++i) {   // W is written by nobody: it is on its way before the kernel before this one ends
-      mbar_expect_tx(&full[warp][i], W_BYTES + MT * 128);
-      tma_load_2d(mine + i * STAGE, &map_w, &full[warp][i], k_begin + i * 32, n0);
-    }
-    wait_for_previous();
-    for (int i = 0; i < early; ++i) tma_load_2d(mine + i * STAGE + W_BYTES, &map_a, &full[warp][i], k_begin + i * 32, 0);
-    issued = early;
-  } else {
-    wait_for_previous();
+  // neighbouring lanes hand their copies to the engine together: one thread that issues them one after another keeps a short
+  // run waiting for its last ones (2,048 x 1,536 and 1,536 x 1,536, 3 tokens: 6.7 us a product, 4.9 together)
+  int issued = min(steps, stages);
+  if (lane < issued) {   // W is written by nobody: it is on its way before the kernel before this one ends
+    mbar_expect_tx(&full[warp][lane], W_BYTES + MT * 128);
+    tma_load_2d(mine + lane * STAGE, &map_w, &full[warp][lane], k_begin + lane * 32, n0);
   }
+  wait_for_previous();
+  if (lane < issued) tma_load_2d(mine + lane * STAGE + W_BYTES, &map_a, &full[warp][lane], k_begin + lane * 32, 0);
   __syncwarp();
   const int row = lane % ROWS, group = lane / ROWS;
   float acc[RPL][OWN];
@@ -199,10 +195,12 @@ rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       }
     }
     __syncwarp();   // every lane has read the stage
-    if (lane == 0 && step + stages < steps) {
-      mbar_expect_tx(&full[warp][stage], W_BYTES + MT * 128);
-      tma_load_2d(mine + stage * STAGE, &map_w, &full[warp][stage], k_begin + (step + stages) * 32, n0);
-      tma_load_2d(mine + stage * STAGE + W_BYTES, &map_a, &full[warp][stage], k_begin + (step + stages) * 32, 0);
+    if (step + stages < steps) {
+      if (lane == 0) mbar_expect_tx(&full[warp][stage], W_BYTES + MT * 128);
+      __syncwarp();
+      if (lane < 2)
+        tma_load_2d(mine + stage * STAGE + (lane == 0 ? 0 : W_BYTES), lane == 0 ? &map_w : &map_a, &full[warp][stage],
+                    k_begin + (step + stages) * 32, lane == 0 ? n0 : 0);
       issued = step + stages + 1;
     }
     if (++stage == stages) { stage = 0; phase ^= 1; }
@@ -472,20 +470,23 @@ int segment_length(int n, int k) {
   return ((k + runs - 1) / runs + 31) / 32 * 32;
 }
 
-// Eighths of a tile's rows (TM) for a product of M rows and `stack` slices: the cheapest by what a CTA costs times the CTAs
-// an SM gets.  Two CTAs run side by side on an SM; one alone takes about 0.7 of the time of two (a warp a scheduler).
-// Fewer rows a thread read more from shared memory an FMA: measured 0.86 of the rate at TM = 8 (41 against 48 TFLOP/s on
-// the 37,888 x 3,584 matrix).  The CTAs' rows beyond M and the last round's empty places are what the choice avoids:
-// 333 rows against the 896 x 4,864 matrix are five tiles of 80 and not six of 64 (86 us against 121).
+// Eighths of a tile's rows (TM) for a product of M rows and `stack` slices: what an SM's CTAs cost, rounds of as many as
+// live on it (two; three of 48 rows, four of 32), the last round at least the cost of two where it is the only one (a CTA
+// alone hides nothing of its latencies) and of 1.25 behind others (its CTAs start as places fall free).  Smaller tiles
+// read more from shared memory an FMA.  The rows beyond M and the empty places of the last round are what the choice
+// avoids.  Measured, 333 rows: the 896 x 4,864 matrix 84 us with the chosen 80 rows a tile, 112 to 136 with 32, 64, 112 or
+// 128; 9,728 x 896: 182 with 112, 188 with 64, 208 with 96; 1,152 x 896: 28 with 32, 45 with 96.
 int tile_rows(int M, int N, int stack) {
-  constexpr int sizes[] = {16, 14, 12, 10, 8, 6, 4};
-  constexpr float rate[] = {1.f, 0.98f, 0.96f, 0.92f, 0.86f, 0.62f, 0.5f};
+  constexpr int sizes[] = {16, 14, 12, 10, 8, 6, 4}, resident[] = {2, 2, 2, 2, 2, 3, 4};
+  constexpr float rate[] = {1.f, 1.f, 1.f, 1.f, 0.95f, 0.7f, 0.75f};
   const long long sms = shrike_device().sm_count, columns = static_cast<long long>((N + TILE_N - 1) / TILE_N) * stack;
   int best = 16;
   float least = 0.f;
   for (int i = 0; i < 7; ++i) {
-    const long long ctas = columns * ((M + 8 * sizes[i] - 1) / (8 * sizes[i])), an_sm = (ctas + sms - 1) / sms;
-    const float cost = ((an_sm / 2) * 2.f + (an_sm % 2) * 1.4f) * sizes[i] / rate[i];
+    const long long ctas = columns * ((M + 8 * sizes[i] - 1) / (8 * sizes[i])), places = sms * resident[i];
+    const long long rounds = ctas / places, rest = ctas % places, an_sm = (rest + sms - 1) / sms;
+    const float alone = rounds > 0 ? 1.25f : 2.f, last = rest == 0 ? 0.f : (an_sm > alone ? an_sm : alone);
+    const float cost = (rounds * resident[i] + last) * sizes[i] / rate[i];
     if (i == 0 || cost < least) {
       least = cost;
       best = sizes[i];
