@@ -53,7 +53,7 @@
 // one chain of 128 rows (64 + 2 x 32 + 256 columns of tensor memory), and one tile of keys that both products read, so that
 // two stages of 128 keys and the query tile fill shared memory.  A stage is free after its last PV; the 32 boxes of a tile of
 // 16-token pages are shared by the warps that bring keys and values otherwise.
-// Measured (2,048 tokens, 12 heads over one row of 256 a token): 50 us a layer, and 172 on the mma.sync kernel, which reads
+// Measured (2,048 tokens, 12 heads over one row of 256 a token): 55 us a layer, and 168 on the mma.sync kernel, which reads
 // every key fragment from shared memory for 16 rows only and is bound by that.
 #include "blackwell.cuh"
 
@@ -181,6 +181,12 @@ __device__ __forceinline__ void find_work(const Args& args, int work, int rows, 
 namespace pair {
 constexpr bool OWN_VALUES = D == 256;         // the keys are their own values: one tile for both products
 constexpr int CHAINS = OWN_VALUES ? 1 : 2;
+// Softmax of the one-chain form: the base of the exponentials is the running maximum itself, and the denominator adds the
+// weights as the product takes them, rounded.  Relative error of the outputs against 64 bits (700 tokens, 12 heads; scores of
+// standard deviation 1, 2, 4, 8): 1.910, 1.794, 1.715, 1.627 x 1e-3; with a base that lags by up to 2^8 and unrounded weights in
+// the sum 1.972, 2.026, 2.045, 1.879; the mma.sync kernel 1.919, 1.799, 1.717, 1.629.
+constexpr bool EXACT_BASE = OWN_VALUES;
+constexpr float BASE_LAG = EXACT_BASE ? 0.0f : 8.0f;   // in powers of two
 constexpr int ROWS = CHAINS * BM;             // query rows per CTA
 constexpr int KEYS = 128;                     // keys per step
 constexpr int PSTAGES = 2;
@@ -511,9 +517,12 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       step_max *= scale_log2;
       // The base of the exponentials follows the running maximum lazily: it moves (and O is
       // rescaled) only when the maximum has grown by more than 2^8; until then probabilities
-      // are at most 2^8, which float32 sums and bfloat16 products hold without loss.
+      // are at most 2^8, which float32 sums and bfloat16 products hold without overflow.  A weight
+      // that is no power of two is rounded to bfloat16 in the product, though, and a lagging base makes
+      // the largest weights such: where the keys are their own values the base does not lag, so that the
+      // largest weight is 1 as in the mma.sync kernel (EXACT_BASE below).
       float correction = 1.0f;
-      if (step_max > row_max + 8.0f || row_max == -INFINITY) {
+      if (step_max > row_max + BASE_LAG || row_max == -INFINITY) {
         const float new_max = fmaxf(row_max, step_max);
         const float base = new_max == -INFINITY ? 0.f : new_max;
         // a row that has seen no key yet has O = 0 and a sum of 0: nothing to rescale
@@ -531,9 +540,14 @@ portions_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           halves_of(fma_pair(pair_of(__uint_as_float(v[g][j]), __uint_as_float(v[g][j + 1])), scale_pair, base_pair), x0, x1);
           x0 = fast_exp2(x0);
           x1 = fast_exp2(x1);
-          sum_pair[(j >> 1) & 1] = add_pair(sum_pair[(j >> 1) & 1], pair_of(x0, x1));
           const __nv_bfloat162 two = __floats2bfloat162_rn(x0, x1);
-          v[0][g * 16 + j / 2] = *reinterpret_cast<const unsigned*>(&two);   // packed over the scores already used
+          const unsigned packed = *reinterpret_cast<const unsigned*>(&two);
+          if (EXACT_BASE) {
+            x0 = __uint_as_float(packed << 16);
+            x1 = __uint_as_float(packed & 0xffff0000u);
+          }
+          sum_pair[(j >> 1) & 1] = add_pair(sum_pair[(j >> 1) & 1], pair_of(x0, x1));
+          v[0][g * 16 + j / 2] = packed;   // over the scores already used
         }
       }
       float sum_lo, sum_hi;
