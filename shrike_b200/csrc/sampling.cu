@@ -273,9 +273,13 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
     }
     above = warp_sum(above), above_low = warp_sum(above_low), above_high = warp_sum(above_high);
     row_publish(make_float4(above, above_low, above_high, __any_sync(0xffffffffu, between) ? 1.f : 0.f), share, buffer, cluster);
-    // no probability lies strictly between the ends: wherever between them the search ended, {p > lo} would be kept
-    if (warp_max(share.warps[buffer][3][lane]) == 0.f) break;
     const bool upper = !(warp_sum(share.warps[buffer][0][lane]) < nucleus);
+    // No probability lies strictly between the ends: every later middle has this one's mass above it, and the search would
+    // end just below `hi` or at `lo` (a `lo` of zero is no threshold: it keeps the tokens of probability zero too).
+    if (warp_max(share.warps[buffer][3][lane]) == 0.f) {
+      if (upper) lo = hi - 1u;
+      break;
+    }
     const bool again = !(warp_sum(share.warps[buffer][upper ? 2 : 1][lane]) < nucleus);
     buffer ^= 1;
     if (upper) lo = mid;

@@ -38,3 +38,23 @@ def test_nucleus_sampling_draws_the_token_the_definition_gives(vocab):
         sets = [pm.top_p_keep(probs, min(max(top_p[r] + d, 1e-9), 1.0)) for d in (-1e-5, 1e-5)]
         allowed = {int(torch.where(kept, score, torch.tensor(-math.inf, dtype=torch.float64)).argmax()) for kept in sets}
         assert int(out[r]) in allowed, (r, int(out[r]), allowed)
+
+
+# one token has all of the mass in 32 bits: it alone is kept, also where logits over a tiny temperature no longer tell tokens
+# apart (10 / 2e-38 is infinite); all of the mass on two equal logits; both forms of the kernel
+@pytest.mark.parametrize("vocab", [5, 1025, 152064, 420000])
+def test_nucleus_of_tokens_that_hold_all_of_the_mass(vocab):
+    ops = cuda_ops(torch.float32)
+    temperature = [2e-38, 1e-9, 1e-3, 0.5, 2e-38, 1e-9]
+    top_p = [0.5, 0.95, 0.999, 0.9, 1e-6, 0.9]
+    rows, best = len(temperature), vocab - 2
+    logits = 10.0 + rnd(rows, vocab, seed=vocab).abs().clamp(max=8.0)
+    logits[:, best] = 19.0
+    logits[3, best] = 1000.0
+    logits[5, 1] = 19.0
+    out = torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+    for seed in range(4):
+        seeds = torch.arange(rows, dtype=torch.int64, device=DEV) + 100 * seed
+        ops.sample(logits, torch.tensor(temperature, device=DEV), torch.tensor(top_p, device=DEV), seeds, out)
+        ops.check_status()
+        assert out[:5].tolist() == [best] * 5 and int(out[5]) in (1, best)
