@@ -81,7 +81,10 @@ template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16*
 //   wait_for_previous();      block until the kernel before this one has finished and its
 //                             writes are visible
 // before it reads or writes any memory that another kernel touches.  Only work on memory
-// that no kernel writes (weights) may come before wait_for_previous().
+// that no kernel writes (weights), or that the caller says no kernel still running writes (a
+// step's metadata, which a copy on the stream brings; states that only earlier steps wrote), may
+// come before wait_for_previous().  That the kernel before this one has begun says nothing about
+// the ones before it: each lets its dependents start before its own wait.
 __device__ __forceinline__ void let_dependents_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

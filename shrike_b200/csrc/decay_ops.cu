@@ -49,6 +49,7 @@ struct ScanArgs {
   int heads, dim, vdim, num_slots, state_stride;
   int slice;                // columns per CTA
   int groups;               // row groups per CTA: thread t owns column t % slice, rows t / slice + i * groups
+  int early_state;          // 1: no kernel still running writes the states: they are read before the wait
 };
 
 // Walk: grid (vdim slices, heads, seqs).  Each thread keeps ROWS elements of the state in registers.
@@ -60,12 +61,13 @@ __global__ void __launch_bounds__(THREADS) walk_kernel(ScanArgs a, int skip_long
   float* v_s = k_s + a.dim;               // [slice]
   float* part = v_s + a.slice;            // [groups][slice]
   let_dependents_start();
+  if (!a.early_state) wait_for_previous();
   const int seq = blockIdx.z, head = blockIdx.y, first_col = blockIdx.x * a.slice;
   const int slot = a.state_slot[seq];
   const int begin = a.q_start[seq], end = a.q_start[seq + 1];
   // no slot, or the chunked form serves it
   if (slot < 0 || slot >= a.num_slots || (skip_longer_than > 0 && end - begin > skip_longer_than)) {
-    wait_for_previous();
+    if (a.early_state) wait_for_previous();   // every CTA waits before it leaves
     return;
   }
   const int cols = min(a.slice, a.vdim - first_col);
@@ -73,7 +75,6 @@ __global__ void __launch_bounds__(THREADS) walk_kernel(ScanArgs a, int skip_long
   const int col = t % a.slice, group = t / a.slice;
   const bool active = group < a.groups && col < cols;
   const float d = a.decays[head];
-  // no other kernel of the step writes this state: it is read while the kernel before this one still runs
   float* mine = a.state + (static_cast<size_t>(slot) * a.heads + head) * a.state_stride;
   float held[ROWS];
 #pragma unroll
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(THREADS) walk_kernel(ScanArgs a, int skip_long
     const int row = group + i * a.groups;
     held[i] = active && row < a.dim ? mine[static_cast<size_t>(row) * a.vdim + first_col + col] : 0.f;
   }
-  wait_for_previous();
+  if (a.early_state) wait_for_previous();
   const int q_at = head * a.dim, k_at = a.heads * a.dim + head * a.dim, v_at = 2 * a.heads * a.dim + head * a.vdim + first_col;
   for (int token = begin; token < end; ++token) {
     const float* row = a.fused + static_cast<size_t>(token) * a.row_width;
@@ -719,10 +720,12 @@ SHRIKE_API int shrike_decay_scan_chunk() { return decay::CHUNK; }
 // `longest`: the most new tokens a sequence of the batch brings, `n` the batch's tokens.  With `chunk_from` > 0 and
 // `longest` >= `chunk_from`, sequences that bring at least `chunk_from` tokens run in the chunked form, for which the
 // caller holds `chunk_state` (float32, shrike_decay_scan_chunks(n, seqs) * heads * dim * vdim); the others walk.
+// `early_state` 1: the caller knows that whatever wrote the states, `q_start` and `state_slot` has finished (an earlier step or
+// copy, not merely an earlier launch), so that the walk may read them while the kernel before it runs.
 SHRIKE_API int shrike_decay_scan(const float* fused, int partials, long long partial_stride, int row_width, const float* decays,
                                  float* state, const int* q_start, const int* state_slot, float* out, int num_seqs, int heads,
                                  int dim, int vdim, int num_slots, int state_stride, int longest, int chunk_from, int n,
-                                 float* chunk_state, cudaStream_t stream) {
+                                 float* chunk_state, int early_state, cudaStream_t stream) {
   using namespace decay;
   if (num_seqs <= 0) return SHRIKE_OK;
   if (heads <= 0 || dim <= 0 || vdim <= 0 || state_stride < dim * vdim || partials < 1) return SHRIKE_BAD_ARGUMENT;
@@ -730,6 +733,7 @@ SHRIKE_API int shrike_decay_scan(const float* fused, int partials, long long par
   a.fused = fused; a.partials = partials; a.partial_stride = partial_stride; a.row_width = row_width; a.decays = decays;
   a.state = state; a.q_start = q_start; a.state_slot = state_slot; a.out = out;
   a.heads = heads; a.dim = dim; a.vdim = vdim; a.num_slots = num_slots; a.state_stride = state_stride;
+  a.early_state = early_state;
   a.slice = vdim < MAX_SLICE ? vdim : MAX_SLICE;
   a.groups = THREADS / a.slice;
   if (a.groups > dim) a.groups = dim;

@@ -175,7 +175,7 @@ class CudaOps:
         lib.shrike_act_mul_blocks.argtypes = [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P]
         lib.shrike_matrix_memory_chunks.argtypes = [_I, _I]
         lib.shrike_matrix_memory_chunks.restype = _LL
-        lib.shrike_decay_scan.argtypes = [_P, _I, _LL, _I, _P, _P, _P, _P, _P] + [_I] * 9 + [_P, _P]
+        lib.shrike_decay_scan.argtypes = [_P, _I, _LL, _I, _P, _P, _P, _P, _P] + [_I] * 9 + [_P, _I, _P]
         lib.shrike_decay_scan_chunks.argtypes = [_I, _I]
         lib.shrike_decay_scan_chunks.restype = _LL
         lib.shrike_norm_gate.argtypes = [_P, _P, _I, _LL, _I, _I, _P, _F, _P, _I, _I, _I, _P]
@@ -1023,13 +1023,16 @@ class CudaOps:
 
     DECAY_CHUNK_FROM = 32   # a sequence that brings at least this many tokens runs its decayed scan over runs of tokens
 
-    def decay_scan(self, fused, decays, state, q_start, state_slot, out, num_seqs, num_heads, dim, vdim, longest=0):
+    def decay_scan(self, fused, decays, state, q_start, state_slot, out, num_seqs, num_heads, dim, vdim, longest=0,
+                   early_state=False):
         """Linear attention with a decay per head over the batch's new tokens: S <- decays[h] S + k v^T, o = S^T q, with
         q (H dim) | k (H dim) | v (H vdim) the SiLU of the first columns of `fused` ([N, total] float32 or a K-split
         stack).  `state` float32 [slots, H, at least dim * vdim] is read and left updated for the slots `state_slot`
         names (-1: the sequence is skipped); `out` float32 [N, H * vdim].  `longest`: the most new tokens a sequence
         of the batch brings (the batch's shape, known on the host); long portions run as products over 64 tokens at a
-        time, short ones and single tokens as a walk, with the same result up to the order of the sums."""
+        time, short ones and single tokens as a walk, with the same result up to the order of the sums.  `early_state`: the
+        states, `q_start` and `state_slot` were last written by an earlier step or a copy (which have finished), not merely by an
+        earlier launch; the walk then reads them while the kernel before it runs."""
         _dense(fused, torch.float32, "fused projection")
         _dense(state, torch.float32, "state")
         _dense(out, torch.float32, "scan output")
@@ -1051,7 +1054,7 @@ class CudaOps:
         _check(self.core.shrike_decay_scan(
             _ptr(fused), partials, stride, total, _ptr(decays), _ptr(state), _ptr(q_start), _ptr(state_slot), _ptr(out),
             num_seqs, num_heads, dim, vdim, state.shape[0], state.shape[2], int(longest), self.DECAY_CHUNK_FROM, n,
-            _ptr(chunk_state), self._stream()), "decay_scan")
+            _ptr(chunk_state), int(bool(early_state)), self._stream()), "decay_scan")
 
     def norm_gate(self, x, gate_source, gate_at, weight, eps, out):
         """out = x (float32 [N, W]), each row over its root mean square times `weight` (float32 [W]; None: the row as it

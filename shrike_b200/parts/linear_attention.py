@@ -78,7 +78,8 @@ class DecayLinearAttention:
         fused = ops.linear(x, self.w_fused, fused, allow_partials=True)
         scanned = rt.buffer("memory_num", (n, self.out_width), torch.float32)
         ops.decay_scan(fused, self.decays, ctx.storage.state[run.cache], ctx.q_start, ctx.state_slot, scanned,
-                       ctx.num_seqs, spec.num_heads, spec.head_dim, spec.value_dim, longest=ctx.max_q_len)
+                       ctx.num_seqs, spec.num_heads, spec.head_dim, spec.value_dim, longest=ctx.max_q_len,
+                       early_state=True)   # a run's state is its own: only earlier steps wrote it
         out = rt.buffer("memory_out", (n, self.out_width), rt.act_dtype)
         ops.norm_gate(scanned, fused, self.gate_at, self.norm_weight, spec.eps, out)
         delta = rt.buffer("memory_delta", (n, spec.width), torch.float32)

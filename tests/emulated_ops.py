@@ -234,7 +234,8 @@ class EmulatedOps:
         out[:, :width] = resid.to(out.dtype)
         out[:, width:] = other.to(out.dtype)
 
-    def decay_scan(self, fused, decays, state, q_start, state_slot, out, num_seqs, num_heads, dim, vdim, longest=0):
+    def decay_scan(self, fused, decays, state, q_start, state_slot, out, num_seqs, num_heads, dim, vdim, longest=0,
+                   early_state=False):
         if fused.dim() == 3:
             fused = fused.sum(0)
         x = fused.float()

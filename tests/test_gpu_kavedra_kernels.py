@@ -109,6 +109,27 @@ def test_decayed_scan_over_unequal_sequences_skips_padding():
         close(state[slot].view(heads, dim, vdim) / big, final / big, 1e-5, f"state of sequence {index}")
 
 
+@pytest.mark.parametrize("heads,dim,vdim,cut", [(2, 64, 48, 1), (1, 16, 16, 1), (4, 128, 128, 1), (1, 520, 64, 1), (2, 32, 48, 3)])
+def test_scans_in_a_row_on_one_state_without_anything_between_them(heads, dim, vdim, cut):
+    """Launches that follow one another directly: each reads the state that the one before it leaves."""
+    ops = cuda_ops(torch.float32)
+    n, decays = 48 * cut, [0.9, 0.999, 0.5, 1.0][:heads]
+    fused, want, final = scan_case(heads, dim, vdim, n, 3 * heads + dim, decays)
+    pieces = [piece.contiguous() for piece in fused.to(DEV).split(cut)]
+    d = torch.tensor(decays, dtype=torch.float32, device=DEV)
+    state = torch.zeros(1, heads, -(-dim * vdim // 4) * 4, dtype=torch.float32, device=DEV)
+    q_start = torch.tensor([0, cut], dtype=torch.int32, device=DEV)
+    slot = torch.tensor([0], dtype=torch.int32, device=DEV)
+    out = torch.full((n, heads * vdim), float("nan"), dtype=torch.float32, device=DEV)
+    rows = out.split(cut)
+    torch.cuda.synchronize()
+    for piece, to in zip(pieces, rows):
+        ops.decay_scan(piece, d, state, q_start, slot, to, 1, heads, dim, vdim, longest=cut)
+    size, big = max(1.0, float(want.abs().max())), max(1.0, float(final.abs().max()))
+    close(out / size, want / size, 2e-5, "outputs")
+    close(state[0, :, : dim * vdim].view(heads, dim, vdim) / big, final / big, 1e-5, "the state left behind")
+
+
 def test_a_decay_of_one_keeps_a_token_for_ever_and_a_small_one_forgets_it():
     """One large key and value at the first token, the matching query 900 tokens later: the head with decay 1 returns
     the value in full, the head with decay 0.98 a share of 0.98^900 of it, in the chunked form and walking."""
