@@ -984,17 +984,11 @@ SHRIKE_API int shrike_paged_attention_bf16_kept(const void* q, const void* k_cac
     if (splits < 1 || splits % cluster || splits / cluster > MAX_SPLITS || arrivals == nullptr) return SHRIKE_BAD_ARGUMENT;
     if (splits > cluster && scratch == nullptr) return SHRIKE_BAD_ARGUMENT;
   }
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e1 = cudaFuncSetAttribute(portions_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PORTIONS_SMEM));
-    cudaError_t e2 = cudaFuncSetAttribute(single_token_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SINGLE_SMEM));
-    if (e1 != cudaSuccess || e2 != cudaSuccess) return static_cast<int>(e1 != cudaSuccess ? e1 : e2);
-    if (CAN_PAGES) {
-      cudaError_t e3 = cudaFuncSetAttribute(single_token_kernel<CAN_PAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SINGLE_PAGES_SMEM));
-      if (e3 != cudaSuccess) return static_cast<int>(e3);
-    }
-    configured = true;
-  }
+  static PerDevice raised[3];
+  int rc = shrike_raise_smem(raised[0], portions_kernel, PORTIONS_SMEM);
+  if (rc == 0) rc = shrike_raise_smem(raised[1], single_token_kernel<false>, SINGLE_SMEM);
+  if (rc == 0 && CAN_PAGES) rc = shrike_raise_smem(raised[2], single_token_kernel<CAN_PAGES>, SINGLE_PAGES_SMEM);
+  if (rc != 0) return rc;
   Params p;
   p.q = static_cast<const bf16*>(q);
   p.k_cache = static_cast<const bf16*>(k_cache);

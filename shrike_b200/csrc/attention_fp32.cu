@@ -433,17 +433,12 @@ SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, c
   p.scale = scale;
   p.softcap = softcap;
   const int share = num_heads / num_kv_heads;
-  static bool configured = false;
-  if (!configured) {
-    constexpr int FEW = static_cast<int>(shared_floats<16>() * 4), MANY = static_cast<int>(shared_floats<64>() * 4);
-    cudaError_t err = cudaFuncSetAttribute(single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(portions_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW);
-    constexpr int SOME = static_cast<int>(shared_floats<32>() * 4);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(portions_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, SOME);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(portions_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, MANY);
-    if (err != cudaSuccess) return static_cast<int>(err);
-    configured = true;
-  }
+  static PerDevice raised[4];
+  int rc = shrike_raise_smem(raised[0], single_kernel, shared_floats<16>() * 4);
+  if (rc == 0) rc = shrike_raise_smem(raised[1], portions_kernel<16>, shared_floats<16>() * 4);
+  if (rc == 0) rc = shrike_raise_smem(raised[2], portions_kernel<32>, shared_floats<32>() * 4);
+  if (rc == 0) rc = shrike_raise_smem(raised[3], portions_kernel<64>, shared_floats<64>() * 4);
+  if (rc != 0) return rc;
   if (has_portions) {
     // 64 rows a CTA read a key from shared memory for 64 rows, 16 only for 16; but tiles of 64 rows that do not fill the
     // device twice leave it waiting for the last tokens' CTAs, which walk every key

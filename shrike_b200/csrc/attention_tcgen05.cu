@@ -755,13 +755,9 @@ SHRIKE_API int shrike_paged_attention_tc_portions_kept(const void* q, const void
   if (num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads || max_blocks <= 0 || max_q_len < 1 ||
       num_seqs > 65535 || (num_tokens + BM - 1) / BM + num_seqs > 65535 || !(page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64))
     return SHRIKE_BAD_ARGUMENT;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t err = cudaFuncSetAttribute(pair::portions_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(pair::PAIR_SMEM));
-    if (err != cudaSuccess) return static_cast<int>(err);
-    configured = true;
-  }
+  static PerDevice raised;
+  const int raise_rc = shrike_raise_smem(raised, pair::portions_pair_kernel, pair::PAIR_SMEM);
+  if (raise_rc != 0) return raise_rc;
   CUtensorMap map_q, map_k, map_v;
   int rc = bw::tensor_map_bf16(q, num_tokens, num_heads * D, BM, &map_q);
   if (rc != SHRIKE_OK) return rc;

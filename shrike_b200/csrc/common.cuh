@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "per_device.cuh"
+
 #define SHRIKE_API extern "C" __attribute__((visibility("default")))
 
 // Element type codes shared with the Python side.
@@ -37,6 +39,17 @@ static inline const ShrikeDevice& shrike_device() {
     f.sm_count = sms;
   }
   return f;
+}
+
+// Raises a kernel's limit of dynamic shared memory on the current device, once per device (`raised`: a static of the launcher).
+// Returns a CUDA error code.
+template <typename Kernel>
+static inline int shrike_raise_smem(PerDevice& raised, Kernel* kernel, size_t bytes) {
+  int device = -1;
+  if (cudaGetDevice(&device) != cudaSuccess) device = -1;
+  return raised.once(device, [&] {
+    return static_cast<int>(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+  });
 }
 
 template <typename T> __device__ __forceinline__ float to_float(T v);

@@ -762,17 +762,9 @@ SHRIKE_API int shrike_decay_scan(const float* fused, int partials, long long par
   if (chunked) {
     ChunkArgs c;
     c.s = a; c.chunk_state = chunk_state; c.num_seqs = num_seqs; c.skip = skip;
-    static size_t raised_local = 0, raised_finish = 0;
-    if (local_smem > raised_local) {
-      if (cudaFuncSetAttribute(chunk_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit)) != cudaSuccess)
-        return SHRIKE_BAD_ARGUMENT;
-      raised_local = limit;
-    }
-    if (finish_smem > raised_finish) {
-      if (cudaFuncSetAttribute(chunk_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit)) != cudaSuccess)
-        return SHRIKE_BAD_ARGUMENT;
-      raised_finish = limit;
-    }
+    static PerDevice raised[2];
+    if (shrike_raise_smem(raised[0], chunk_local_kernel, limit) != 0 || shrike_raise_smem(raised[1], chunk_finish_kernel, limit) != 0)
+      return SHRIKE_BAD_ARGUMENT;
     // a CTA takes every value column of its run and head (q, k and the scores are staged once) when the runs and heads
     // alone fill the device twice over, else 64 columns
     c.span = static_cast<long long>(chunks) * heads >= 2ll * shrike_device().sm_count ? slices * MAX_SLICE : MAX_SLICE;

@@ -394,14 +394,11 @@ int launch_rows(const float* A, const float* W, const float* bias, float* C, int
   const size_t smem = static_cast<size_t>(WARPS) * stages * STAGE + 1024;
   static_assert(WARPS * 2 * STAGE <= MOST, "two stages must fit");
   static_assert(S == 1 || S * MT * ROWS * RPL * 4 <= WARPS * STAGE, "the runs' partial sums lie in the first stages");
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t err = cudaFuncSetAttribute(rows_kernel<ROWS, RPL, MT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST + 1024);
-    if (err != cudaSuccess) return static_cast<int>(err);
-    configured = true;
-  }
+  static PerDevice raised;
+  int rc = shrike_raise_smem(raised, rows_kernel<ROWS, RPL, MT, S>, MOST + 1024);
+  if (rc != 0) return rc;
   CUtensorMap map_w, map_a;
-  int rc = tensor_map_f32(W, N, K, ROWS * RPL, &map_w);
+  rc = tensor_map_f32(W, N, K, ROWS * RPL, &map_w);
   if (rc != SHRIKE_OK) return rc;
   rc = tensor_map_f32(A, M, K, MT, &map_a);
   if (rc != SHRIKE_OK) return rc;
@@ -442,14 +439,11 @@ int launch_tiles(const float* A, const float* W, const float* bias, float* C, in
                  cudaStream_t stream) {
   constexpr int TILE_M = 8 * TM, STAGE = (TILE_M + TILE_N) * 128;
   constexpr size_t smem = static_cast<size_t>(TILE_STAGES) * STAGE + 1024;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t err = cudaFuncSetAttribute(tile_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (err != cudaSuccess) return static_cast<int>(err);
-    configured = true;
-  }
+  static PerDevice raised;
+  int rc = shrike_raise_smem(raised, tile_kernel<TM>, smem);
+  if (rc != 0) return rc;
   CUtensorMap map_w, map_a;
-  int rc = tensor_map_f32(W, N, K, TILE_N, &map_w);
+  rc = tensor_map_f32(W, N, K, TILE_N, &map_w);
   if (rc != SHRIKE_OK) return rc;
   rc = tensor_map_f32(A, M, K, TILE_M, &map_a);
   if (rc != SHRIKE_OK) return rc;

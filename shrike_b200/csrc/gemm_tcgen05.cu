@@ -299,14 +299,11 @@ static int launch_gemm_tc(const void* x, const void* w, const float* bias, void*
   stages = stages > MAX_STAGES ? MAX_STAGES : stages;
   if (stages > per_split) stages = per_split < 2 ? 2 : per_split;
   const size_t smem = stage_bytes * stages + sizeof(Shared) + 1024;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t err = cudaFuncSetAttribute(gemm_swap_ab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, device.max_smem);
-    if (err != cudaSuccess) return static_cast<int>(err);
-    configured = true;
-  }
+  static PerDevice raised;
+  int rc = shrike_raise_smem(raised, gemm_swap_ab_kernel, device.max_smem);
+  if (rc != 0) return rc;
   CUtensorMap map_w, map_x;
-  int rc = tensor_map_bf16(w, n, k, BM, &map_w);
+  rc = tensor_map_bf16(w, n, k, BM, &map_w);
   if (rc != SHRIKE_OK) return rc;
   rc = tensor_map_bf16(x, tokens, k, tn, &map_x);
   if (rc != SHRIKE_OK) return rc;

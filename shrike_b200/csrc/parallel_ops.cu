@@ -1302,15 +1302,12 @@ SHRIKE_API int shrike_matrix_memory_scan(const float* fused, int partials, long 
   const size_t local_bytes = longest >= CHUNK_FROM && scratch ? chunk_smem_bytes(dim, &scores_bytes, &finish_bytes) : 0;
   const int slices = (vdim + CHUNK_COLS - 1) / CHUNK_COLS;
   if (local_bytes > 0 && slices <= 65535) {
-    static bool chunk_configured = false;
-    if (!chunk_configured) {
-      const int most = shrike_device().max_smem;
-      cudaError_t err = cudaFuncSetAttribute(matrix_memory_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      if (err == cudaSuccess) err = cudaFuncSetAttribute(matrix_memory_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      if (err == cudaSuccess) err = cudaFuncSetAttribute(matrix_memory_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      if (err != cudaSuccess) return static_cast<int>(err);
-      chunk_configured = true;
-    }
+    static PerDevice raised[3];
+    const int most = shrike_device().max_smem;
+    int rc = shrike_raise_smem(raised[0], matrix_memory_local_kernel, most);
+    if (rc == 0) rc = shrike_raise_smem(raised[1], matrix_memory_scores_kernel, most);
+    if (rc == 0) rc = shrike_raise_smem(raised[2], matrix_memory_finish_kernel, most);
+    if (rc != 0) return rc;
     ChunkArgs c = {};
     c.scan = ScanArgs{fused, stride, partials, total, gate_bias, state, q_start, state_slot, numerator, denominator,
                       heads, dim, vdim, CHUNK_COLS, num_slots, cap, q_scale, floor_, head_stride};
@@ -1330,12 +1327,10 @@ SHRIKE_API int shrike_matrix_memory_scan(const float* fused, int partials, long 
   size_t smem = 0;
   const int cols = scan_columns(dim, vdim, &smem);
   if (cols == 0) return SHRIKE_BAD_ARGUMENT;
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    const cudaError_t err = cudaFuncSetAttribute(matrix_memory_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 shrike_device().max_smem);
-    if (err != cudaSuccess) return static_cast<int>(err);
-    configured = shrike_device().max_smem;
+  if (smem > 48 * 1024) {
+    static PerDevice raised;
+    const int rc = shrike_raise_smem(raised, matrix_memory_scan_kernel, shrike_device().max_smem);
+    if (rc != 0) return rc;
   }
   ScanArgs a = {fused, stride, partials, total, gate_bias, state, q_start, state_slot, numerator, denominator,
                 heads, dim, vdim, cols, num_slots, cap, q_scale, floor_, head_stride};

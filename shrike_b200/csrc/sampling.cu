@@ -342,12 +342,9 @@ int launch_sample(const float* logits, const float* temperature, const float* to
   const size_t smem = static_cast<size_t>((vocab + SAMPLE_THREADS - 1) / SAMPLE_THREADS) * ROW_THREADS * sizeof(float);
   constexpr size_t MOST = 200 * 1024;
   if (smem <= MOST) {
-    static bool configured = false;
-    if (!configured) {
-      err = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(MOST));
-      if (err != cudaSuccess) return static_cast<int>(err);
-      configured = true;
-    }
+    static PerDevice raised;
+    const int rc = shrike_raise_smem(raised, sample_cluster_kernel, MOST);
+    if (rc != 0) return rc;
     err = launch_dependent_clusters(sample_cluster_kernel, dim3(rows * ROW_CTAS), dim3(ROW_THREADS), smem, stream, ROW_CTAS, logits,
                                     temperature, top_p, seeds, out, static_cast<const float*>(scratch_value),
                                     static_cast<const int*>(scratch_index), vocab, chunks, status);

@@ -23,7 +23,8 @@
 //     at zero).  Two calls that overlap on the GPU (different streams, or different
 //     threads without ordering) race on it: serialise them.
 //   * The first call on each device looks up the array's device address
-//     (cudaGetSymbolAddress, with that device current).  Make that first call outside any
+//     (cudaGetSymbolAddress, with that device current) and raises the sampling kernel's limit
+//     of shared memory there (cudaFuncSetAttribute).  Make that first call outside any
 //     stream capture.
 //   * Devices with an index of 64 or more are refused (SHRIKE_SAMPLE_NO_ALLOC_BAD_DEVICE).
 //   * A row whose logits are all NaN has no largest element; it yields token 0.
