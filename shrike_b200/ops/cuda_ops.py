@@ -15,6 +15,7 @@ from __future__ import annotations
 import ctypes
 
 import torch
+from torch.multiprocessing.reductions import StorageWeakRef
 
 from . import build
 
@@ -107,7 +108,7 @@ class CudaOps:
         self.gemm_tc = None
         self.tensor_core_attention = True   # tcgen05 kernel for portions where the head and page sizes allow
         self.tensor_core_gemm_max_tokens = 64   # above this the library product is used
-        self._partials = {}      # data_ptr of an output buffer -> its stack of K-split partial results
+        self._partials = {}      # data_ptr of an output buffer -> (its memory, weakly; its stack of K-split partial results)
         # one host-visible word (of four): the first kernel whose bounded wait ran out, or that met
         # a row without a finite logit, leaves its code here; see `describe_status`
         self.status = torch.zeros(4, dtype=torch.int32, device=self.device)
@@ -541,7 +542,7 @@ class CudaOps:
             _dense(out, torch.float32, "linear output")
             # K is cut into the same runs, added in the same order, whether they leave as a stack or summed
             stack = self.core.shrike_gemm_fp32_stack(n, o, k) if allow_partials and bias is None else 1
-            if stack > 1 and (x.data_ptr() | w.data_ptr()) % 16:
+            if stack > 1 and ((x.data_ptr() | w.data_ptr()) % 16 or stack * n * o > self.FP32_STACK_FLOATS):
                 stack = 1
             target = self._partial_stack(out, stack) if stack > 1 else out
             _check(self.core.shrike_gemm_fp32(_ptr(x), _ptr(w), _ptr(bias), _ptr(target), n, o, k, stack, _ptr(self.status),
@@ -569,16 +570,21 @@ class CudaOps:
             out.add_(bias)
         return out
 
+    FP32_STACK_FLOATS = 64 << 20   # at most 256 MiB for the runs of a 32-bit product; they are summed by the product beyond that
+
     def _partial_stack(self, out, splits):
-        """The float32 [splits, N, O] stack that belongs to the output buffer `out`."""
+        """The float32 [splits, N, O] stack that belongs to the output buffer `out`, for as long as that buffer's memory lives:
+        a stack whose buffer was replaced is given back when the next one is made."""
         n, o = out.shape
-        key = out.data_ptr()
-        held = self._partials.get(key)
+        key, memory = out.data_ptr(), out.untyped_storage()
+        owner, held = self._partials.get(key, (None, None))
         need = splits * n * o
-        if held is None or held.numel() < need:
-            capacity = max(need, 16 * self.tensor_core_gemm_max_tokens * o)
-            held = torch.empty(capacity, dtype=torch.float32, device=self.device)
-            self._partials[key] = held
+        if owner is None or owner.cdata != memory._cdata or held.numel() < need:
+            self._partials = {k: v for k, v in self._partials.items() if not v[0].expired() and k != key}
+            # as many rows as the few-token forms of the product take: the stack of a growing batch stays where it is
+            rows = splits * 16 if self.dtype == torch.float32 else 16 * self.tensor_core_gemm_max_tokens
+            held = torch.empty(max(need, rows * o), dtype=torch.float32, device=self.device)
+            self._partials[key] = (StorageWeakRef(memory), held)
             self.generation += 1
         return held[:need].view(splits, n, o)
 

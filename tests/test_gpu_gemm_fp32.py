@@ -44,3 +44,20 @@ def test_gemm_fp32_gives_a_row_the_same_bits_in_every_batch(n, k):
         ops.linear(x[:m].contiguous(), w, with_bias, bias=bias, allow_partials=True)
         assert torch.equal(with_bias, whole + bias), m
     ops.check_status()
+
+
+def test_gemm_fp32_sums_its_runs_itself_where_their_stack_would_be_too_large():
+    ops = cuda_ops(torch.float32)
+    m, n, k = 40, 96, 9000
+    x, w = rnd(m, k, seed=1), rnd(n, k, seed=2)
+    stack = ops.linear(x, w, torch.empty(m, n, device=DEV), allow_partials=True)
+    assert stack.dim() == 3
+    total = stack[0].clone()
+    for part in stack[1:]:
+        total += part
+    ops.FP32_STACK_FLOATS = stack.numel()
+    assert ops.linear(x, w, torch.empty(m, n, device=DEV), allow_partials=True).dim() == 3
+    ops.FP32_STACK_FLOATS = stack.numel() - 1
+    out = torch.empty(m, n, device=DEV)
+    got = ops.linear(x, w, out, allow_partials=True)
+    assert got.data_ptr() == out.data_ptr() and torch.equal(got, total)
