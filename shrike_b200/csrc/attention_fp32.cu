@@ -45,7 +45,7 @@ struct Params {
   float* partial;        // [seqs][heads][chunks][D + 2]: outputs, maximum, sum; null: rows are finished here
   int max_blocks, num_heads, num_kv_heads, page_size, num_pages, window, keep_first, num_tokens, num_seqs, chunks;
   int heads_per_cta, head_groups, skip_single;
-  int aligned;           // q and out lie on 16 bytes
+  int aligned, kv_aligned;   // q and out lie on 16 bytes; keys and values do
   float scale, softcap;
 };
 
@@ -54,6 +54,13 @@ template <int R> constexpr size_t shared_floats() { return static_cast<size_t>(R
 __device__ __forceinline__ void copy16(float* smem, const float* from, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))), "l"(from),
                "r"(valid ? 16 : 0));
+}
+// The same for four elements that do not lie on 16 bytes.
+__device__ __forceinline__ void copy4_each(float* smem, const float* from, bool valid) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem + e))), "l"(from + e),
+                 "r"(valid ? 4 : 0));
 }
 
 // One row's running softmax.  Explicit roundings: every use of the row gives the same bits.
@@ -150,8 +157,13 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
       const int r = i / (D / 4), c = i % (D / 4);
       const long long row = row_s[walked & 3][r];
       const size_t at = row >= 0 ? static_cast<size_t>(row) * key_stride + static_cast<size_t>(kv_head) * D + c * 4 : 0;
-      copy16(k_to + r * ROW + c * 4, p.k_cache + at, row >= 0);
-      copy16(v_to + r * ROW + c * 4, p.v_cache + at, row >= 0);
+      if (p.kv_aligned) {
+        copy16(k_to + r * ROW + c * 4, p.k_cache + at, row >= 0);
+        copy16(v_to + r * ROW + c * 4, p.v_cache + at, row >= 0);
+      } else {
+        copy4_each(k_to + r * ROW + c * 4, p.k_cache + at, row >= 0);
+        copy4_each(v_to + r * ROW + c * 4, p.v_cache + at, row >= 0);
+      }
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
@@ -430,6 +442,7 @@ SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, c
   p.chunks = chunks;
   p.skip_single = has_single;
   p.aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  p.kv_aligned = ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
   p.scale = scale;
   p.softcap = softcap;
   const int share = num_heads / num_kv_heads;

@@ -74,3 +74,24 @@ def test_fp32_attention_keeps_a_later_tokens_values_out():
     case["values"][page, 7] = float("inf")   # the value of position 39
     got = attention(ops, case, case["q"], *args)
     assert torch.equal(got[:39], want[:39]) and not torch.isfinite(got[39]).all()
+
+
+def test_fp32_attention_takes_pages_that_do_not_lie_on_16_bytes():
+    """Views into a larger array, one element behind a 16-byte border: plain loads in place of wide ones, the same bits."""
+    ops = cuda_ops(torch.float32)
+    heads, kv_heads, dim, lens = 6, 2, 48, [70, 1, 33]
+    case = paged_case(torch.float32, heads, kv_heads, dim, 16, lens, lens, seed=5)
+    shifted = dict(case)
+    for name in ("keys", "values"):
+        room = torch.empty(case[name].numel() + 1, device=DEV)
+        shifted[name] = room[1:].view(case[name].shape)
+        shifted[name].copy_(case[name])
+    last = (case["q_start"][1:] - 1).long()
+    index = torch.arange(len(lens) + 1, dtype=torch.int32, device=DEV)
+    for which in (("keys",), ("values",), ("keys", "values")):
+        moved = dict(case, **{name: shifted[name] for name in which})
+        whole = [attention(ops, c, c["q"], c["q_start"], c["ctx_len"], c["seq_of"], c["table"], heads, kv_heads, dim, lens) for c in (case, moved)]
+        assert torch.equal(*whole)
+        alone = [attention(ops, c, c["q"][last].contiguous(), index, c["ctx_len"], index[: len(lens)], c["table"], heads, kv_heads, dim, [1] * len(lens))
+                 for c in (case, moved)]
+        assert torch.equal(*alone) and torch.equal(alone[0], whole[0][last])
