@@ -45,6 +45,7 @@ struct Params {
   float* partial;        // [seqs][heads][chunks][D + 2]: outputs, maximum, sum; null: rows are finished here
   int max_blocks, num_heads, num_kv_heads, page_size, num_pages, window, keep_first, num_tokens, num_seqs, chunks;
   int heads_per_cta, head_groups, skip_single;
+  int early_metadata;    // 1: no kernel still running writes the tables, starts and lengths: they are read before the wait
   int aligned, kv_aligned;   // q and out lie on 16 bytes; keys and values do
   float scale, softcap;
 };
@@ -191,7 +192,7 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
     row_s[0][t] = lookup(tile);
     if (second < tile_end) row_s[1][t] = lookup(second);
   }
-  wait_for_previous();   // so far the step's metadata alone was read, which no kernel writes
+  if (p.early_metadata) wait_for_previous();   // so far the step's metadata alone was read
   for (int i = t; i < R * (D / 4); i += THREADS) {
     const int r = i / (D / 4), c = i % (D / 4);
     const bool valid = r < rows;
@@ -328,11 +329,12 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
 __global__ void __launch_bounds__(THREADS) single_kernel(const Params p) {
   extern __shared__ __align__(16) float smem[];
   let_dependents_start();
+  if (!p.early_metadata) wait_for_previous();
   const int seq = blockIdx.z, kv_head = blockIdx.y / p.head_groups, group = blockIdx.y % p.head_groups;
   const int token = p.q_start[seq];
   // a longer entry: the portions kernel's; or the table is wider than the sequence is long
   if (p.q_start[seq + 1] - token != 1 || (p.chunks > 1 && static_cast<int>(blockIdx.x) * CHUNK >= p.ctx_len[seq])) {
-    wait_for_previous();
+    if (p.early_metadata) wait_for_previous();   // every CTA waits before it leaves
     return;
   }
   const int share = p.num_heads / p.num_kv_heads, head = kv_head * share + group * p.heads_per_cta;
@@ -380,6 +382,7 @@ template <int R>
 __global__ void __launch_bounds__(THREADS) portions_kernel(const Params p) {
   extern __shared__ __align__(16) float smem[];
   let_dependents_start();
+  if (!p.early_metadata) wait_for_previous();
   const int kv_head = blockIdx.y / p.head_groups, group = blockIdx.y % p.head_groups;
   const int share = p.num_heads / p.num_kv_heads, head = kv_head * share + group * p.heads_per_cta;
   const int heads = min(p.heads_per_cta, share - group * p.heads_per_cta);
@@ -395,7 +398,7 @@ __global__ void __launch_bounds__(THREADS) portions_kernel(const Params p) {
     }
     token = stop > token ? stop : token + 1;
   }
-  wait_for_previous();
+  if (p.early_metadata) wait_for_previous();
 }
 
 }  // namespace attn32
@@ -406,13 +409,14 @@ SHRIKE_API int shrike_attention_head_dim() { return attn32::D; }
 SHRIKE_API int shrike_attention_fp32_chunk() { return attn32::CHUNK; }
 
 // `has_single`: single tokens run on CTAs per chunk (scratch: float32 [seqs][heads][chunks][head size + 2]); `has_portions`: the
-// entries of more than one token (all entries when there is no `has_single`) run on tiles of tokens.
+// entries of more than one token (all entries when there is no `has_single`) run on tiles of tokens.  `early_metadata` 1: the
+// caller knows that whatever wrote the block table, q_start, ctx_len and seq_of_token has finished (a copy, or an earlier step).
 SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
                                            int max_blocks, const int* q_start, const int* ctx_len, const int* seq_of_token,
                                            int num_tokens, int num_seqs, int num_heads, int num_kv_heads, int page_size, int num_pages,
                                            float scale, int window, float softcap, const float* slopes, const float* sinks,
-                                           int keep_first, int has_single, int has_portions, int chunks, float* scratch, void* out,
-                                           cudaStream_t stream) {
+                                           int keep_first, int has_single, int has_portions, int chunks, float* scratch,
+                                           int early_metadata, void* out, cudaStream_t stream) {
   using namespace attn32;
   if (num_tokens <= 0) return SHRIKE_OK;
   if (keep_first < 0 || num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads || page_size <= 0 || max_blocks <= 0 || num_seqs <= 0 ||
@@ -441,6 +445,7 @@ SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, c
   p.num_seqs = num_seqs;
   p.chunks = chunks;
   p.skip_single = has_single;
+  p.early_metadata = early_metadata;
   p.aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   p.kv_aligned = ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
   p.scale = scale;

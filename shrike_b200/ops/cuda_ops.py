@@ -240,7 +240,7 @@ class CudaOps:
                 lib.shrike_paged_attention_generic_kept.restype = _I
             else:
                 lib.shrike_paged_attention_fp32.argtypes = (
-                    [_P, _P, _P, _P, _I, _P, _P, _P] + [_I] * 6 + [_F, _I, _F, _P, _P] + [_I] * 4 + [_P, _P, _P]
+                    [_P, _P, _P, _P, _I, _P, _P, _P] + [_I] * 6 + [_F, _I, _F, _P, _P] + [_I] * 4 + [_P, _I, _P, _P]
                 )
                 lib.shrike_paged_attention_fp32.restype = _I
                 lib.shrike_attention_fp32_chunk.restype = _I
@@ -526,7 +526,8 @@ class CudaOps:
                                              vdim, width // heads, self._stream()), "element_gate")
 
     def linear(self, x, w, out, bias=None, allow_partials=False):
-        """x[N, K] @ w[O, K]^T (+ bias) into `out` [N, O] (float32 or the activation type).
+        """x[N, K] @ w[O, K]^T (+ bias) into `out` [N, O] (float32 or the activation type).  `w` is a parameter, not something a
+        kernel of this step computes: it is read while the kernels launched before may still run.
 
         Returns the array to consume: `out`, or, when `allow_partials` and the product was
         split along K, a float32 stack [P, N, O] whose sum over P is the result (the
@@ -667,7 +668,7 @@ class CudaOps:
     def paged_attention(self, q, keys, values, block_table, q_start, ctx_len, seq_of_token,
                         num_heads, num_kv_heads, head_dim, scale, window, out,
                         max_q_len=0, max_ctx_len=0, min_q_len=0, q_lens=None, softcap=None, slopes=None, chunk=None,
-                        sinks=None, keep_first=0):
+                        sinks=None, keep_first=0, early_metadata=False):
         """Attention of the batch's new tokens over the paged cache.  `window`: a query sees the `window`
         latest keys.  `chunk` (instead of a window): a query at position p sees key j <= p only when
         floor(p / chunk) = floor(j / chunk).  `max_q_len` and
@@ -677,7 +678,10 @@ class CudaOps:
         s = scale * q.k, in this order: s <- softcap * tanh(s / softcap), then
         s <- s - slopes[head] * (query position - key position).  `sinks` (float32 [num_heads]): exp(sinks[head])
         is one more term of every softmax's denominator: a weight that goes to nothing (the raw number, without `scale`).
-        `keep_first` (with a window): the sequence's first `keep_first` keys stay visible to every later query."""
+        `keep_first` (with a window): the sequence's first `keep_first` keys stay visible to every later query.
+        `early_metadata`: `block_table`, `q_start`, `ctx_len` and `seq_of_token` were last written by a copy or an earlier step
+        (which have finished), not by a kernel of this step; they are then read while the kernel before this one runs.  In
+        bfloat16 (heads of up to 256) they always are, and have to be such."""
         _dense(q, self.dtype, "q")
         if sinks is not None:
             _dense(sinks, torch.float32, "softmax sinks")
@@ -712,8 +716,8 @@ class CudaOps:
             _check(lib.shrike_paged_attention_fp32(
                 _ptr(q), _ptr(keys), _ptr(values), _ptr(block_table), max_blocks, _ptr(q_start), _ptr(ctx_len), _ptr(seq_of_token),
                 q.shape[0], num_seqs, num_heads, num_kv_heads, page_size, num_pages, scale, window or 0, softcap or 0.0,
-                _ptr(slopes), _ptr(sinks), keep_first, has_single, has_portions, chunks, _ptr(scratch), _ptr(out),
-                self._stream()), "paged_attention_fp32")
+                _ptr(slopes), _ptr(sinks), keep_first, has_single, has_portions, chunks, _ptr(scratch),
+                int(bool(early_metadata)), _ptr(out), self._stream()), "paged_attention_fp32")
             return
         if slopes is not None:
             _dense(slopes, torch.float32, "distance slopes")

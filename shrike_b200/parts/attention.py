@@ -114,6 +114,7 @@ class PagedAttention:
             q, keys, values, view.block_table, ctx.q_start, ctx.ctx_len, ctx.seq_of_token,
             spec.num_heads, spec.num_kv_heads, spec.head_dim, spec.scale, spec.window, attn,
             max_q_len=ctx.max_q_len, max_ctx_len=ctx.max_ctx_len, min_q_len=ctx.min_q_len, q_lens=ctx.q_lens,
+            early_metadata=True,
         )
         delta = rt.buffer("mixer_delta", (n, spec.width), torch.float32)
         return ops.linear(attn, self.w_o, delta, bias=self.b_o, allow_partials=True)
@@ -185,6 +186,7 @@ class SharedKeyValueAttention:
             q, keys, values, view.block_table, ctx.q_start, ctx.ctx_len, ctx.seq_of_token,
             spec.num_heads, spec.num_kv_heads, self.padded, spec.scale, spec.window, attn,
             max_q_len=ctx.max_q_len, max_ctx_len=ctx.max_ctx_len, min_q_len=ctx.min_q_len, q_lens=ctx.q_lens,
+            early_metadata=True,
             softcap=spec.softcap, slopes=self.slopes,
         )
         delta = rt.buffer("mixer_delta", (n, spec.width), torch.float32)
@@ -354,6 +356,7 @@ class GatedHeadAttention:
             q, keys, values, view.block_table, ctx.q_start, ctx.ctx_len, ctx.seq_of_token,
             spec.num_heads, spec.num_kv_heads, self.padded, spec.scale, spec.window, attn,
             max_q_len=ctx.max_q_len, max_ctx_len=ctx.max_ctx_len, min_q_len=ctx.min_q_len, q_lens=ctx.q_lens,
+            early_metadata=True,
             **({"chunk": spec.chunk} if spec.chunk is not None else {}),
             **({"sinks": self.sinks} if self.sinks is not None else {}),
             **({"softcap": spec.softcap} if getattr(spec, "softcap", None) else {}),

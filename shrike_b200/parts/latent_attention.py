@@ -100,6 +100,7 @@ class LatentAttention:
             q, latents, latents, view.block_table, ctx.q_start, ctx.ctx_len, ctx.seq_of_token,
             heads, 1, padded, spec.scale, None, attended,
             max_q_len=ctx.max_q_len, max_ctx_len=ctx.max_ctx_len, min_q_len=ctx.min_q_len, q_lens=ctx.q_lens,
+            early_metadata=True,
         )
         if spec.gated:
             ops.head_scale(attended, gate, heads, padded)
@@ -199,6 +200,7 @@ class RotaryLatentAttention:
             q, latents, latents, view.block_table, ctx.q_start, ctx.ctx_len, ctx.seq_of_token,
             heads, 1, padded, spec.scale, spec.window, attended,
             max_q_len=ctx.max_q_len, max_ctx_len=ctx.max_ctx_len, min_q_len=ctx.min_q_len, q_lens=ctx.q_lens,
+            early_metadata=True,
         )
         out = rt.buffer("latent_gated", (n, self.out_width), rt.act_dtype)
         if self.gated:

@@ -95,3 +95,25 @@ def test_fp32_attention_takes_pages_that_do_not_lie_on_16_bytes():
         alone = [attention(ops, c, c["q"][last].contiguous(), index, c["ctx_len"], index[: len(lens)], c["table"], heads, kv_heads, dim, [1] * len(lens))
                  for c in (case, moved)]
         assert torch.equal(*alone) and torch.equal(alone[0], whole[0][last])
+
+
+def test_fp32_attention_reads_lengths_that_kernels_of_the_stream_just_wrote():
+    """One request that grows by a token a round: its length is written by a kernel, the store of its newest key and value and
+    the attention follow directly, round after round."""
+    ops = cuda_ops(torch.float32)
+    heads, kv_heads, dim, page, n = 6, 2, 64, 16, 130
+    case = paged_case(torch.float32, heads, kv_heads, dim, page, [n], [n], seed=8)
+    want = attention(ops, case, case["q"], case["q_start"], case["ctx_len"], case["seq_of"], case["table"], heads, kv_heads, dim, [n])
+    q, k, v = (t.to(DEV).reshape(n, -1).contiguous() for t in case["seqs"][0])
+    keys, values = torch.full_like(case["keys"], float("nan")), torch.full_like(case["values"], float("nan"))
+    table = case["table"].long()[0]
+    slots = (table[torch.arange(n, device=DEV) // page] * page + torch.arange(n, device=DEV) % page).to(torch.int32)
+    q_start, seq_of = torch.tensor([0, 1], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ctx_len, out = torch.zeros(1, dtype=torch.int32, device=DEV), torch.full((n, heads * dim), float("nan"), device=DEV)
+    torch.cuda.synchronize()
+    for i in range(n):
+        ctx_len.add_(1)
+        ops.kv_write(k[i: i + 1], v[i: i + 1], keys, values, slots[i: i + 1])
+        ops.paged_attention(q[i: i + 1], keys, values, case["table"], q_start, ctx_len, seq_of, heads, kv_heads, dim, dim ** -0.5, None,
+                            out[i: i + 1], max_q_len=1, min_q_len=1)
+    assert torch.equal(out, want)
