@@ -420,8 +420,12 @@ SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, c
   using namespace attn32;
   if (num_tokens <= 0) return SHRIKE_OK;
   if (keep_first < 0 || num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads || page_size <= 0 || max_blocks <= 0 || num_seqs <= 0 ||
-      num_seqs > 65535 || chunks < 1 || (has_single && chunks > 1 && scratch == nullptr))
+      chunks < 1 || (has_single && chunks > 1 && scratch == nullptr))
     return SHRIKE_BAD_ARGUMENT;
+  if (num_seqs > 65535) {   // more than a grid's z: tiles of tokens serve entries of any length, with the same bits
+    has_single = 0;
+    has_portions = 1;
+  }
   Params p = {};
   p.q = static_cast<const float*>(q);
   p.k_cache = static_cast<const float*>(k_cache);

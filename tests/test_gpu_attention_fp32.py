@@ -117,3 +117,18 @@ def test_fp32_attention_reads_lengths_that_kernels_of_the_stream_just_wrote():
         ops.paged_attention(q[i: i + 1], keys, values, case["table"], q_start, ctx_len, seq_of, heads, kv_heads, dim, dim ** -0.5, None,
                             out[i: i + 1], max_q_len=1, min_q_len=1)
     assert torch.equal(out, want)
+
+
+def test_fp32_attention_of_more_sequences_than_a_grid_has_places():
+    ops = cuda_ops(torch.float32)
+    count, heads, dim, page = 65600, 2, 16, 4
+    keys, values = rnd(count, page, 1, dim, seed=1), rnd(count, page, 1, dim, seed=2)
+    q = rnd(count, heads * dim, seed=3)
+    table = torch.randperm(count, generator=torch.Generator().manual_seed(4)).to(torch.int32).to(DEV).view(count, 1)
+    ctx_len = torch.randint(1, page + 1, (count,), generator=torch.Generator().manual_seed(5)).to(torch.int32).to(DEV)
+    index = torch.arange(count + 1, dtype=torch.int32, device=DEV)
+    case = {"keys": keys, "values": values}
+    whole = attention(ops, case, q, index, ctx_len, index[:count], table, heads, 1, dim, [1] * count)
+    few = attention(ops, case, q[-300:].contiguous(), index[:301].clone(), ctx_len[-300:].contiguous(), index[:300], table[-300:].contiguous(), heads, 1,
+                    dim, [1] * 300)
+    assert torch.isfinite(whole).all() and torch.equal(whole[-300:], few)
