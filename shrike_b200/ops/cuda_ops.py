@@ -831,16 +831,24 @@ class CudaOps:
         of clusters starts late (a cluster needs all its places free in one part of the chip
         at once, while the kernel before it is still leaving), and the splits then meet in
         global memory instead, eight partials to a round trip.  Long contexts take several
-        clusters per pair, whose partials meet in global memory too."""
+        clusters per pair, whose partials meet in global memory too.  Two exceptions, measured for heads of
+        64 and 128 at 24 to 148 pairs and contexts of 120 to 3,000 keys: few keys for many pairs stay on
+        one CTA, and a count of splits between two powers of two is taken, without clusters, where it
+        leaves a CTA fewer tiles than the power below it."""
         want = max(1, min(tiles, resident // max(1, groups)))
-        if groups >= 64 and tiles <= 4:   # 256 keys: what a second CTA saves it spends on adding up (80 pairs: 6.9 us against 8.6)
+        # up to 256 keys: what a second CTA saves it spends on adding up (250 keys, heads of 128: 64 pairs 6.6 us and 7.1 with
+        # four, 80 pairs 6.8 and 8.4 with two, 148 pairs 6.4 and 9.8)
+        if groups >= 64 and tiles <= 4:
             return 1, 1
         cluster = 1
         while cluster * 2 <= min(want, 8):
             cluster *= 2
         if cluster == 8 and groups * 8 * 3 > resident * 2:
             return min(want, 32) // 8 * 8, 1
-        if groups >= 24 and cluster < want < 2 * cluster:   # places that a power of two leaves empty (80 pairs: 3 splits 11.1 us, 2 13.9)
+        # places that a power of two leaves empty (1,000 keys: 80 pairs 12.4 us with 3 splits and 15.0 with 2, 48 pairs 9.9 with 6
+        # and 10.4 with 4; 24 pairs 3,000 keys 12.1 with 12 and 13.1 with 8).  Where a CTA's tiles do not get fewer they only add
+        # partials to add up (24 pairs, 1,000 keys: 9.8 with 12 and 8.5 with 8; 48 pairs, 500 keys: 8.9 with 6 and 8.4 with 4).
+        if groups >= 24 and cluster < want < 2 * cluster and -(-tiles // want) < -(-tiles // cluster):
             return want, 1
         if tiles <= 4 * cluster or want < 2 * cluster:
             return cluster, cluster

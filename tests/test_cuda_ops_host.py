@@ -35,3 +35,26 @@ def test_a_stack_lives_as_long_as_the_buffer_it_belongs_to(dtype):
     assert again.data_ptr() == where and ops.generation > stamp
     grown = ops._partial_stack(kept.view(2048, 8), 4)
     assert grown.shape == (4, 2048, 8)
+
+
+def test_single_token_splits_where_the_places_of_a_power_of_two_would_stay_empty():
+    """Every count of pairs up to the device's places: no clusters beyond two thirds of it, and splits between two powers of
+    two only where they leave a CTA fewer tiles."""
+    resident = 296
+    for tiles in range(1, 200):
+        for groups in range(1, 300):
+            splits, cluster = CudaOps.single_token_splits(tiles, groups, resident)
+            want = max(1, min(tiles, resident // groups))
+            assert 1 <= splits <= want and splits % cluster == 0 and splits // cluster <= 32
+            power = 1 << (min(want, 8).bit_length() - 1)
+            if splits & (splits - 1) and cluster == 1:
+                assert groups >= 24 and (splits == want or splits % 8 == 0)
+                assert splits % 8 == 0 or -(-tiles // splits) < -(-tiles // power)
+            if tiles <= 4 and groups >= 64:
+                assert (splits, cluster) == (1, 1)
+    assert CudaOps.single_token_splits(16, 24, resident) == (8, 8)      # twelve CTAs would have two tiles too
+    assert CudaOps.single_token_splits(64, 24, resident) == (12, 1)     # six tiles a CTA instead of eight
+    assert CudaOps.single_token_splits(8, 48, resident) == (4, 4)
+    assert CudaOps.single_token_splits(16, 48, resident) == (6, 1)
+    assert CudaOps.single_token_splits(16, 80, resident) == (3, 1)
+    assert CudaOps.single_token_splits(4, 63, resident) == (4, 4)
