@@ -102,6 +102,7 @@ class CudaOps:
         self.dtype = dtype
         self.code = _DTYPE_CODE[dtype]
         self.device = torch.device(device)
+        self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.core = build.core_library()
         self._declare_core()
         self._attention = {}
@@ -724,7 +725,8 @@ class CudaOps:
             if slopes.numel() != num_heads:
                 raise KernelError("one distance slope per query head")
         plan = self.attention_plan(num_heads, num_kv_heads, head_dim, num_seqs, max_blocks, page_size, max_q_len, min_q_len,
-                                   q.shape[0], q_lens, keep_first=keep_first, own_values=keys.data_ptr() == values.data_ptr())
+                                   q.shape[0], q_lens, keep_first=keep_first, own_values=keys.data_ptr() == values.data_ptr(),
+                                   max_ctx_len=max_ctx_len)
         self.launches += plan.has_single + plan.has_portions + (1 if plan.portion_splits > 1 else 0)
         has_portions = plan.has_portions
         if plan.tc_portions:
@@ -752,7 +754,7 @@ class CudaOps:
         same.  `keys`: what the block tables can hold."""
         chunks = -(-keys // lib.shrike_attention_fp32_chunk())
         need = num_seqs * num_heads * chunks * (head_dim + 2)
-        if num_seqs * num_kv_heads >= 4 * 148 or need > self.FP32_SCRATCH_FLOATS:
+        if num_seqs * num_kv_heads >= 4 * self.sm_count or need > self.FP32_SCRATCH_FLOATS:
             chunks = 1
         if chunks == 1:
             return 1, None
@@ -773,7 +775,7 @@ class CudaOps:
         return tiles
 
     def attention_plan(self, num_heads, num_kv_heads, head_dim, num_seqs, max_blocks, page_size, max_q_len, min_q_len,
-                       num_tokens=0, q_lens=None, keep_first=0, own_values=False):
+                       num_tokens=0, q_lens=None, keep_first=0, own_values=False, max_ctx_len=0):
         """How a bfloat16 batch's attention is cut: which kernels run (single tokens, portions, the
         tensor-core form of the latter), the key splits and clusters of the single-token kernel, the
         key splits of the portions kernel, and their scratch.  A function of the batch's shape alone."""
@@ -797,9 +799,8 @@ class CudaOps:
                 self._arrivals = torch.zeros(max(groups, 4096), dtype=torch.int32, device=self.device)
                 self.generation += 1
             scratch, arrivals = self._scratch, self._arrivals
-        # the tensor-core form walks long contexts several times faster, but starts slower: a prompt of 43 tokens takes 5.6 us
-        # with it and 4.4 with the mma.sync kernel (14 heads of 64), one of 100 the same with both
-        short = max_q_len <= 64 and max_blocks * page_size <= 128
+        short = self.short_portions(max_q_len, max_blocks * page_size, max_ctx_len, head_dim,
+                                    num_heads * (sum(q > 1 or not has_single for q in q_lens) if q_lens is not None else num_seqs))
         tc_portions = bool(has_portions and self.tensor_core_attention and lib.shrike_attention_tc_available() and not short
                            and page_size in (8, 16, 32, 64) and (own_values or not lib.shrike_attention_tc_own_values()))
         portion_splits, portion_scratch = 1, None
@@ -820,6 +821,25 @@ class CudaOps:
                 portion_scratch = self._portion_scratch
         return AttentionPlan(int(has_single), int(has_portions), int(tc_portions), splits, cluster, scratch, arrivals,
                              portion_splits, portion_scratch)
+
+    SHORT_CONTEXT = 64   # keys: a launch captured for a batch's lengths holds for contexts on the same side of it
+
+    def short_portions(self, max_q_len, table_keys, max_ctx_len, head_dim, ctas) -> bool:
+        """Whether portions run on the mma.sync kernel although the tcgen05 one serves them: portions of up to 64 tokens over few
+        keys.  The tcgen05 kernel walks long contexts several times faster, but starts slower (its set-up alone is 5.5 us) and
+        gives a portion of any length a whole SM, so that a batch of more (portion, head) pairs (`ctas`) than SMs takes it
+        another round.  Measured, tcgen05 and mma.sync, us: nothing before the tokens: 14 heads of 64, 43 tokens 5.4 and 4.1; 12
+        heads of 128 6.2 and 5.2; 12 own-value heads of 256 7.4 and 6.8; 13 such portions of 128 12.4 and 8.0.  Between half the
+        SMs and all of them the longer portions lose on heads of 128 and 256 (28 heads, 4 portions of 24, 33 and 64 tokens: 6.8 and
+        4.9, 6.8 and 6.3, 7.1 and 7.6) and win on heads of 64 (6.3 and 5.3).  Up to 128 keys with some before the tokens: heads of 64
+        6.3 and 5.8 to 6.1 (one portion), 7.4 and 8.4 (ten of 64 tokens); heads of 128 6.8 and 8.1."""
+        if max_q_len > 64:
+            return False
+        keys = min(table_keys, max_ctx_len) if max_ctx_len > 0 else table_keys
+        few = max_q_len <= 32 or 2 * ctas <= self.sm_count or ctas > self.sm_count
+        if keys <= self.SHORT_CONTEXT:
+            return few or head_dim <= 64
+        return keys <= 2 * self.SHORT_CONTEXT and head_dim <= 64 and few
 
     @staticmethod
     def single_token_splits(tiles: int, groups: int, resident: int):

@@ -193,7 +193,7 @@ class LayerProgram:
         step.down_splits = 1 if library else splits_of(n, width, inter)
         step.gated_fused = int(bool(feed_forward.run) and not library and (2 * inter) % 32 == 0)
         plan = ops.attention_plan(spec.num_heads, spec.num_kv_heads, spec.head_dim, ctx.num_seqs, view.max_blocks, page_size,
-                                  ctx.max_q_len, ctx.min_q_len, n, ctx.q_lens)
+                                  ctx.max_q_len, ctx.min_q_len, n, ctx.q_lens, max_ctx_len=ctx.max_ctx_len)
         step.portion_splits = plan.portion_splits
         step.portion_tiles = ops.portion_tiles(ctx.q_lens, plan.has_single,
                                                ops._attention_lib(spec.head_dim).shrike_attention_tc_portions_rows())

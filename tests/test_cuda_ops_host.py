@@ -58,3 +58,40 @@ def test_single_token_splits_where_the_places_of_a_power_of_two_would_stay_empty
     assert CudaOps.single_token_splits(16, 48, resident) == (6, 1)
     assert CudaOps.single_token_splits(16, 80, resident) == (3, 1)
     assert CudaOps.single_token_splits(4, 63, resident) == (4, 4)
+
+
+@pytest.mark.parametrize("max_q_len,table_keys,max_ctx_len,head_dim,ctas,short", [
+    (43, 128, 43, 64, 14, True), (43, 128, 43, 128, 12, True), (64, 128, 64, 256, 74, True),    # a short prompt
+    (65, 128, 65, 64, 14, False), (43, 256, 300, 128, 12, False), (2, 256, 129, 64, 14, False),   # longer ones, longer contexts
+    (36, 128, 100, 64, 14, True), (36, 128, 100, 128, 12, False), (36, 128, 0, 128, 12, False), (17, 64, 0, 128, 12, True),
+    (33, 128, 64, 128, 75, False), (32, 128, 64, 128, 75, True), (64, 128, 64, 128, 148, False), (64, 128, 64, 128, 149, True),
+    (64, 128, 64, 64, 112, True), (64, 128, 128, 64, 112, False), (64, 128, 128, 64, 154, True), (32, 128, 128, 64, 140, True),
+])
+def test_which_portions_are_short(max_q_len, table_keys, max_ctx_len, head_dim, ctas, short):
+    ops = bare_ops(torch.bfloat16)
+    ops.sm_count = 148
+    assert ops.short_portions(max_q_len, table_keys, max_ctx_len, head_dim, ctas) is short
+
+
+@pytest.mark.parametrize("dtype,apart", [("bfloat16", True), ("float32", False)])
+def test_a_captured_portion_holds_for_contexts_on_one_side_of_the_short_ones(dtype, apart):
+    """Two steps of the same lengths and table widths, over 40 and over 100 keys: other kernels in bfloat16."""
+    from shrike_b200.config import parse_config
+    from shrike_b200.engine.batch import StepEntry
+    from shrike_b200.engine.runner import ModelRunner
+    from shrike_b200.weights.random_init import random_tensors
+    from tests.emulated_ops import EmulatedOps
+    from tests.tiny_configs import TINY
+
+    config, ops = parse_config(TINY["C"]), EmulatedOps()
+    ops.SHORT_CONTEXT = CudaOps.SHORT_CONTEXT
+    runner = ModelRunner(config, dict(random_tensors(config, 1)), ops, "cpu", dtype, page_size=16, num_pages=24, max_slots=4)
+    keys = []
+    for start in (0, 60):
+        cache = runner.cache.open()
+        runner.cache.append(cache, 0, start + 40)
+        keys.append(runner.prepare([StepEntry(cache, [3] * 40, start, [39])]).key)
+    assert (keys[0] != keys[1]) == apart
+    cache = runner.cache.open()
+    runner.cache.append(cache, 0, 101)
+    assert runner.prepare([StepEntry(cache, [3], 100, [0])]).key == runner.prepare([StepEntry(cache, [3], 9, [0])]).key
