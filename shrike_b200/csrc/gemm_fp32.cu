@@ -465,19 +465,23 @@ int segment_length(int n, int k) {
 }
 
 // Eighths of a tile's rows (TM) for a product of M rows and `stack` slices: what an SM's CTAs cost, rounds of as many as
-// live on it (two; three of 48 rows, four of 32), the last round at least the cost of two where it is the only one (a CTA
-// alone hides nothing of its latencies) and of 1.25 behind others (its CTAs start as places fall free).  Smaller tiles
-// read more from shared memory an FMA.  The rows beyond M and the empty places of the last round are what the choice
-// avoids.  Measured, 333 rows: the 896 x 4,864 matrix 84 us with the chosen 80 rows a tile, 112 to 136 with 32, 64, 112 or
-// 128; 9,728 x 896: 182 with 112, 188 with 64, 208 with 96; 1,152 x 896: 28 with 32, 45 with 96.
+// live on it (two by their registers; three of 32 rows by their shared memory), the last round at least the cost of two where it is
+// the only one (a CTA alone hides nothing of its latencies) and of 1.25 behind others (its CTAs start as places fall free).
+// Smaller tiles read more from shared memory an FMA.  The rows beyond M and the empty places of the last round are what the
+// choice avoids.  Measured over 17 to 2,048 rows of ten matrices of 0.5B, 1.5B and 7B widths (183 products, every height
+// each): 0.7% above the best height's time on average, 12% at worst (333 rows, 2,048 x 1,536 in one slice: 164 us with 32, 147
+// with 48 rows a tile).  333 rows: the 896 x 4,864 matrix 84 us with the chosen 80 rows a tile, 112 to 136 with 32, 64, 112 or 128;
+// 1,152 x 896: 28 with 32, 45 with 96.  96 rows are slower than both neighbours (1,024 rows, 9,728 x 896: 497 us, 435 with 80).
 int tile_rows(int M, int N, int stack) {
-  constexpr int sizes[] = {16, 14, 12, 10, 8, 6, 4}, resident[] = {2, 2, 2, 2, 2, 3, 4};
-  constexpr float rate[] = {1.f, 1.f, 1.f, 1.f, 0.95f, 0.7f, 0.75f};
+  constexpr int sizes[] = {16, 14, 12, 10, 8, 4}, resident[] = {2, 2, 2, 2, 2, 3};
+  constexpr float rate[] = {1.f, 1.f, 0.9f, 1.f, 0.95f, 0.75f};
   const long long sms = shrike_device().sm_count, columns = static_cast<long long>((N + TILE_N - 1) / TILE_N) * stack;
   int best = 16;
   float least = 0.f;
-  for (int i = 0; i < 7; ++i) {
-    const long long ctas = columns * ((M + 8 * sizes[i] - 1) / (8 * sizes[i])), places = sms * resident[i];
+  for (int i = 0; i < 6; ++i) {
+    const long long rows = (M + 8LL * sizes[i] - 1) / (8 * sizes[i]);
+    if (i > 0 && rows > 65535) continue;   // more than a grid's y
+    const long long ctas = columns * rows, places = sms * resident[i];
     const long long rounds = ctas / places, rest = ctas % places, an_sm = (rest + sms - 1) / sms;
     const float alone = rounds > 0 ? 1.25f : 2.f, last = rest == 0 ? 0.f : (an_sm > alone ? an_sm : alone);
     const float cost = (rounds * resident[i] + last) * sizes[i] / rate[i];
@@ -509,8 +513,9 @@ SHRIKE_API int shrike_gemm_fp32_stack(int m, int n, int k) {
 }
 
 // `stack` > 1 (as shrike_gemm_fp32_stack says, no bias): C is [stack][M][N], one slice a run of K, to be added in order.
+// `tile` 0: the tile height that the rule above gives; n: 8 n rows.
 SHRIKE_API int shrike_gemm_fp32(const float* A, const float* W, const float* bias, float* C, int M, int N,
-                                int K, int stack, int* status, cudaStream_t stream) {
+                                int K, int stack, int tile, int* status, cudaStream_t stream) {
   using namespace fp32;
   if (M <= 0 || N <= 0) return SHRIKE_OK;
   if (K <= 0 || stack < 1) return SHRIKE_BAD_ARGUMENT;
@@ -531,15 +536,15 @@ SHRIKE_API int shrike_gemm_fp32(const float* A, const float* W, const float* bia
     if (runs > 8) return rows_of_tokens<16>(A, W, bias, C, M, N, K, length, stack, status, stream);
     return rows_of_tokens<8>(A, W, bias, C, M, N, K, length, stack, status, stream);
   }
-  switch (tile_rows(M, N, stack)) {
+  switch (tile > 0 ? tile : tile_rows(M, N, stack)) {
 #define SHRIKE_TILE(TM) case TM: return launch_tiles<TM>(A, W, bias, C, M, N, K, length, stack, status, stream)
     SHRIKE_TILE(4);
-    SHRIKE_TILE(6);
     SHRIKE_TILE(8);
     SHRIKE_TILE(10);
     SHRIKE_TILE(12);
     SHRIKE_TILE(14);
-    default: return launch_tiles<16>(A, W, bias, C, M, N, K, length, stack, status, stream);
+    SHRIKE_TILE(16);
+    default: return SHRIKE_BAD_ARGUMENT;
 #undef SHRIKE_TILE
   }
 }

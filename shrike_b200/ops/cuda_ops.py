@@ -138,6 +138,7 @@ class CudaOps:
         self._delta_scratch = None    # the delta rule's blocks of tokens: what the walk over them reads
         self._delta_runs = None       # and, where few walks are cut into runs, what those hand to one another
         self.delta_run_blocks = None  # None: the kernel library's rule; n: runs of n blocks (0: none; tests)
+        self.gemm_fp32_tile = 0  # 0: the kernel library's rule; n: tiles of 8 n rows in the 32-bit product (tests)
         self.portion_splits = 0  # 0: the kernel library's rule; n: that many key splits for portions (tests)
         self.generation = 0      # grows when the scratch moves
         self._held_stream = None
@@ -158,7 +159,7 @@ class CudaOps:
         lib.shrike_silu_mul.argtypes = [_P, _P, _I, _I, _I, _I, _P]
         lib.shrike_rope_kv_write.argtypes = [_P] * 10 + [_I] * 5 + [_LL, _I, _LL, _P]
         lib.shrike_kv_write.argtypes = [_P] * 5 + [_I, _I, _I, _LL, _P]
-        lib.shrike_gemm_fp32.argtypes = [_P, _P, _P, _P, _I, _I, _I, _I, _P, _P]
+        lib.shrike_gemm_fp32.argtypes = [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P]
         lib.shrike_gemm_fp32_stack.argtypes = [_I, _I, _I]
         lib.shrike_sample.argtypes = [_P, _P, _P, _P, _P, _P, _P, _I, _I, _P, _P]
         lib.shrike_embed_positions.argtypes = [_P, _P, _I, _P, _I, _I, _I, _P, _I, _P, _P, _I, _P]
@@ -547,8 +548,8 @@ class CudaOps:
             if stack > 1 and ((x.data_ptr() | w.data_ptr()) % 16 or stack * n * o > self.FP32_STACK_FLOATS):
                 stack = 1
             target = self._partial_stack(out, stack) if stack > 1 else out
-            _check(self.core.shrike_gemm_fp32(_ptr(x), _ptr(w), _ptr(bias), _ptr(target), n, o, k, stack, _ptr(self.status),
-                                              self._stream()), "gemm_fp32")
+            _check(self.core.shrike_gemm_fp32(_ptr(x), _ptr(w), _ptr(bias), _ptr(target), n, o, k, stack, self.gemm_fp32_tile,
+                                              _ptr(self.status), self._stream()), "gemm_fp32")
             return target
         _dense(x, torch.bfloat16, "linear input")
         _dense(w, torch.bfloat16, "linear weight")

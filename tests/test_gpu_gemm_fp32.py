@@ -61,3 +61,24 @@ def test_gemm_fp32_sums_its_runs_itself_where_their_stack_would_be_too_large():
     out = torch.empty(m, n, device=DEV)
     got = ops.linear(x, w, out, allow_partials=True)
     assert got.data_ptr() == out.data_ptr() and torch.equal(got, total)
+
+
+# every height of a tile, one row below it, at it, one and half a tile above; one run, several runs added where they lie, and
+# a stack of runs; n and k that end within a tile
+@pytest.mark.parametrize("tile", [4, 8, 10, 12, 14, 16])
+@pytest.mark.parametrize("n,k", [(257, 500), (130, 4100), (96, 900), (300, 9000)])
+def test_gemm_fp32_gives_the_same_bits_at_every_tile_height(tile, n, k):
+    ops = cuda_ops(torch.float32)
+    x, w, bias = rnd(12 * tile + 3, k, seed=tile), rnd(n, k, seed=2), rnd(n, seed=3)
+    want = torch.cat([ops.linear(part.contiguous(), w, torch.empty(len(part), n, device=DEV)) for part in x.split(16)])   # few rows
+    want_stack = [ops.linear(part.contiguous(), w, torch.empty(len(part), n, device=DEV), allow_partials=True) for part in x.split(16)]
+    ops.gemm_fp32_tile = tile
+    for m in (8 * tile - 1, 8 * tile, 8 * tile + 1, 12 * tile + 3):
+        out = torch.full((m, n), float("nan"), device=DEV)
+        assert torch.equal(ops.linear(x[:m].contiguous(), w, out), want[:m]), m
+        assert torch.equal(ops.linear(x[:m].contiguous(), w, out, bias=bias), want[:m] + bias), m
+        stack = ops.linear(x[:m].contiguous(), w, torch.empty(m, n, device=DEV), allow_partials=True)
+        assert (stack.dim() == 3) == (k > 512)
+        if stack.dim() == 3:
+            assert torch.equal(stack, torch.cat([s for s in want_stack], dim=1)[:, :m]), m
+    ops.check_status()
