@@ -46,7 +46,7 @@ struct Params {
   int max_blocks, num_heads, num_kv_heads, page_size, num_pages, window, keep_first, num_tokens, num_seqs, chunks;
   int heads_per_cta, head_groups, skip_single;
   int early_metadata;    // 1: no kernel still running writes the tables, starts and lengths: they are read before the wait
-  int aligned, kv_aligned;   // q and out lie on 16 bytes; keys and values do
+  int aligned;           // q and out lie on 16 bytes
   float scale, softcap;
 };
 
@@ -56,12 +56,10 @@ __device__ __forceinline__ void copy16(float* smem, const float* from, bool vali
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))), "l"(from),
                "r"(valid ? 16 : 0));
 }
-// The same for four elements that do not lie on 16 bytes.
-__device__ __forceinline__ void copy4_each(float* smem, const float* from, bool valid) {
-#pragma unroll
-  for (int e = 0; e < 4; ++e)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem + e))), "l"(from + e),
-                 "r"(valid ? 4 : 0));
+// The same for an element.
+__device__ __forceinline__ void copy4(float* smem, const float* from, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))), "l"(from),
+               "r"(valid ? 4 : 0));
 }
 
 // One row's running softmax.  Explicit roundings: every use of the row gives the same bits.
@@ -120,7 +118,8 @@ __device__ __forceinline__ void add_values(float (&acc)[RI][COLS * 4], const flo
 }
 
 // Rows: the tokens [token, token + count) of sequence `seq`, heads [head, head + heads) of one kv head; chunks [c_begin, c_end).
-template <int R>
+// WIDE: keys and values lie on 16 bytes.
+template <int R, bool WIDE>
 __device__ void attend(const Params& p, float* smem, int seq, int token, int count, int head, int heads, int kv_head, int c_begin, int c_end,
                        bool whole) {
   constexpr int RI = R / 16;
@@ -158,12 +157,15 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
       const int r = i / (D / 4), c = i % (D / 4);
       const long long row = row_s[walked & 3][r];
       const size_t at = row >= 0 ? static_cast<size_t>(row) * key_stride + static_cast<size_t>(kv_head) * D + c * 4 : 0;
-      if (p.kv_aligned) {
+      if (WIDE) {
         copy16(k_to + r * ROW + c * 4, p.k_cache + at, row >= 0);
         copy16(v_to + r * ROW + c * 4, p.v_cache + at, row >= 0);
       } else {
-        copy4_each(k_to + r * ROW + c * 4, p.k_cache + at, row >= 0);
-        copy4_each(v_to + r * ROW + c * 4, p.v_cache + at, row >= 0);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          copy4(k_to + r * ROW + c * 4 + e, p.k_cache + at + e, row >= 0);
+          copy4(v_to + r * ROW + c * 4 + e, p.v_cache + at + e, row >= 0);
+        }
       }
     }
     asm volatile("cp.async.commit_group;\n" ::);
@@ -326,6 +328,7 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
 }
 
 // Single tokens: grid (chunks, kv heads times head groups, sequences).
+template <bool WIDE>
 __global__ void __launch_bounds__(THREADS) single_kernel(const Params p) {
   extern __shared__ __align__(16) float smem[];
   let_dependents_start();
@@ -339,7 +342,7 @@ __global__ void __launch_bounds__(THREADS) single_kernel(const Params p) {
   }
   const int share = p.num_heads / p.num_kv_heads, head = kv_head * share + group * p.heads_per_cta;
   const int heads = min(p.heads_per_cta, share - group * p.heads_per_cta);
-  attend<16>(p, smem, seq, token, 1, head, heads, kv_head, blockIdx.x, p.chunks > 1 ? blockIdx.x + 1 : 0x7ffffff, p.chunks == 1);
+  attend<16, WIDE>(p, smem, seq, token, 1, head, heads, kv_head, blockIdx.x, p.chunks > 1 ? blockIdx.x + 1 : 0x7ffffff, p.chunks == 1);
 }
 
 // A warp a (sequence, head): the chunks of a single token's row, in ascending order.
@@ -378,7 +381,7 @@ __global__ void __launch_bounds__(128) merge_kernel(const Params p) {
 }
 
 // Portions: grid (tiles of tokens of the flat batch, kv heads times head groups); a tile's sequences one after another.
-template <int R>
+template <int R, bool WIDE = true>
 __global__ void __launch_bounds__(THREADS) portions_kernel(const Params p) {
   extern __shared__ __align__(16) float smem[];
   let_dependents_start();
@@ -394,7 +397,7 @@ __global__ void __launch_bounds__(THREADS) portions_kernel(const Params p) {
     const int stop = min(end, p.q_start[seq + 1]);
     if (!p.skip_single || p.q_start[seq + 1] - p.q_start[seq] > 1) {
       __syncthreads();   // the sequence before is done with shared memory
-      attend<R>(p, smem, seq, token, stop - token, head, heads, kv_head, 0, 0x7ffffff, true);
+      attend<R, WIDE>(p, smem, seq, token, stop - token, head, heads, kv_head, 0, 0x7ffffff, true);
     }
     token = stop > token ? stop : token + 1;
   }
@@ -451,27 +454,34 @@ SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, c
   p.skip_single = has_single;
   p.early_metadata = early_metadata;
   p.aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  p.kv_aligned = ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
   p.scale = scale;
   p.softcap = softcap;
+  const bool wide = ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
   const int share = num_heads / num_kv_heads;
-  static PerDevice raised[4];
-  int rc = shrike_raise_smem(raised[0], single_kernel, shared_floats<16>() * 4);
+  static PerDevice raised[6];
+  int rc = shrike_raise_smem(raised[0], single_kernel<true>, shared_floats<16>() * 4);
+  if (rc == 0) rc = shrike_raise_smem(raised[4], single_kernel<false>, shared_floats<16>() * 4);
+  if (rc == 0) rc = shrike_raise_smem(raised[5], portions_kernel<16, false>, shared_floats<16>() * 4);
   if (rc == 0) rc = shrike_raise_smem(raised[1], portions_kernel<16>, shared_floats<16>() * 4);
   if (rc == 0) rc = shrike_raise_smem(raised[2], portions_kernel<32>, shared_floats<32>() * 4);
   if (rc == 0) rc = shrike_raise_smem(raised[3], portions_kernel<64>, shared_floats<64>() * 4);
   if (rc != 0) return rc;
   if (has_portions) {
-    // 64 rows a CTA read a key from shared memory for 64 rows, 16 only for 16; but tiles of 64 rows that do not fill the
-    // device twice leave it waiting for the last tokens' CTAs, which walk every key
+    // 64 rows a CTA read a key from shared memory for 64 rows, 16 only for 16; but fewer of them live on an SM (two for heads of
+    // 64, one for wider ones; of 16 rows three, two and one), and where they are few the device waits for the last tokens' CTAs,
+    // which walk every key.  Measured, us with 16, 32 and 64 rows: 14 heads of 64 over 2: 100 tokens 12.8, 15.6, 22.6; 333 tokens
+    // 43.5, 43.1, 54.1; 1,500 tokens 371, 285, 300; 28 heads of 128 over 4: 100 tokens 24.4, 23.3, 31.6; 400 tokens 131, 95.7,
+    // 91.3; 1,500 tokens 1,402, 881, 771.  What is chosen is within 7% of the best at 17 to 1,500 tokens of five head layouts.
+    // Pages that do not lie on 16 bytes have the smallest form alone.
     const long long rows = static_cast<long long>(num_tokens) * share, sms = shrike_device().sm_count;
-    const int a_cta = (rows + 63) / 64 * num_kv_heads >= 2 * sms ? 64 : ((rows + 31) / 32 * num_kv_heads * 5 >= 4 * sms ? 32 : 16);
+    const int a_cta = !wide ? 16 : (rows + 63) / 64 * num_kv_heads >= 2 * sms ? 64 : ((rows + 31) / 32 * num_kv_heads * 5 >= 4 * sms ? 32 : 16);
     p.heads_per_cta = share < a_cta ? share : a_cta;
     p.head_groups = (share + p.heads_per_cta - 1) / p.heads_per_cta;
     const int a_tile = a_cta / p.heads_per_cta;
     if (static_cast<long long>(num_kv_heads) * p.head_groups > 65535) return SHRIKE_BAD_ARGUMENT;
     const dim3 grid((num_tokens + a_tile - 1) / a_tile, num_kv_heads * p.head_groups);
-    const cudaError_t err = a_cta == 64   ? launch_dependent(portions_kernel<64>, grid, dim3(THREADS), shared_floats<64>() * 4, stream, p)
+    const cudaError_t err = !wide         ? launch_dependent(portions_kernel<16, false>, grid, dim3(THREADS), shared_floats<16>() * 4, stream, p)
+                            : a_cta == 64   ? launch_dependent(portions_kernel<64>, grid, dim3(THREADS), shared_floats<64>() * 4, stream, p)
                             : a_cta == 32 ? launch_dependent(portions_kernel<32>, grid, dim3(THREADS), shared_floats<32>() * 4, stream, p)
                                           : launch_dependent(portions_kernel<16>, grid, dim3(THREADS), shared_floats<16>() * 4, stream, p);
     if (err != cudaSuccess) return static_cast<int>(err);
@@ -480,7 +490,7 @@ SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, c
     p.heads_per_cta = share < 16 ? share : 16;
     p.head_groups = (share + p.heads_per_cta - 1) / p.heads_per_cta;
     if (static_cast<long long>(num_kv_heads) * p.head_groups > 65535) return SHRIKE_BAD_ARGUMENT;
-    cudaError_t err = launch_dependent(single_kernel, dim3(chunks, num_kv_heads * p.head_groups, num_seqs), dim3(THREADS),
+    cudaError_t err = launch_dependent(wide ? single_kernel<true> : single_kernel<false>, dim3(chunks, num_kv_heads * p.head_groups, num_seqs), dim3(THREADS),
                                        shared_floats<16>() * 4, stream, p);
     if (err == cudaSuccess && chunks > 1)
       err = launch_dependent(merge_kernel, dim3((num_seqs * num_heads + 3) / 4), dim3(128), 0, stream, p);
