@@ -75,6 +75,28 @@ def test_sum_norm_adds_pending_sums_and_norms(dtype, n, width, stacks, row):
     close(out, want, loose, "normed sum")
 
 
+@pytest.mark.parametrize("n,width,stacks", [(5, 256, (3,)), (70, 96, (3, 1, 8)), (3, 50, (2, 2)), (2, 6000, (16, 16, 16, 16)), (300, 1000, (7, 16))])
+def test_sum_norm_gives_a_stack_the_bits_of_its_sum(n, width, stacks):
+    """The slices of a product that leaves as a stack, added in order, are what the product would have left by itself."""
+    ops = cuda_ops(torch.float32)
+    g = torch.Generator().manual_seed(n + width)
+    weight = (1 + 0.1 * torch.randn(width, generator=g)).cuda()
+    resid = torch.randn(n, width, generator=g).cuda()
+    stack = [torch.randn(p, n, width, generator=g).cuda() for p in stacks]
+    plain = []
+    for slices in stack:
+        total = slices[0].clone()
+        for one in slices[1:]:
+            total += one
+        plain.append(total)
+    results = []
+    for terms in (stack, plain):
+        at, out = resid.clone(), torch.empty(n, width, device="cuda")
+        ops.sum_norm(at, [(t, 0.4 + 0.3 * i) for i, t in enumerate(terms)], weight, 1e-6, out)
+        results.append((at, out))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n,heads,vdim,padded,partials", [(1, 3, 16, 16, 1), (9, 4, 24, 32, 3), (70, 2, 128, 128, 1), (5, 3, 5, 16, 2), (300, 6, 40, 48, 1)])
 def test_gate_per_element(dtype, n, heads, vdim, padded, partials):
