@@ -35,7 +35,7 @@ constexpr int PLAIN_THREADS = 256;
 
 __global__ void __launch_bounds__(PLAIN_THREADS)
 plain_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-             float* __restrict__ C, int M, int N, int K, int vec_ok, int segment_length) {
+             float* __restrict__ C, int M, int N, int K, int segment_length) {
   __shared__ __align__(16) float a_tile[BK][BM + 4];
   __shared__ __align__(16) float w_tile[BK][BN + 4];
   let_dependents_start();
@@ -65,23 +65,13 @@ plain_kernel(const float* __restrict__ A, const float* __restrict__ W, const flo
     const int am = m0 + load_row, wn = n0 + load_row;
     if (am < M) {
       const float* src = A + static_cast<size_t>(am) * K + k;
-      if (vec_ok && k + 3 < K) {
-        const float4 v = *reinterpret_cast<const float4*>(src);
-        a_reg[0] = v.x; a_reg[1] = v.y; a_reg[2] = v.z; a_reg[3] = v.w;
-      } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) if (k + i < K) a_reg[i] = src[i];
-      }
+      for (int i = 0; i < 4; ++i) if (k + i < K) a_reg[i] = src[i];
     }
     if (wn < N) {
       const float* src = W + static_cast<size_t>(wn) * K + k;
-      if (vec_ok && k + 3 < K) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(src));
-        w_reg[0] = v.x; w_reg[1] = v.y; w_reg[2] = v.z; w_reg[3] = v.w;
-      } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) if (k + i < K) w_reg[i] = __ldg(src + i);
-      }
+      for (int i = 0; i < 4; ++i) if (k + i < K) w_reg[i] = __ldg(src + i);
     }
     __syncthreads();  // the previous tile has been consumed
 #pragma unroll
@@ -454,9 +444,10 @@ int launch_tiles(const float* A, const float* W, const float* bias, float* C, in
   return err == cudaSuccess ? shrike_launch_status() : static_cast<int>(err);
 }
 
-// Elements of a run of K: a multiple of 32.  A matrix is cut into as many runs as give every SM two warps of 64 rows when a
-// few tokens are multiplied (1.5B widths, 3 tokens, the 1,536 x 8,960 matrix: 22.5 us with eight runs of 1,120); never shorter
-// than a hundred elements or so, for every run of a prompt's product is one more addition to its result.
+// Elements of a run of K: a multiple of 32.  A matrix is cut into as many runs as give every SM of a B200 two warps of 64 rows when
+// a few tokens are multiplied (the number of SMs is written out: it fixes the order of the sums, which is the matrix's alone; 1.5B
+// widths, 3 tokens, the 1,536 x 8,960 matrix: 22.5 us with eight runs of 1,120, 15.3 with the sixteen of 576 that this gives); never
+// shorter than a hundred elements or so, for every run of a prompt's product is one more addition to its result.
 int segment_length(int n, int k) {
   const int most = k < 512 ? 1 : (k < 1024 ? 4 : (k < 8192 ? 8 : 16));
   int runs = 1;
@@ -525,8 +516,7 @@ SHRIKE_API int shrike_gemm_fp32(const float* A, const float* W, const float* bia
   if (!aligned) {
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return SHRIKE_BAD_ARGUMENT;
-    plain_kernel<<<grid, PLAIN_THREADS, 0, stream>>>(A, W, bias, C, M, N, K, K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
-                                                     reinterpret_cast<uintptr_t>(W) % 16 == 0, length);
+    plain_kernel<<<grid, PLAIN_THREADS, 0, stream>>>(A, W, bias, C, M, N, K, length);
     return shrike_launch_status();
   }
   if (M <= 16) {
