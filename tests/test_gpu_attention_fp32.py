@@ -24,7 +24,7 @@ def attention(ops, case, rows, q_start, ctx_len, seq_of, table, heads, kv_heads,
     return out
 
 
-# contexts around a tile of 32 and a chunk of 128 keys; shared heads below, at and above the 16 and 64 rows of a CTA
+# contexts around a tile of 32 and a chunk of 64 keys; shared heads below, at and above the 16 and 64 rows of a CTA
 @pytest.mark.parametrize("heads,kv_heads,dim,page", [(7, 1, 128, 16), (16, 1, 64, 16), (17, 1, 48, 5), (66, 1, 16, 8), (4, 2, 256, 16)])
 @pytest.mark.parametrize("options", [{}, {"window": 40}, {"window": 40, "keep_first": 5}, {"chunk": 48}, {"softcap": 3.0, "sinks": True}])
 def test_fp32_attention_gives_a_token_the_same_bits_in_a_prompt_and_alone(heads, kv_heads, dim, page, options):
@@ -32,7 +32,7 @@ def test_fp32_attention_gives_a_token_the_same_bits_in_a_prompt_and_alone(heads,
     options = dict(options)
     if options.pop("sinks", False):
         options["sinks"] = rnd(heads, seed=9)
-    ctx_lens = [1, 31, 33, 127, 128, 129, 300, 517]
+    ctx_lens = [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 300, 517]
     case = paged_case(torch.float32, heads, kv_heads, dim, page, ctx_lens, ctx_lens, seed=heads)
     whole = attention(ops, case, case["q"], case["q_start"], case["ctx_len"], case["seq_of"], case["table"], heads, kv_heads, dim, ctx_lens, **options)
     assert torch.isfinite(whole).all()

@@ -57,3 +57,53 @@ def test_own_values_are_as_close_to_float64_as_on_the_mma_kernel(q_len, ctx_len,
         ops.check_status()
         errors[tensor_cores] = float((out.double() - want).norm() / want.norm())
     assert errors[True] <= 1.01 * errors[False], errors
+
+
+# what the launch accepts beside a window, each where a step of 64 keys, a tile of 128 and the last query tile end; the oracle in float64
+@pytest.mark.parametrize("kv_heads,heads", [(1, 3), (2, 4)])
+@pytest.mark.parametrize("options", [{}, {"sinks": True}, {"softcap": 5.0}, {"slopes": True}, {"window": 70, "keep_first": 5},
+                                     {"window": 130, "keep_first": 129, "sinks": True}, {"chunk": 96}, {"softcap": 3.0, "slopes": True, "window": 200}])
+@pytest.mark.parametrize("ctx_lens,q_lens,splits", [([129, 66, 1], [129, 65, 1], 0), ([400], [300], 3)])
+def test_own_values_with_everything_a_score_can_have(kv_heads, heads, options, ctx_lens, q_lens, splits):
+    ops = cuda_ops(torch.bfloat16)
+    dim, page = 256, 16
+    options = dict(options)
+    window, keep, chunk, cap = options.get("window"), options.get("keep_first", 0), options.get("chunk"), options.get("softcap")
+    generator = torch.Generator().manual_seed(heads)
+    sinks = torch.randn(heads, generator=generator).cuda() if options.pop("sinks", False) else None
+    slopes = torch.rand(heads, generator=generator).mul(0.05).cuda() if options.pop("slopes", False) else None
+    case = paged_case(torch.bfloat16, heads, kv_heads, dim, page, ctx_lens, q_lens, seed=heads + len(ctx_lens))
+    ops.portion_splits = splits
+    plan = ops.attention_plan(heads, kv_heads, dim, len(ctx_lens), case["table"].shape[1], page, max(q_lens), min(q_lens), sum(q_lens), list(q_lens),
+                              keep_first=keep, own_values=True, max_ctx_len=max(ctx_lens))
+    assert plan.tc_portions, "the case is meant for the tensor-core kernel"
+    out = torch.full_like(case["q"], float("nan"))
+    options.pop("window", None)
+    ops.paged_attention(case["q"], case["keys"], case["keys"], case["table"], case["q_start"], case["ctx_len"], case["seq_of"], heads, kv_heads, dim,
+                        dim ** -0.5, window, out, max_q_len=max(q_lens), max_ctx_len=max(ctx_lens), min_q_len=min(q_lens), q_lens=list(q_lens),
+                        sinks=sinks, slopes=slopes, **options)
+    ops.check_status()
+    want = []
+    for (q, k, _), n in zip(case["seqs"], q_lens):
+        total = len(q)
+        position, key = torch.arange(total - n, total, device="cuda")[:, None], torch.arange(total, device="cuda")[None]
+        hidden = key > position
+        if window:
+            hidden = hidden | ((position - key >= window) & (key >= keep))
+        if chunk:
+            hidden = hidden | (position // chunk != key // chunk)
+        rows = []
+        for a in range(heads):
+            held = k[:, a * kv_heads // heads].double().cuda()
+            score = q[total - n:, a].double().cuda() @ held.T * dim ** -0.5
+            if cap:
+                score = cap * torch.tanh(score / cap)
+            if slopes is not None:
+                score = score - slopes[a].double() * (position - key)
+            score = score.masked_fill(hidden, float("-inf"))
+            if sinks is not None:
+                score = torch.cat([score, sinks[a].double().expand(n, 1)], dim=1)
+            rows.append(torch.softmax(score, dim=1)[:, :total] @ held)
+        want.append(torch.stack(rows, dim=1).reshape(n, heads * dim))
+    # probabilities rounded to bfloat16 (2^-9 each, relative) and one rounding of outputs of order one, as above
+    assert torch.isfinite(out).all() and (out.double() - torch.cat(want)).abs().max() < 2e-2

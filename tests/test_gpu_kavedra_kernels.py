@@ -109,6 +109,20 @@ def test_decayed_scan_over_unequal_sequences_skips_padding():
         close(state[slot].view(heads, dim, vdim) / big, final / big, 1e-5, f"state of sequence {index}")
 
 
+@pytest.mark.parametrize("heads,dim,vdim", [(1, 377, 40), (2, 420, 24), (1, 440, 72)])
+def test_heads_that_fit_the_chunked_form_since_it_holds_less(heads, dim, vdim):
+    """Heads of 377 rows and more came to the runs of tokens when their products gave up an array in shared memory."""
+    ops = cuda_ops(torch.float32)
+    decays = (0.98, 1.0)[:heads]
+    fused, want, final = scan_case(heads, dim, vdim, 150, dim, decays)
+    size, big = max(1.0, float(want.abs().max())), max(1.0, float(final.abs().max()))
+    state = torch.zeros(1, heads, -(-dim * vdim // 4) * 4, dtype=torch.float32, device=DEV)
+    for cuts, walk in (([150], False), ([150], True), ([33, 64, 53], False)):
+        state.zero_()
+        close(run_scan(ops, fused, decays, state, 0, cuts, heads, dim, vdim, walk=walk) / size, want / size, 2e-5, f"cuts {cuts}")
+        close(state[0, :, : dim * vdim].view(heads, dim, vdim) / big, final / big, 1e-5, "the state left behind")
+
+
 @pytest.mark.parametrize("heads,dim,vdim,cut", [(2, 64, 48, 1), (1, 16, 16, 1), (4, 128, 128, 1), (1, 520, 64, 1), (2, 32, 48, 3)])
 def test_scans_in_a_row_on_one_state_without_anything_between_them(heads, dim, vdim, cut):
     """Launches that follow one another directly: each reads the state that the one before it leaves."""
