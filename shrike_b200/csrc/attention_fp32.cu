@@ -11,6 +11,8 @@
 // 32, a key that the row does not see adds nothing, and every 64 keys (a chunk) are an attention of their own whose
 // (maximum, sum, outputs) are merged into the row's in ascending order.  So the chunks of a few decoding requests can run on
 // CTAs of their own (R = 16, grid over chunks, `merge_kernel`) and give the bits of a prompt's CTA that walks them all (R = 64).
+// Where such tiles would stay nearly empty (few keys, heads that share their keys with nobody) a warp takes a row (`warps_kernel`),
+// with every operation in the same order.
 //
 // Measured (one B200; a warp a row before): 3 requests of 200 tokens, 12 heads of 128 over 2: 83.6 us a layer before, 13.0
 // and 3.6 for the merge now; 333 tokens, 14 heads of 64 over 2: 123 us before, 37 now.
@@ -55,11 +57,6 @@ template <int R> constexpr size_t shared_floats() { return static_cast<size_t>(R
 __device__ __forceinline__ void copy16(float* smem, const float* from, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))), "l"(from),
                "r"(valid ? 16 : 0));
-}
-// The same for an element.
-__device__ __forceinline__ void copy4(float* smem, const float* from, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))), "l"(from),
-               "r"(valid ? 4 : 0));
 }
 
 // One row's running softmax.  Explicit roundings: every use of the row gives the same bits.
@@ -118,8 +115,7 @@ __device__ __forceinline__ void add_values(float (&acc)[RI][COLS * 4], const flo
 }
 
 // Rows: the tokens [token, token + count) of sequence `seq`, heads [head, head + heads) of one kv head; chunks [c_begin, c_end).
-// WIDE: keys and values lie on 16 bytes.
-template <int R, bool WIDE>
+template <int R>
 __device__ void attend(const Params& p, float* smem, int seq, int token, int count, int head, int heads, int kv_head, int c_begin, int c_end,
                        bool whole) {
   constexpr int RI = R / 16;
@@ -157,16 +153,8 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
       const int r = i / (D / 4), c = i % (D / 4);
       const long long row = row_s[walked & 3][r];
       const size_t at = row >= 0 ? static_cast<size_t>(row) * key_stride + static_cast<size_t>(kv_head) * D + c * 4 : 0;
-      if (WIDE) {
-        copy16(k_to + r * ROW + c * 4, p.k_cache + at, row >= 0);
-        copy16(v_to + r * ROW + c * 4, p.v_cache + at, row >= 0);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          copy4(k_to + r * ROW + c * 4 + e, p.k_cache + at + e, row >= 0);
-          copy4(v_to + r * ROW + c * 4 + e, p.v_cache + at + e, row >= 0);
-        }
-      }
+      copy16(k_to + r * ROW + c * 4, p.k_cache + at, row >= 0);
+      copy16(v_to + r * ROW + c * 4, p.v_cache + at, row >= 0);
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
@@ -328,7 +316,6 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
 }
 
 // Single tokens: grid (chunks, kv heads times head groups, sequences).
-template <bool WIDE>
 __global__ void __launch_bounds__(THREADS) single_kernel(const Params p) {
   extern __shared__ __align__(16) float smem[];
   let_dependents_start();
@@ -342,7 +329,7 @@ __global__ void __launch_bounds__(THREADS) single_kernel(const Params p) {
   }
   const int share = p.num_heads / p.num_kv_heads, head = kv_head * share + group * p.heads_per_cta;
   const int heads = min(p.heads_per_cta, share - group * p.heads_per_cta);
-  attend<16, WIDE>(p, smem, seq, token, 1, head, heads, kv_head, blockIdx.x, p.chunks > 1 ? blockIdx.x + 1 : 0x7ffffff, p.chunks == 1);
+  attend<16>(p, smem, seq, token, 1, head, heads, kv_head, blockIdx.x, p.chunks > 1 ? blockIdx.x + 1 : 0x7ffffff, p.chunks == 1);
 }
 
 // A warp a (sequence, head): the chunks of a single token's row, in ascending order.
@@ -381,7 +368,7 @@ __global__ void __launch_bounds__(128) merge_kernel(const Params p) {
 }
 
 // Portions: grid (tiles of tokens of the flat batch, kv heads times head groups); a tile's sequences one after another.
-template <int R, bool WIDE = true>
+template <int R>
 __global__ void __launch_bounds__(THREADS) portions_kernel(const Params p) {
   extern __shared__ __align__(16) float smem[];
   let_dependents_start();
@@ -397,11 +384,121 @@ __global__ void __launch_bounds__(THREADS) portions_kernel(const Params p) {
     const int stop = min(end, p.q_start[seq + 1]);
     if (!p.skip_single || p.q_start[seq + 1] - p.q_start[seq] > 1) {
       __syncthreads();   // the sequence before is done with shared memory
-      attend<R, WIDE>(p, smem, seq, token, stop - token, head, heads, kv_head, 0, 0x7ffffff, true);
+      attend<R>(p, smem, seq, token, stop - token, head, heads, kv_head, 0, 0x7ffffff, true);
     }
     token = stop > token ? stop : token + 1;
   }
   if (p.early_metadata) wait_for_previous();
+}
+
+// A warp a row: short contexts, and rows that share their keys with nobody, for which a CTA's tiles stay nearly empty.  A lane
+// forms a key's score, then the warp walks the tile's keys, a lane D / 32 columns.  Every operation and its order are those of
+// `attend`, so are the bits.  `which`: 0 every token, 1 those of entries of one token, 2 the others.  WIDE: keys lie on 16 bytes.
+constexpr int WARPS = 4;
+template <bool WIDE>
+__global__ void __launch_bounds__(WARPS * 32) warps_kernel(const Params p, int which) {
+  __shared__ __align__(16) float q_s[WARPS][D];
+  let_dependents_start();
+  if (!p.early_metadata) wait_for_previous();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long work = static_cast<long long>(blockIdx.x) * WARPS + warp;
+  const int token = static_cast<int>(work / p.num_heads), head = static_cast<int>(work % p.num_heads);
+  const int seq = token < p.num_tokens ? p.seq_of_token[token] : 0;
+  const int start = p.q_start[seq], q_len = p.q_start[seq + 1] - start;
+  if (token >= p.num_tokens || (which == 1 && q_len != 1) || (which == 2 && q_len == 1)) {
+    if (p.early_metadata) wait_for_previous();
+    return;
+  }
+  constexpr int OWN = (D + 31) / 32, AHEAD = OWN <= 4 ? 4 : 2;   // columns of a lane; keys whose values are on their way together
+  const int position = p.ctx_len[seq] - q_len + (token - start), first = first_visible_key(position, p.window);
+  const int kept = p.window > 0 ? min(p.keep_first, first) : 0;
+  const int* table = p.block_table + static_cast<size_t>(seq) * p.max_blocks;
+  const size_t key_stride = static_cast<size_t>(p.num_kv_heads) * D, column = static_cast<size_t>(head / (p.num_heads / p.num_kv_heads)) * D;
+  const float slope = p.slopes != nullptr ? p.slopes[head] : 0.f;
+  if (p.early_metadata) wait_for_previous();
+  const float* q = p.q + (static_cast<size_t>(token) * p.num_heads + head) * D;
+  for (int d = lane; d < D; d += 32) q_s[warp][d] = q[d];
+  __syncwarp();
+  Running all{-INFINITY, 0.f}, run{-INFINITY, 0.f};
+  float total[OWN], acc[OWN];
+#pragma unroll
+  for (int i = 0; i < OWN; ++i) total[i] = acc[i] = 0.f;
+  const int tile_end = position / KEYS + 1;
+  auto next_tile = [&](int tile) { return tile * KEYS < kept || tile >= first / KEYS ? tile : first / KEYS; };
+  for (int tile = next_tile(0); position >= 0 && tile < tile_end;) {
+    const int key = tile * KEYS + lane, block = key / p.page_size;
+    const int page = key <= position && block < p.max_blocks ? table[block] : -1;
+    const long long row = page >= 0 && page < p.num_pages ? static_cast<long long>(page) * p.page_size + (key - block * p.page_size) : -1;
+    bool seen = row >= 0 && (key >= first || (p.window > 0 && key < p.keep_first));
+    float score = 0.f;
+    if (seen) {
+      const float* k = p.k_cache + static_cast<size_t>(row) * key_stride + column;
+#pragma unroll 8
+      for (int c = 0; c < D; c += 4) {
+        float4 b;
+        if (WIDE) b = *reinterpret_cast<const float4*>(k + c);
+        else b = make_float4(k[c], k[c + 1], k[c + 2], k[c + 3]);
+        const float4 a = *reinterpret_cast<const float4*>(&q_s[warp][c]);
+        score = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, score))));
+      }
+      score = __fmul_rn(score, p.scale);
+      if (p.softcap > 0.f) score = __fmul_rn(p.softcap, tanhf(__fdiv_rn(score, p.softcap)));
+      if (p.slopes != nullptr) score = __fmaf_rn(-slope, static_cast<float>(position - key), score);
+    }
+    const float now = fmaxf(run.top, warp_max(seen ? score : -INFINITY));
+    seen = seen && now != -INFINITY;   // nothing but -inf so far: the keys weigh nothing
+    const float weight = seen ? expf(__fadd_rn(score, -now)) : 0.f;
+    float sum = weight;
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, offset));
+    if (now != -INFINITY) {
+      const float shrink = expf(__fadd_rn(run.top, -now));
+      run.sum = __fadd_rn(__fmul_rn(run.sum, shrink), sum);
+      run.top = now;
+#pragma unroll
+      for (int i = 0; i < OWN; ++i) acc[i] = __fmul_rn(acc[i], shrink);
+    }
+    for (unsigned left = __ballot_sync(0xffffffffu, seen); left != 0;) {   // the keys that the row sees, in ascending order
+      float v[AHEAD][OWN], w[AHEAD];
+      int count = 0;
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a) {
+        const int j = left != 0 ? __ffs(left) - 1 : 0;
+        w[a] = __shfl_sync(0xffffffffu, weight, j);
+        const long long row_j = __shfl_sync(0xffffffffu, row, j);
+        if (left != 0) {
+          const float* from = p.v_cache + static_cast<size_t>(row_j) * key_stride + column;
+#pragma unroll
+          for (int i = 0; i < OWN; ++i) v[a][i] = lane + 32 * i < D ? from[lane + 32 * i] : 0.f;
+          count = a + 1;
+          left &= left - 1;
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a)
+        if (a < count) {
+#pragma unroll
+          for (int i = 0; i < OWN; ++i) acc[i] = fmaf(w[a], v[a][i], acc[i]);
+        }
+    }
+    const int following = next_tile(tile + 1);
+    if (following >= tile_end || following / (CHUNK / KEYS) != tile / (CHUNK / KEYS)) {   // a chunk ends: it joins the row
+      if (run.top != -INFINITY) {
+        const float2 f = join(all, run);
+#pragma unroll
+        for (int i = 0; i < OWN; ++i) total[i] = joined(total[i], f.x, acc[i], f.y);
+      }
+      run = Running{-INFINITY, 0.f};
+#pragma unroll
+      for (int i = 0; i < OWN; ++i) acc[i] = 0.f;
+    }
+    tile = following;
+  }
+  const float inverse = finish(all, p.sinks, head);
+  float* to = p.out + (static_cast<size_t>(token) * p.num_heads + head) * D;
+#pragma unroll
+  for (int i = 0; i < OWN; ++i)
+    if (lane + 32 * i < D) to[lane + 32 * i] = total[i] * inverse;
 }
 
 }  // namespace attn32
@@ -411,9 +508,34 @@ SHRIKE_API int shrike_attention_head_dim() { return attn32::D; }
 // Keys of a chunk: single tokens want chunks = ceil(table width * page size / this) and, above one, that much scratch.
 SHRIKE_API int shrike_attention_fp32_chunk() { return attn32::CHUNK; }
 
-// `has_single`: single tokens run on CTAs per chunk (scratch: float32 [seqs][heads][chunks][head size + 2]); `has_portions`: the
-// entries of more than one token (all entries when there is no `has_single`) run on tiles of tokens.  `early_metadata` 1: the
-// caller knows that whatever wrote the block table, q_start, ctx_len and seq_of_token has finished (a copy, or an earlier step).
+// How single tokens (portions) should run: 1 the CTA forms, 2 a warp a row.  `keys`: what the block tables can hold, or what is
+// known to be the longest context.
+//
+// A CTA's sixteen rows are the heads of one kv head; with one or two of them it multiplies mostly zeros, which costs nothing
+// while SMs are idle, and many such pairs are quicker with a warp a row.  Measured, us with tiles and with warps: 8 heads of 64 over 8,
+// 64 requests: 20 keys 12.3 and 6.0, 128 keys 32.0 and 22.0, 1,000 keys 195 and 306; 128 requests: 1,000 keys 381 and 314; 32 heads
+// of 128 over 32: 8 requests 20 keys 11.6 and 9.0, 128 keys 30.5 and 35.9; 32 requests 128 keys 95.8 and 77.4, 1,000 keys 704 and 546;
+// 16 heads of 64 over 8, 128 requests: 128 keys 51.6 and 49.4.  From three heads a kv head on only the first few keys are quicker
+// that way (12 heads of 128 over 2, 64 requests: 3 keys 9.7 and 6.4, 20 keys 9.9 and 9.4, 64 keys 15.9 and 21.7).
+SHRIKE_API int shrike_attention_fp32_single_form(int num_seqs, int num_heads, int num_kv_heads, int keys) {
+  if (keys <= 8) return 2;
+  if (num_kv_heads <= 0 || num_heads / num_kv_heads > 2) return 1;
+  const long long pairs = static_cast<long long>(num_seqs) * num_kv_heads;
+  return pairs >= 1024 || (pairs >= 256 && keys <= 128) ? 2 : 1;
+}
+// A CTA takes its tokens' sequences one after another: with entries of few rows, several of them to a tile of sixteen (us with tiles and
+// with warps: 8 heads of 64 over 8: 8 entries of 2 tokens 26.8 and 4.1, 32 of 4 tokens over 60 keys 23.1 and 14.2, of 8 tokens over
+// 200 keys 44.7 and 73.9; 16 heads over 8: 100 entries of 3 tokens 55.9 and 26.7 [6 rows], 32 of 4 over 60 keys 15.3 and 24.4 [8 rows]).
+SHRIKE_API int shrike_attention_fp32_portion_form(int num_tokens, int num_seqs, int num_heads, int num_kv_heads) {
+  if (num_kv_heads <= 0) return 1;
+  return num_seqs > 1 && static_cast<long long>(num_tokens) * (num_heads / num_kv_heads) <= 6LL * num_seqs ? 2 : 1;
+}
+
+// `has_single` 1: single tokens run on CTAs per chunk (scratch: float32 [seqs][heads][chunks][head size + 2]); `has_portions` 1: the
+// entries of more than one token (all entries when there is no `has_single`) run on tiles of tokens; 2: a warp a row.  All give
+// the same bits.  Keys or values that do not lie on 16 bytes, and more sequences or kv heads than a grid has places for, go to
+// the warps.  `early_metadata` 1: the caller knows that whatever wrote the block table, q_start, ctx_len and seq_of_token has
+// finished (a copy, or an earlier step).
 SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
                                            int max_blocks, const int* q_start, const int* ctx_len, const int* seq_of_token,
                                            int num_tokens, int num_seqs, int num_heads, int num_kv_heads, int page_size, int num_pages,
@@ -423,12 +545,8 @@ SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, c
   using namespace attn32;
   if (num_tokens <= 0) return SHRIKE_OK;
   if (keep_first < 0 || num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads || page_size <= 0 || max_blocks <= 0 || num_seqs <= 0 ||
-      chunks < 1 || (has_single && chunks > 1 && scratch == nullptr))
+      chunks < 1 || (has_single == 1 && chunks > 1 && scratch == nullptr))
     return SHRIKE_BAD_ARGUMENT;
-  if (num_seqs > 65535) {   // more than a grid's z: tiles of tokens serve entries of any length, with the same bits
-    has_single = 0;
-    has_portions = 1;
-  }
   Params p = {};
   p.q = static_cast<const float*>(q);
   p.k_cache = static_cast<const float*>(k_cache);
@@ -456,41 +574,46 @@ SHRIKE_API int shrike_paged_attention_fp32(const void* q, const void* k_cache, c
   p.aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   p.scale = scale;
   p.softcap = softcap;
-  const bool wide = ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
+  const bool wide_keys = (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0, wide = wide_keys && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0;
   const int share = num_heads / num_kv_heads;
-  static PerDevice raised[6];
-  int rc = shrike_raise_smem(raised[0], single_kernel<true>, shared_floats<16>() * 4);
-  if (rc == 0) rc = shrike_raise_smem(raised[4], single_kernel<false>, shared_floats<16>() * 4);
-  if (rc == 0) rc = shrike_raise_smem(raised[5], portions_kernel<16, false>, shared_floats<16>() * 4);
+  static PerDevice raised[4];
+  int rc = shrike_raise_smem(raised[0], single_kernel, shared_floats<16>() * 4);
   if (rc == 0) rc = shrike_raise_smem(raised[1], portions_kernel<16>, shared_floats<16>() * 4);
   if (rc == 0) rc = shrike_raise_smem(raised[2], portions_kernel<32>, shared_floats<32>() * 4);
   if (rc == 0) rc = shrike_raise_smem(raised[3], portions_kernel<64>, shared_floats<64>() * 4);
   if (rc != 0) return rc;
-  if (has_portions) {
+  const bool places = static_cast<long long>(num_kv_heads) * ((share + 15) / 16) <= 65535;
+  if (has_single && (!wide || !places || num_seqs > 65535)) has_single = 2;
+  if (has_portions && (!wide || !places)) has_portions = 2;
+  if (has_single == 2 || has_portions == 2) {
+    const long long blocks = (static_cast<long long>(num_tokens) * num_heads + WARPS - 1) / WARPS;
+    if (blocks > 0x7fffffffLL) return SHRIKE_BAD_ARGUMENT;
+    const int which = has_portions != 2 ? 1 : (has_single == 1 ? 2 : 0);
+    const cudaError_t err = launch_dependent(wide_keys ? warps_kernel<true> : warps_kernel<false>, dim3(static_cast<unsigned>(blocks)),
+                                             dim3(WARPS * 32), 0, stream, p, which);
+    if (err != cudaSuccess) return static_cast<int>(err);
+  }
+  if (has_portions == 1) {
     // 64 rows a CTA read a key from shared memory for 64 rows, 16 only for 16; but fewer of them live on an SM (two for heads of
     // 64, one for wider ones; of 16 rows three, two and one), and where they are few the device waits for the last tokens' CTAs,
     // which walk every key.  Measured, us with 16, 32 and 64 rows: 14 heads of 64 over 2: 100 tokens 12.8, 15.6, 22.6; 333 tokens
     // 43.5, 43.1, 54.1; 1,500 tokens 371, 285, 300; 28 heads of 128 over 4: 100 tokens 24.4, 23.3, 31.6; 400 tokens 131, 95.7,
     // 91.3; 1,500 tokens 1,402, 881, 771.  What is chosen is within 7% of the best at 17 to 1,500 tokens of five head layouts.
-    // Pages that do not lie on 16 bytes have the smallest form alone.
     const long long rows = static_cast<long long>(num_tokens) * share, sms = shrike_device().sm_count;
-    const int a_cta = !wide ? 16 : (rows + 63) / 64 * num_kv_heads >= 2 * sms ? 64 : ((rows + 31) / 32 * num_kv_heads * 5 >= 4 * sms ? 32 : 16);
+    const int a_cta = (rows + 63) / 64 * num_kv_heads >= 2 * sms ? 64 : ((rows + 31) / 32 * num_kv_heads * 5 >= 4 * sms ? 32 : 16);
     p.heads_per_cta = share < a_cta ? share : a_cta;
     p.head_groups = (share + p.heads_per_cta - 1) / p.heads_per_cta;
     const int a_tile = a_cta / p.heads_per_cta;
-    if (static_cast<long long>(num_kv_heads) * p.head_groups > 65535) return SHRIKE_BAD_ARGUMENT;
     const dim3 grid((num_tokens + a_tile - 1) / a_tile, num_kv_heads * p.head_groups);
-    const cudaError_t err = !wide         ? launch_dependent(portions_kernel<16, false>, grid, dim3(THREADS), shared_floats<16>() * 4, stream, p)
-                            : a_cta == 64   ? launch_dependent(portions_kernel<64>, grid, dim3(THREADS), shared_floats<64>() * 4, stream, p)
+    const cudaError_t err = a_cta == 64   ? launch_dependent(portions_kernel<64>, grid, dim3(THREADS), shared_floats<64>() * 4, stream, p)
                             : a_cta == 32 ? launch_dependent(portions_kernel<32>, grid, dim3(THREADS), shared_floats<32>() * 4, stream, p)
                                           : launch_dependent(portions_kernel<16>, grid, dim3(THREADS), shared_floats<16>() * 4, stream, p);
     if (err != cudaSuccess) return static_cast<int>(err);
   }
-  if (has_single) {
+  if (has_single == 1) {
     p.heads_per_cta = share < 16 ? share : 16;
     p.head_groups = (share + p.heads_per_cta - 1) / p.heads_per_cta;
-    if (static_cast<long long>(num_kv_heads) * p.head_groups > 65535) return SHRIKE_BAD_ARGUMENT;
-    cudaError_t err = launch_dependent(wide ? single_kernel<true> : single_kernel<false>, dim3(chunks, num_kv_heads * p.head_groups, num_seqs), dim3(THREADS),
+    cudaError_t err = launch_dependent(single_kernel, dim3(chunks, num_kv_heads * p.head_groups, num_seqs), dim3(THREADS),
                                        shared_floats<16>() * 4, stream, p);
     if (err == cudaSuccess && chunks > 1)
       err = launch_dependent(merge_kernel, dim3((num_seqs * num_heads + 3) / 4), dim3(128), 0, stream, p);

@@ -138,6 +138,7 @@ class CudaOps:
         self._delta_scratch = None    # the delta rule's blocks of tokens: what the walk over them reads
         self._delta_runs = None       # and, where few walks are cut into runs, what those hand to one another
         self.delta_run_blocks = None  # None: the kernel library's rule; n: runs of n blocks (0: none; tests)
+        self.fp32_attention_form = 0  # 0: the kernel library's rule; 1: tiles of rows, 2: a warp a row (tests)
         self.gemm_fp32_tile = 0  # 0: the kernel library's rule; n: tiles of 8 n rows in the 32-bit product (tests)
         self.portion_splits = 0  # 0: the kernel library's rule; n: that many key splits for portions (tests)
         self.generation = 0      # grows when the scratch moves
@@ -246,6 +247,9 @@ class CudaOps:
                 )
                 lib.shrike_paged_attention_fp32.restype = _I
                 lib.shrike_attention_fp32_chunk.restype = _I
+                lib.shrike_attention_fp32_single_form.argtypes = [_I] * 4
+                lib.shrike_attention_fp32_portion_form.argtypes = [_I] * 4
+                lib.shrike_attention_fp32_single_form.restype = lib.shrike_attention_fp32_portion_form.restype = _I
             if head_dim <= build.TENSOR_CORE_HEAD_DIM:
                 self._declare_tensor_core_attention(lib)
             self._attention[head_dim] = lib
@@ -711,10 +715,19 @@ class CudaOps:
                 self._stream()), "paged_attention")
             return
         if self.dtype == torch.float32:
-            has_single = max_q_len == 1 or (max_q_len > 1 and min_q_len == 1)
-            has_portions = max_q_len != 1   # lengths that are not known among them: that kernel takes entries of any length
-            chunks, scratch = self.fp32_chunks(lib, num_seqs, num_heads, num_kv_heads, head_dim, max_blocks * page_size) if has_single else (1, None)
-            self.launches += has_portions + has_single + (chunks > 1)
+            # 0: none, 1: tiles of rows, 2: a warp a row, with the same bits
+            has_single = has_portions = 0
+            if max_q_len == 1 or (max_q_len > 1 and min_q_len == 1):
+                reach = max_ctx_len if 0 < max_ctx_len <= self.FEW_KEYS else max_blocks * page_size
+                has_single = self.fp32_attention_form or lib.shrike_attention_fp32_single_form(num_seqs, num_heads, num_kv_heads, reach)
+            if max_q_len != 1:   # lengths that are not known among them: that kernel takes entries of any length
+                longer = [length for length in q_lens if length > 1 or not has_single] if q_lens is not None else None
+                tokens, entries = (sum(longer), len(longer)) if longer else (q.shape[0], num_seqs)
+                has_portions = self.fp32_attention_form or lib.shrike_attention_fp32_portion_form(tokens, entries, num_heads, num_kv_heads)
+            chunks, scratch = (1, None)
+            if has_single == 1:
+                chunks, scratch = self.fp32_chunks(lib, num_seqs, num_heads, num_kv_heads, head_dim, max_blocks * page_size)
+            self.launches += (has_single == 1) + (has_portions == 1) + (has_single == 2 or has_portions == 2) + (chunks > 1)
             _check(lib.shrike_paged_attention_fp32(
                 _ptr(q), _ptr(keys), _ptr(values), _ptr(block_table), max_blocks, _ptr(q_start), _ptr(ctx_len), _ptr(seq_of_token),
                 q.shape[0], num_seqs, num_heads, num_kv_heads, page_size, num_pages, scale, window or 0, softcap or 0.0,
@@ -823,7 +836,14 @@ class CudaOps:
         return AttentionPlan(int(has_single), int(has_portions), int(tc_portions), splits, cluster, scratch, arrivals,
                              portion_splits, portion_scratch)
 
-    SHORT_CONTEXT = 64   # keys: a launch captured for a batch's lengths holds for contexts on the same side of it
+    SHORT_CONTEXT = 64   # keys up to which `short_portions` looks at the longest context
+    FEW_KEYS = 8         # and up to which the 32-bit path's single tokens do
+
+    def context_class(self, decode, max_ctx_len) -> int:
+        """Which side of the lines above a batch's longest context lies on: a captured launch sequence holds for that side alone."""
+        if self.dtype == torch.float32:
+            return int(max_ctx_len <= self.FEW_KEYS)
+        return int(not decode and max_ctx_len <= self.SHORT_CONTEXT)
 
     def short_portions(self, max_q_len, table_keys, max_ctx_len, head_dim, ctas) -> bool:
         """Whether portions run on the mma.sync kernel although the tcgen05 one serves them: portions of up to 64 tokens over few

@@ -73,9 +73,10 @@ def test_which_portions_are_short(max_q_len, table_keys, max_ctx_len, head_dim, 
     assert ops.short_portions(max_q_len, table_keys, max_ctx_len, head_dim, ctas) is short
 
 
-@pytest.mark.parametrize("dtype,apart", [("bfloat16", True), ("float32", False)])
-def test_a_captured_portion_holds_for_contexts_on_one_side_of_the_short_ones(dtype, apart):
-    """Two steps of the same lengths and table widths, over 40 and over 100 keys: other kernels in bfloat16."""
+@pytest.mark.parametrize("dtype,lengths,start,apart", [("bfloat16", 40, 60, True), ("bfloat16", 1, 60, False), ("float32", 40, 60, False),
+                                                       ("float32", 1, 60, True)])
+def test_a_captured_step_holds_for_contexts_for_which_the_same_kernels_run(dtype, lengths, start, apart):
+    """Two steps of the same lengths and table widths, from the start and further on."""
     from shrike_b200.config import parse_config
     from shrike_b200.engine.batch import StepEntry
     from shrike_b200.engine.runner import ModelRunner
@@ -84,14 +85,11 @@ def test_a_captured_portion_holds_for_contexts_on_one_side_of_the_short_ones(dty
     from tests.tiny_configs import TINY
 
     config, ops = parse_config(TINY["C"]), EmulatedOps()
-    ops.SHORT_CONTEXT = CudaOps.SHORT_CONTEXT
+    ops.context_class = bare_ops(getattr(torch, dtype)).context_class
     runner = ModelRunner(config, dict(random_tensors(config, 1)), ops, "cpu", dtype, page_size=16, num_pages=24, max_slots=4)
     keys = []
-    for start in (0, 60):
+    for first in (0, start):
         cache = runner.cache.open()
-        runner.cache.append(cache, 0, start + 40)
-        keys.append(runner.prepare([StepEntry(cache, [3] * 40, start, [39])]).key)
+        runner.cache.append(cache, 0, first + lengths)
+        keys.append(runner.prepare([StepEntry(cache, [3] * lengths, first, [lengths - 1])]).key)
     assert (keys[0] != keys[1]) == apart
-    cache = runner.cache.open()
-    runner.cache.append(cache, 0, 101)
-    assert runner.prepare([StepEntry(cache, [3], 100, [0])]).key == runner.prepare([StepEntry(cache, [3], 9, [0])]).key

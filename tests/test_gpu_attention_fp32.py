@@ -59,6 +59,11 @@ def test_fp32_attention_gives_a_token_the_same_bits_in_a_prompt_and_alone(heads,
     seq_of = torch.repeat_interleave(torch.arange(count), torch.tensor(q_lens)).to(torch.int32).to(DEV)
     mixed = attention(ops, case, rows, starts, case["ctx_len"], seq_of, case["table"], heads, kv_heads, dim, q_lens, **options)
     assert torch.equal(mixed[: count - 1], whole[last[:-1]]) and torch.equal(mixed[count - 1:], whole[last[-1] - 9: last[-1] + 1])
+    # a warp a row
+    ops.fp32_attention_form = 2
+    assert torch.equal(attention(ops, case, case["q"], case["q_start"], case["ctx_len"], case["seq_of"], case["table"], heads, kv_heads, dim, ctx_lens,
+                                 **options), whole)
+    assert torch.equal(attention(ops, case, rows, starts, case["ctx_len"], seq_of, case["table"], heads, kv_heads, dim, q_lens, **options), mixed)
     if set(options) <= {"window"}:
         want = torch.cat([pm.causal_attention(q.double().to(DEV), k.double().to(DEV), v.double().to(DEV), options.get("window"))
                           for q, k, v in case["seqs"]]).reshape(whole.shape)
@@ -132,3 +137,18 @@ def test_fp32_attention_of_more_sequences_than_a_grid_has_places():
     few = attention(ops, case, q[-300:].contiguous(), index[:301].clone(), ctx_len[-300:].contiguous(), index[:300], table[-300:].contiguous(), heads, 1,
                     dim, [1] * 300)
     assert torch.isfinite(whole).all() and torch.equal(whole[-300:], few)
+
+
+# the batches that a rule sends to a warp a row, beside ones just short of it: many pairs of one or two heads, few keys, many short entries
+@pytest.mark.parametrize("heads,kv_heads,q_lens,ctx_lens", [
+    (32, 32, [1] * 32, list(range(1, 33))), (32, 32, [1] * 7, [5, 128, 33, 64, 65, 1, 127]), (32, 32, [1] * 8, [5, 128, 33, 64, 65, 1, 127, 31]),
+    (6, 2, [1] * 3, [8, 3, 1]), (6, 2, [1] * 3, [9, 3, 1]), (4, 4, [2, 5, 1, 3], [70, 5, 1, 33]), (4, 2, [3, 3], [40, 3]), (4, 2, [3, 4], [40, 4])])
+def test_fp32_attention_by_either_form_gives_the_same_bits(heads, kv_heads, q_lens, ctx_lens):
+    ops = cuda_ops(torch.float32)
+    case = paged_case(torch.float32, heads, kv_heads, 48, 16, ctx_lens, q_lens, seed=heads + len(q_lens))
+    args = (case["q"], case["q_start"], case["ctx_len"], case["seq_of"], case["table"], heads, kv_heads, 48, q_lens)
+    outs = []
+    for form in (0, 1, 2):
+        ops.fp32_attention_form = form
+        outs.append(attention(ops, case, *args))
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
