@@ -117,7 +117,7 @@ __device__ __forceinline__ void add_values(float (&acc)[RI][COLS * 4], const flo
 // Rows: the tokens [token, token + count) of sequence `seq`, heads [head, head + heads) of one kv head; chunks [c_begin, c_end).
 template <int R>
 __device__ void attend(const Params& p, float* smem, int seq, int token, int count, int head, int heads, int kv_head, int c_begin, int c_end,
-                       bool whole) {
+                       bool whole, int slot = 0) {
   constexpr int RI = R / 16;
   float* q_s = smem;                       // [R][ROW]
   float* k_s = q_s + R * ROW;              // [2][KEYS][ROW]
@@ -301,7 +301,7 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
         }
       }
     } else {
-      float* to = p.partial + ((static_cast<size_t>(seq) * p.num_heads + row_head[i]) * p.chunks + c_begin) * (D + 2);
+      float* to = p.partial + ((static_cast<size_t>(seq) * p.num_heads + row_head[i]) * p.chunks + slot) * (D + 2);
 #pragma unroll
       for (int c = 0; c < COLS; ++c)
 #pragma unroll
@@ -315,7 +315,17 @@ __device__ void attend(const Params& p, float* smem, int seq, int token, int cou
   }
 }
 
-// Single tokens: grid (chunks, kv heads times head groups, sequences).
+// The chunks that a single token's row sees: `kept` of the kept first keys, then those from `from` on that hold its window.
+struct Visible {
+  int kept, from, count;
+};
+__device__ __forceinline__ Visible visible_chunks(const Params& p, int position) {
+  const int first = first_visible_key(position, p.window), kept = p.window > 0 ? (min(p.keep_first, first) + CHUNK - 1) / CHUNK : 0;
+  const int from = max(first / CHUNK, kept);
+  return Visible{kept, from, position < 0 ? 0 : min(p.chunks, kept + max(0, position / CHUNK - from + 1))};
+}
+
+// Single tokens: grid (chunks that a row can see, kv heads times head groups, sequences).
 __global__ void __launch_bounds__(THREADS) single_kernel(const Params p) {
   extern __shared__ __align__(16) float smem[];
   let_dependents_start();
@@ -323,13 +333,16 @@ __global__ void __launch_bounds__(THREADS) single_kernel(const Params p) {
   const int seq = blockIdx.z, kv_head = blockIdx.y / p.head_groups, group = blockIdx.y % p.head_groups;
   const int token = p.q_start[seq];
   // a longer entry: the portions kernel's; or the table is wider than the sequence is long
-  if (p.q_start[seq + 1] - token != 1 || (p.chunks > 1 && static_cast<int>(blockIdx.x) * CHUNK >= p.ctx_len[seq])) {
+  const int index = blockIdx.x;
+  const Visible seen = visible_chunks(p, p.ctx_len[seq] - 1);
+  const int chunk = p.chunks == 1 ? 0 : (index < seen.kept ? index : seen.from + index - seen.kept);
+  if (p.q_start[seq + 1] - token != 1 || (p.chunks > 1 && index >= seen.count)) {
     if (p.early_metadata) wait_for_previous();   // every CTA waits before it leaves
     return;
   }
   const int share = p.num_heads / p.num_kv_heads, head = kv_head * share + group * p.heads_per_cta;
   const int heads = min(p.heads_per_cta, share - group * p.heads_per_cta);
-  attend<16>(p, smem, seq, token, 1, head, heads, kv_head, blockIdx.x, p.chunks > 1 ? blockIdx.x + 1 : 0x7ffffff, p.chunks == 1);
+  attend<16>(p, smem, seq, token, 1, head, heads, kv_head, chunk, p.chunks > 1 ? chunk + 1 : 0x7ffffff, p.chunks == 1, index);
 }
 
 // A warp a (sequence, head): the chunks of a single token's row, in ascending order.
@@ -341,7 +354,7 @@ __global__ void __launch_bounds__(128) merge_kernel(const Params p) {
   const int seq = work / p.num_heads, head = work % p.num_heads;
   const int token = p.q_start[seq];
   if (p.q_start[seq + 1] - token != 1) return;
-  const int chunks = min(p.chunks, (p.ctx_len[seq] + CHUNK - 1) / CHUNK);
+  const int chunks = visible_chunks(p, p.ctx_len[seq] - 1).count;
   const float* from = p.partial + static_cast<size_t>(work) * p.chunks * (D + 2);
   constexpr int OWN = (D + 31) / 32;
   float total[OWN];
@@ -505,8 +518,15 @@ __global__ void __launch_bounds__(WARPS * 32) warps_kernel(const Params p, int w
 
 SHRIKE_API int shrike_attention_head_dim() { return attn32::D; }
 
-// Keys of a chunk: single tokens want chunks = ceil(table width * page size / this) and, above one, that much scratch.
-SHRIKE_API int shrike_attention_fp32_chunk() { return attn32::CHUNK; }
+// Chunks of single tokens' keys: what tables of `keys` keys hold, no more than a window (or run of positions, `window` < 0) and the
+// kept first keys can reach.
+SHRIKE_API int shrike_attention_fp32_chunks(int keys, int window, int keep_first) {
+  constexpr long long C = attn32::CHUNK;
+  const long long all = (static_cast<long long>(keys) + C - 1) / C, span = window < 0 ? -static_cast<long long>(window) : window;
+  if (window == 0) return static_cast<int>(all);
+  const long long seen = (span + C - 1) / C + 1 + (window > 0 ? (keep_first + C - 1) / C : 0);
+  return static_cast<int>(seen < all ? seen : all);
+}
 
 // How single tokens (portions) should run: 1 the CTA forms, 2 a warp a row.  `keys`: what the block tables can hold, or what is
 // known to be the longest context.

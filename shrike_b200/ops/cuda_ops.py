@@ -246,7 +246,8 @@ class CudaOps:
                     [_P, _P, _P, _P, _I, _P, _P, _P] + [_I] * 6 + [_F, _I, _F, _P, _P] + [_I] * 4 + [_P, _I, _P, _P]
                 )
                 lib.shrike_paged_attention_fp32.restype = _I
-                lib.shrike_attention_fp32_chunk.restype = _I
+                lib.shrike_attention_fp32_chunks.argtypes = [_I, _I, _I]
+                lib.shrike_attention_fp32_chunks.restype = _I
                 lib.shrike_attention_fp32_single_form.argtypes = [_I] * 4
                 lib.shrike_attention_fp32_portion_form.argtypes = [_I] * 4
                 lib.shrike_attention_fp32_single_form.restype = lib.shrike_attention_fp32_portion_form.restype = _I
@@ -726,7 +727,7 @@ class CudaOps:
                 has_portions = self.fp32_attention_form or lib.shrike_attention_fp32_portion_form(tokens, entries, num_heads, num_kv_heads)
             chunks, scratch = (1, None)
             if has_single == 1:
-                chunks, scratch = self.fp32_chunks(lib, num_seqs, num_heads, num_kv_heads, head_dim, max_blocks * page_size)
+                chunks, scratch = self.fp32_chunks(lib, num_seqs, num_heads, num_kv_heads, head_dim, max_blocks * page_size, window or 0, keep_first)
             self.launches += (has_single == 1) + (has_portions == 1) + (has_single == 2 or has_portions == 2) + (chunks > 1)
             _check(lib.shrike_paged_attention_fp32(
                 _ptr(q), _ptr(keys), _ptr(values), _ptr(block_table), max_blocks, _ptr(q_start), _ptr(ctx_len), _ptr(seq_of_token),
@@ -762,11 +763,11 @@ class CudaOps:
 
     FP32_SCRATCH_FLOATS = 64 << 20   # at most 256 MiB of partial rows for the 32-bit path's single tokens
 
-    def fp32_chunks(self, lib, num_seqs, num_heads, num_kv_heads, head_dim, keys):
+    def fp32_chunks(self, lib, num_seqs, num_heads, num_kv_heads, head_dim, keys, window=0, keep_first=0):
         """(chunks of keys that run on CTAs of their own, their scratch) for single tokens in float32: all of them where
         the kv heads of the batch alone would leave SMs idle, else one CTA walks a row's chunks itself; the bits are the
         same.  `keys`: what the block tables can hold."""
-        chunks = -(-keys // lib.shrike_attention_fp32_chunk())
+        chunks = lib.shrike_attention_fp32_chunks(keys, window, keep_first)
         need = num_seqs * num_heads * chunks * (head_dim + 2)
         if num_seqs * num_kv_heads >= 4 * self.sm_count or need > self.FP32_SCRATCH_FLOATS:
             chunks = 1

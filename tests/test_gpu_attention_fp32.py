@@ -152,3 +152,19 @@ def test_fp32_attention_by_either_form_gives_the_same_bits(heads, kv_heads, q_le
         ops.fp32_attention_form = form
         outs.append(attention(ops, case, *args))
     assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+# windows and kept keys whose chunks meet, touch and lie apart; the chunks on CTAs of their own against one warp that walks them all
+@pytest.mark.parametrize("options", [{"window": 1}, {"window": 64}, {"window": 65, "keep_first": 1}, {"window": 100, "keep_first": 64}, {"window": 30, "keep_first": 130},
+                                     {"window": 500, "keep_first": 65}, {"chunk": 64}, {"chunk": 200}])
+def test_fp32_single_tokens_walk_the_chunks_that_a_window_reaches(options):
+    ops = cuda_ops(torch.float32)
+    heads, kv_heads, dim, ctx_lens = 6, 2, 48, [1, 63, 64, 65, 128, 129, 190, 193, 257, 700, 1025]
+    case = paged_case(torch.float32, heads, kv_heads, dim, 16, ctx_lens, [1] * len(ctx_lens), seed=11)
+    wide = torch.full((len(ctx_lens), 160), -1, dtype=torch.int32, device=DEV)   # tables far wider than what is held
+    wide[:, : case["table"].shape[1]] = case["table"]
+    outs = []
+    for form, table in ((2, case["table"]), (1, case["table"]), (1, wide)):
+        ops.fp32_attention_form = form
+        outs.append(attention(ops, case, case["q"], case["q_start"], case["ctx_len"], case["seq_of"], table, heads, kv_heads, dim, [1] * len(ctx_lens), **options))
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
