@@ -109,8 +109,8 @@ sample_slices_kernel(const float* __restrict__ logits, const float* __restrict__
   }
 }
 
-// Stage 2 for vocabularies whose rows do not fit a cluster's shared memory (above some 400,000 tokens): one block per row,
-// the row read from memory at every step of the bisection.
+// Stage 2 for vocabularies whose rows do not fit a cluster's shared memory (above some 400,000 tokens), and for small ones, whose
+// rows are quickly read: one block per row, the row read at every step of the bisection.
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
               const float* __restrict__ top_p, const long long* __restrict__ seeds, int* __restrict__ out,
@@ -333,7 +333,7 @@ SHRIKE_API int shrike_sample_slices(int vocab) {
 }
 
 namespace {
-// Both stages; rows that fit a cluster's shared memory take the cluster form of stage 2.
+// Both stages.
 int launch_sample(const float* logits, const float* temperature, const float* top_p, const long long* seeds, int* out,
                   float* scratch_value, int* scratch_index, int rows, int vocab, int chunks, int* status, cudaStream_t stream) {
   cudaError_t err = launch_dependent(sample_slices_kernel, dim3(chunks, rows), SLICE_THREADS, 0, stream, logits, temperature, top_p,
@@ -341,7 +341,12 @@ int launch_sample(const float* logits, const float* temperature, const float* to
   if (err != cudaSuccess) return static_cast<int>(err);
   const size_t smem = static_cast<size_t>((vocab + SAMPLE_THREADS - 1) / SAMPLE_THREADS) * ROW_THREADS * sizeof(float);
   constexpr size_t MOST = 200 * 1024;
-  if (smem <= MOST) {
+  // The cluster form costs 0.3 us a cluster to start, whatever a row holds; a block a row costs a scan of the row at every step of
+  // the bisection.  Measured, us with clusters and with blocks: 1,000 tokens 20 and 19 (1 row), 37 and 23 (64), 96 and 29 (256);
+  // 2,000 tokens 22 and 23 (8), 30 and 23 (32); 5,000 tokens 40 and 52 (64), 54 and 57 (128), 103 and 59 (256); 12,000 tokens 109
+  // and 112 (256), 206 and 217 (512); 152,000 tokens 183 and 1,117 (64).  Both give the same tokens.
+  const bool clusters = vocab >= 12000 || (vocab >= 4096 && rows <= 128) || (vocab >= 1536 && rows <= 8);
+  if (clusters && smem <= MOST) {
     static PerDevice raised;
     const int rc = shrike_raise_smem(raised, sample_cluster_kernel, MOST);
     if (rc != 0) return rc;
