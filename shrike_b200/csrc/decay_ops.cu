@@ -240,8 +240,10 @@ __device__ __forceinline__ void stage_rows(float* dst, int pitch, int fill_to, c
 #pragma unroll
       for (int b = 0; b < STAGE_AHEAD; ++b) {
         const int i = i0 + b * THREADS, j = i / quads, e = (i - j * quads) << 2;
-        v[b].x = silu(v[b].x); v[b].y = silu(v[b].y); v[b].z = silu(v[b].z); v[b].w = silu(v[b].w);
-        if (j < CHUNK) *reinterpret_cast<float4*>(dst + j * pitch + e) = v[b];
+        if (j < CHUNK) {   // heads of 64 have half a batch
+          v[b].x = silu(v[b].x); v[b].y = silu(v[b].y); v[b].z = silu(v[b].z); v[b].w = silu(v[b].w);
+          *reinterpret_cast<float4*>(dst + j * pitch + e) = v[b];
+        }
       }
     }
     return;
@@ -256,10 +258,12 @@ __device__ __forceinline__ void stage_rows(float* dst, int pitch, int fill_to, c
 }
 
 // grid (column groups of `span`, heads, runs): intra-run outputs and L_c, 64 columns at a time.
-// Three CTAs an SM (their staging, products and stores overlap, and the runs and heads of a usual prompt are one round of
-// CTAs): once the scores stand in registers q is not needed, and the scores and the value columns take its place.
-// Measured (2,048 tokens, 12 heads of 128 x 128): 56.7 us, and 84.9 with two CTAs an SM and loads one at a time.
-__global__ void __launch_bounds__(THREADS, 3) chunk_local_kernel(ChunkArgs c) {
+// RESIDENT: CTAs an SM, by registers (80 and a few spilled ones a thread, or 122).  Three overlap their staging, products and stores, and
+// the runs and heads of a long prompt make fewer rounds; once the scores stand in registers q is not needed, and the scores and the
+// value columns take its place.  Measured (2,048 tokens, 12 heads of 128 x 128): 56.7 us, and 84.9 with two CTAs an SM and loads
+// one at a time.
+template <int RESIDENT>
+__global__ void __launch_bounds__(THREADS, RESIDENT) chunk_local_kernel(ChunkArgs c) {
   extern __shared__ __align__(16) float shared[];
   const ScanArgs& a = c.s;
   const int pitch = chunk_pitch(a.dim), dim8 = (a.dim + 7) & ~7, dim4 = (a.dim + 3) & ~3;
@@ -673,10 +677,10 @@ __global__ void __launch_bounds__(THREADS) concat_cast_kernel(float* __restrict_
                                                               T* __restrict__ out, long long total, int width, int wide) {
   let_dependents_start();
   wait_for_previous();
-  if (wide) {   // a block a row, four elements at a time
+  if (wide) {   // gridDim.y blocks a row, four elements at a time
     const size_t at = static_cast<size_t>(blockIdx.x) * width;
     T* to = out + 2 * at;
-    for (int e = threadIdx.x * 4; e < width; e += THREADS * 4) {
+    for (int e = (blockIdx.y * THREADS + threadIdx.x) * 4; e < width; e += gridDim.y * THREADS * 4) {
       float v[4], o[4], add[4];
       load4<float>(resid + at + e, v);
       load4<float>(other + at + e, o);
@@ -762,14 +766,21 @@ SHRIKE_API int shrike_decay_scan(const float* fused, int partials, long long par
   if (chunked) {
     ChunkArgs c;
     c.s = a; c.chunk_state = chunk_state; c.num_seqs = num_seqs; c.skip = skip;
-    static PerDevice raised[2];
-    if (shrike_raise_smem(raised[0], chunk_local_kernel, limit) != 0 || shrike_raise_smem(raised[1], chunk_finish_kernel, limit) != 0)
+    static PerDevice raised[3];
+    if (shrike_raise_smem(raised[0], chunk_local_kernel<3>, limit) != 0 || shrike_raise_smem(raised[1], chunk_finish_kernel, limit) != 0 ||
+        shrike_raise_smem(raised[2], chunk_local_kernel<2>, limit) != 0)
       return SHRIKE_BAD_ARGUMENT;
     // a CTA takes every value column of its run and head (q, k and the scores are staged once) when the runs and heads
     // alone fill the device twice over, else 64 columns
     c.span = static_cast<long long>(chunks) * heads >= 2ll * shrike_device().sm_count ? slices * MAX_SLICE : MAX_SLICE;
     const dim3 per_chunk((vdim + c.span - 1) / c.span, heads, chunks);
-    err = launch_dependent(chunk_local_kernel, per_chunk, dim3(THREADS), local_smem, stream, c);
+    // Two CTAs an SM where they are one round that fills its places, or so few that an SM has one.  The whole scan over 12 heads of 128 x
+    // 128, us with three and with two: 512 tokens (96 CTAs) 60.6 and 51.4, 700 (132) 62.7 and 53.1, 1,024 (192) 64.2 and 71.7, 1,536
+    // (288) 98.0 and 81.1, 2,048 (384) 100 and 114, 4,096 (768) 207 and 229; over 28 heads: 300 (140) 62.5 and 53.7, 512 (224) 84.2 and
+    // 83.4, 700 (308) 96.1 and 105, 2,048 (896) 246 and 263.
+    const long long ctas = static_cast<long long>(per_chunk.x) * per_chunk.y * per_chunk.z, sms = shrike_device().sm_count;
+    const bool two = ctas <= sms || (2 * ctas > 3 * sms && ctas <= 2 * sms);
+    err = launch_dependent(two ? chunk_local_kernel<2> : chunk_local_kernel<3>, per_chunk, dim3(THREADS), local_smem, stream, c);
     if (err != cudaSuccess) return static_cast<int>(err);
     // four elements a thread where every head's state and every run's addition start on 16 bytes
     const bool carry_wide = (dim * vdim) % 4 == 0 && state_stride % 4 == 0;
@@ -847,8 +858,10 @@ SHRIKE_API int shrike_concat_cast(float* resid, const float* const* data, const 
   for (int k = 0; k < count; ++k) wide = wide && on16(terms.data[k]) && terms.stride[k] % 4 == 0;
   const long long blocks = wide ? n : (total + decay::THREADS - 1) / decay::THREADS;
   if (blocks > 0x7fffffffLL) return SHRIKE_BAD_ARGUMENT;
+  // few rows: as many blocks a row as give each thread one access (1 row of 3,584 with eight slices: 4.3 us with one block)
+  const unsigned parts = wide ? static_cast<unsigned>(shrike_spread(n, (width / 4 + decay::THREADS - 1) / decay::THREADS)) : 1;
 #define SHRIKE_CONCAT(T)                                                                                        \
-  launch_dependent(decay::concat_cast_kernel<T>, dim3(static_cast<unsigned>(blocks)), dim3(decay::THREADS), 0, stream, resid, \
+  launch_dependent(decay::concat_cast_kernel<T>, dim3(static_cast<unsigned>(blocks), parts), dim3(decay::THREADS), 0, stream, resid, \
                    terms, other, static_cast<T*>(out), total, width, wide ? 1 : 0)
   if (dtype == SHRIKE_F32) SHRIKE_CONCAT(float);
   else if (dtype == SHRIKE_BF16) SHRIKE_CONCAT(__nv_bfloat16);
