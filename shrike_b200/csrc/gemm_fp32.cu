@@ -17,8 +17,9 @@
 //                        them; both operands stay K-major as TMA brings them, and a thread reads a
 //                        column's worth of pieces, two rows' FMAs in one instruction.  Three stages, two CTAs an SM.
 //                        Where the tiles alone would not fill the device the runs go to CTAs of their own and leave
-//                        as a stack that the consumer adds in order.
-//   otherwise            `plain_kernel` (K not a multiple of four, operands not aligned to 16 bytes)
+//                        as a stack that the consumer, or `sum_runs_kernel`, adds in order.
+//   small products       `plain_kernel`: 64 x 64 tiles, 16 of k at a time (also K not a multiple of four, and operands not aligned to
+//                        16 bytes)
 //
 // Measured (one B200, the plain kernel's time first): 1.5B widths, 3 tokens: the products of a decode step 30.3 and 1.55 ms,
 // the 17,920 x 1,536 matrix 20.1 us (5.5 TB/s) and the 1,536 x 8,960 one 15.3 (3.6 TB/s); 0.5B widths, 333 tokens: the
@@ -33,6 +34,8 @@ enum : int { ERR_ROWS = 41, ERR_TILE_PRODUCER = 42, ERR_TILE = 43, ERR_DRAIN = 4
 constexpr int BM = 64, BN = 64, BK = 16;   // the plain kernel's tile
 constexpr int PLAIN_THREADS = 256;
 
+// VEC: rows and operands lie on 16 bytes.
+template <bool VEC>
 __global__ void __launch_bounds__(PLAIN_THREADS)
 plain_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
              float* __restrict__ C, int M, int N, int K, int segment_length) {
@@ -44,54 +47,58 @@ plain_kernel(const float* __restrict__ A, const float* __restrict__ W, const flo
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int load_row = tid >> 2, load_k = (tid & 3) * 4;
   const int ty = tid >> 4, tx = tid & 15;
+  const int am = m0 + load_row, wn = n0 + load_row;
   float acc[4][4], total[4][4];
+  for (int begin = 0; begin < K; begin += segment_length) {   // a run: a multiple of BK
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    if (k0 > 0 && k0 % segment_length == 0) {   // a multiple of BK
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const int end = min(K, begin + segment_length);
+    for (int k0 = begin; k0 < end; k0 += BK) {
+      float a_reg[4] = {0.f, 0.f, 0.f, 0.f}, w_reg[4] = {0.f, 0.f, 0.f, 0.f};
+      const int k = k0 + load_k;
+      if (am < M) {
+        const float* src = A + static_cast<size_t>(am) * K + k;
+        if (VEC) {
+          if (k < K) load4<float>(src, a_reg);
+        } else {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          total[i][j] = k0 == segment_length ? acc[i][j] : total[i][j] + acc[i][j];
-          acc[i][j] = 0.f;
+          for (int i = 0; i < 4; ++i) if (k + i < K) a_reg[i] = src[i];
         }
+      }
+      if (wn < N) {
+        const float* src = W + static_cast<size_t>(wn) * K + k;
+        if (VEC) {
+          if (k < K) load4<float>(src, w_reg);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) if (k + i < K) w_reg[i] = __ldg(src + i);
+        }
+      }
+      __syncthreads();  // the previous tile has been consumed
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a_tile[load_k + i][load_row] = a_reg[i];
+        w_tile[load_k + i][load_row] = w_reg[i];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int kk = 0; kk < BK; ++kk) {
+        const float4 a = *reinterpret_cast<const float4*>(&a_tile[kk][ty * 4]);
+        const float4 w = *reinterpret_cast<const float4*>(&w_tile[kk][tx * 4]);
+        const float av[4] = {a.x, a.y, a.z, a.w}, wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+      }
     }
-    float a_reg[4] = {0.f, 0.f, 0.f, 0.f}, w_reg[4] = {0.f, 0.f, 0.f, 0.f};
-    const int k = k0 + load_k;
-    const int am = m0 + load_row, wn = n0 + load_row;
-    if (am < M) {
-      const float* src = A + static_cast<size_t>(am) * K + k;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) if (k + i < K) a_reg[i] = src[i];
-    }
-    if (wn < N) {
-      const float* src = W + static_cast<size_t>(wn) * K + k;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) if (k + i < K) w_reg[i] = __ldg(src + i);
-    }
-    __syncthreads();  // the previous tile has been consumed
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      a_tile[load_k + i][load_row] = a_reg[i];
-      w_tile[load_k + i][load_row] = w_reg[i];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      const float4 a = *reinterpret_cast<const float4*>(&a_tile[kk][ty * 4]);
-      const float4 w = *reinterpret_cast<const float4*>(&w_tile[kk][tx * 4]);
-      const float av[4] = {a.x, a.y, a.z, a.w}, wv[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-    }
+      for (int j = 0; j < 4; ++j) total[i][j] = begin == 0 ? acc[i][j] : total[i][j] + acc[i][j];
   }
-  const bool cut = K > segment_length;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int m = m0 + ty * 4 + i;
@@ -99,10 +106,28 @@ plain_kernel(const float* __restrict__ A, const float* __restrict__ W, const flo
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
-      const float sum = cut ? total[i][j] + acc[i][j] : acc[i][j];
-      if (n < N) C[static_cast<size_t>(m) * N + n] = bias ? sum + bias[n] : sum;
+      if (n < N) C[static_cast<size_t>(m) * N + n] = bias ? total[i][j] + bias[n] : total[i][j];
     }
   }
+}
+
+// The runs of a stack added up in order, then the bias: what the kernels above leave when they add the runs themselves.
+template <int VEC>
+__global__ void __launch_bounds__(256) sum_runs_kernel(const float* __restrict__ runs, int count, const float* __restrict__ bias, float* __restrict__ C,
+                                                       long long total, int N) {
+  let_dependents_start();
+  wait_for_previous();
+  const long long at = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * VEC;
+  if (at >= total) return;
+  float v[VEC];
+  if constexpr (VEC == 4) sum_partials4(runs + at, total, count, v);
+  else v[0] = sum_partials(runs + at, total, count);
+  if (bias != nullptr) {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) v[e] += bias[(at + e) % N];
+  }
+  if constexpr (VEC == 4) store4<float>(C + at, v);
+  else C[at] = v[0];
 }
 
 // Tiles want 1024-byte alignment: the swizzle pattern repeats every 1024 bytes.
@@ -504,9 +529,12 @@ SHRIKE_API int shrike_gemm_fp32_stack(int m, int n, int k) {
 }
 
 // `stack` > 1 (as shrike_gemm_fp32_stack says, no bias): C is [stack][M][N], one slice a run of K, to be added in order.
-// `tile` 0: the tile height that the rule above gives; n: 8 n rows.
+// `tile` 0: the tile height that the rule above gives; n: 8 n rows.  `scratch` (float32 [runs][M][N], or null; for a plain result of more
+// than 16 rows where shrike_gemm_fp32_stack says more than 1): the runs go there on CTAs of their own and are then added up.  Measured,
+// us with the runs one after another in a CTA and with them side by side and a sum: 17 rows, 1,152 x 896: 57.6 and 16.4; 500 rows 80.3
+// and 31.2; 300 rows, 9,728 x 896: 180 and 164; 300 rows, 1,536 x 8,960: 756 and 237; at worst 300 rows, 9,472 x 516: 80.6 and 83.6.
 SHRIKE_API int shrike_gemm_fp32(const float* A, const float* W, const float* bias, float* C, int M, int N,
-                                int K, int stack, int tile, int* status, cudaStream_t stream) {
+                                int K, int stack, int tile, float* scratch, int* status, cudaStream_t stream) {
   using namespace fp32;
   if (M <= 0 || N <= 0) return SHRIKE_OK;
   if (K <= 0 || stack < 1) return SHRIKE_BAD_ARGUMENT;
@@ -516,8 +544,8 @@ SHRIKE_API int shrike_gemm_fp32(const float* A, const float* W, const float* bia
   if (!aligned) {
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return SHRIKE_BAD_ARGUMENT;
-    plain_kernel<<<grid, PLAIN_THREADS, 0, stream>>>(A, W, bias, C, M, N, K, length);
-    return shrike_launch_status();
+    const cudaError_t err = launch_dependent(plain_kernel<false>, grid, dim3(PLAIN_THREADS), 0, stream, A, W, bias, C, M, N, K, length);
+    return err == cudaSuccess ? shrike_launch_status() : static_cast<int>(err);
   }
   if (M <= 16) {
     if (runs == 1 || stack > 1) return rows_of_tokens<1>(A, W, bias, C, M, N, K, length, stack, status, stream);
@@ -525,6 +553,28 @@ SHRIKE_API int shrike_gemm_fp32(const float* A, const float* W, const float* bia
     if (runs <= 4) return rows_of_tokens<4>(A, W, bias, C, M, N, K, length, stack, status, stream);
     if (runs > 8) return rows_of_tokens<16>(A, W, bias, C, M, N, K, length, stack, status, stream);
     return rows_of_tokens<8>(A, W, bias, C, M, N, K, length, stack, status, stream);
+  }
+  if (tile == 0 && runs == 1) {
+    // A chain of FMAs that nothing hides runs quicker in the small tiles, as long as they are one round of CTAs (us with large and
+    // with small tiles: 129 rows, 192 x 192: 13.3 and 11.2; 500 rows, 640 x 384 [80 small tiles]: 27.2 and 23.7; 1,000 rows [160]: 40.7 and
+    // 40.5; 2,000 rows [320]: 45.9 and 57.5; 129 rows, 4,000 x 300 [189]: 35.7 and 35.0).
+    const long long small = static_cast<long long>((N + BN - 1) / BN) * ((M + BM - 1) / BM);
+    if (small <= shrike_device().sm_count) {
+      const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+      const cudaError_t err = launch_dependent(plain_kernel<true>, grid, dim3(PLAIN_THREADS), 0, stream, A, W, bias, C, M, N, K, length);
+      return err == cudaSuccess ? shrike_launch_status() : static_cast<int>(err);
+    }
+  }
+  if (scratch != nullptr && stack == 1 && runs > 1) {
+    const int rc = shrike_gemm_fp32(A, W, nullptr, scratch, M, N, K, runs, tile, nullptr, status, stream);
+    if (rc != SHRIKE_OK) return rc;
+    const long long total = static_cast<long long>(M) * N;
+    const bool vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
+    const long long blocks = ((vec ? total / 4 : total) + 255) / 256;
+    if (blocks > 0x7fffffffLL) return SHRIKE_BAD_ARGUMENT;
+    const cudaError_t err = launch_dependent(vec ? sum_runs_kernel<4> : sum_runs_kernel<1>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream,
+                                             static_cast<const float*>(scratch), runs, bias, C, total, N);
+    return err == cudaSuccess ? shrike_launch_status() : static_cast<int>(err);
   }
   switch (tile > 0 ? tile : tile_rows(M, N, stack)) {
 #define SHRIKE_TILE(TM) case TM: return launch_tiles<TM>(A, W, bias, C, M, N, K, length, stack, status, stream)

@@ -139,6 +139,7 @@ class CudaOps:
         self._delta_runs = None       # and, where few walks are cut into runs, what those hand to one another
         self.delta_run_blocks = None  # None: the kernel library's rule; n: runs of n blocks (0: none; tests)
         self.fp32_attention_form = 0  # 0: the kernel library's rule; 1: tiles of rows, 2: a warp a row (tests)
+        self._gemm_scratch = None    # the runs of a 32-bit product that are added up before it leaves
         self.gemm_fp32_tile = 0  # 0: the kernel library's rule; n: tiles of 8 n rows in the 32-bit product (tests)
         self.portion_splits = 0  # 0: the kernel library's rule; n: that many key splits for portions (tests)
         self.generation = 0      # grows when the scratch moves
@@ -160,7 +161,7 @@ class CudaOps:
         lib.shrike_silu_mul.argtypes = [_P, _P, _I, _I, _I, _I, _P]
         lib.shrike_rope_kv_write.argtypes = [_P] * 10 + [_I] * 5 + [_LL, _I, _LL, _P]
         lib.shrike_kv_write.argtypes = [_P] * 5 + [_I, _I, _I, _LL, _P]
-        lib.shrike_gemm_fp32.argtypes = [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P]
+        lib.shrike_gemm_fp32.argtypes = [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P]
         lib.shrike_gemm_fp32_stack.argtypes = [_I, _I, _I]
         lib.shrike_sample.argtypes = [_P, _P, _P, _P, _P, _P, _P, _I, _I, _P, _P]
         lib.shrike_embed_positions.argtypes = [_P, _P, _I, _P, _I, _I, _I, _P, _I, _P, _P, _I, _P]
@@ -549,12 +550,21 @@ class CudaOps:
             _dense(w, torch.float32, "linear weight")
             _dense(out, torch.float32, "linear output")
             # K is cut into the same runs, added in the same order, whether they leave as a stack or summed
-            stack = self.core.shrike_gemm_fp32_stack(n, o, k) if allow_partials and bias is None else 1
+            stack, scratch, target = self.core.shrike_gemm_fp32_stack(n, o, k), None, out
             if stack > 1 and ((x.data_ptr() | w.data_ptr()) % 16 or stack * n * o > self.FP32_STACK_FLOATS):
                 stack = 1
-            target = self._partial_stack(out, stack) if stack > 1 else out
+            if stack > 1 and allow_partials and bias is None:
+                target = self._partial_stack(out, stack)
+            elif stack > 1:
+                if n > 16 and not self.gemm_fp32_tile:
+                    if self._gemm_scratch is None or self._gemm_scratch.numel() < stack * n * o:
+                        self._gemm_scratch = torch.empty(stack * n * o, dtype=torch.float32, device=self.device)
+                        self.generation += 1
+                    scratch = self._gemm_scratch
+                    self.launches += 1
+                stack = 1
             _check(self.core.shrike_gemm_fp32(_ptr(x), _ptr(w), _ptr(bias), _ptr(target), n, o, k, stack, self.gemm_fp32_tile,
-                                              _ptr(self.status), self._stream()), "gemm_fp32")
+                                              _ptr(scratch), _ptr(self.status), self._stream()), "gemm_fp32")
             return target
         _dense(x, torch.bfloat16, "linear input")
         _dense(w, torch.bfloat16, "linear weight")
@@ -578,7 +588,7 @@ class CudaOps:
             out.add_(bias)
         return out
 
-    FP32_STACK_FLOATS = 64 << 20   # at most 256 MiB for the runs of a 32-bit product; they are summed by the product beyond that
+    FP32_STACK_FLOATS = 64 << 20   # at most 256 MiB for the runs of a 32-bit product; a CTA adds them up beyond that
 
     def _partial_stack(self, out, splits):
         """The float32 [splits, N, O] stack that belongs to the output buffer `out`, for as long as that buffer's memory lives:

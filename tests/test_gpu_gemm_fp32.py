@@ -82,3 +82,21 @@ def test_gemm_fp32_gives_the_same_bits_at_every_tile_height(tile, n, k):
         if stack.dim() == 3:
             assert torch.equal(stack, torch.cat([s for s in want_stack], dim=1)[:, :m]), m
     ops.check_status()
+
+
+# one run in small tiles, up to as many as SMs and just beyond; runs side by side and added up, with a bias, an odd width, an output that
+# does not lie on 16 bytes, and without the scratch
+@pytest.mark.parametrize("m,n,k", [(17, 8, 4), (65, 130, 500), (64 * 37, 256, 36), (64 * 37 + 1, 256, 36), (17, 130, 900), (200, 131, 4100), (333, 300, 9000)])
+def test_gemm_fp32_plain_results_of_prompts(m, n, k):
+    ops = cuda_ops(torch.float32)
+    x, w, bias = rnd(m, k, seed=m), rnd(n, k, seed=2), rnd(n, seed=3)
+    want = torch.cat([ops.linear(part.contiguous(), w, torch.empty(len(part), n, device=DEV)) for part in x.split(16)])   # few rows
+    shifted = torch.empty(m * n + 1, device=DEV)[1:].view(m, n)
+    for out in (torch.full((m, n), float("nan"), device=DEV), shifted):
+        assert torch.equal(ops.linear(x, w, out), want)
+        assert torch.equal(ops.linear(x, w, out, bias=bias), want + bias)
+    ops.gemm_fp32_tile = 16
+    assert torch.equal(ops.linear(x, w, torch.empty(m, n, device=DEV), bias=bias), want + bias)
+    ops.gemm_fp32_tile, ops.FP32_STACK_FLOATS = 0, 0
+    assert torch.equal(ops.linear(x, w, torch.empty(m, n, device=DEV), bias=bias), want + bias)
+    ops.check_status()
