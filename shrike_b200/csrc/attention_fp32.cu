@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(WARPS * 32) warps_kernel(const Params p, int w
     if (p.early_metadata) wait_for_previous();
     return;
   }
-  constexpr int OWN = (D + 31) / 32, AHEAD = OWN <= 4 ? 4 : 2;   // columns of a lane; keys whose values are on their way together
+  constexpr int OWN = (D + 31) / 32, AHEAD = OWN <= 4 ? 8 : 4;   // columns of a lane; keys whose values are on their way together
   const int position = p.ctx_len[seq] - q_len + (token - start), first = first_visible_key(position, p.window);
   const int kept = p.window > 0 ? min(p.keep_first, first) : 0;
   const int* table = p.block_table + static_cast<size_t>(seq) * p.max_blocks;
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(WARPS * 32) warps_kernel(const Params p, int w
     float score = 0.f;
     if (seen) {
       const float* k = p.k_cache + static_cast<size_t>(row) * key_stride + column;
-#pragma unroll 8
+#pragma unroll 32
       for (int c = 0; c < D; c += 4) {
         float4 b;
         if (WIDE) b = *reinterpret_cast<const float4*>(k + c);
@@ -528,24 +528,25 @@ SHRIKE_API int shrike_attention_fp32_chunks(int keys, int window, int keep_first
   return static_cast<int>(seen < all ? seen : all);
 }
 
-// How single tokens (portions) should run: 1 the CTA forms, 2 a warp a row.  `keys`: what the block tables can hold, or what is
-// known to be the longest context.
+// How single tokens (portions) should run: 1 the CTA forms, 2 a warp a row.  `keys`: the most that a row can see.
 //
 // A CTA's sixteen rows are the heads of one kv head; with one or two of them it multiplies mostly zeros, which costs nothing
-// while SMs are idle, and many such pairs are quicker with a warp a row.  Measured, us with tiles and with warps: 8 heads of 64 over 8,
-// 64 requests: 20 keys 12.3 and 6.0, 128 keys 32.0 and 22.0, 1,000 keys 195 and 306; 128 requests: 1,000 keys 381 and 314; 32 heads
-// of 128 over 32: 8 requests 20 keys 11.6 and 9.0, 128 keys 30.5 and 35.9; 32 requests 128 keys 95.8 and 77.4, 1,000 keys 704 and 546;
-// 16 heads of 64 over 8, 128 requests: 128 keys 51.6 and 49.4.  From three heads a kv head on only the first few keys are quicker
-// that way (12 heads of 128 over 2, 64 requests: 3 keys 9.7 and 6.4, 20 keys 9.9 and 9.4, 64 keys 15.9 and 21.7).
+// while SMs are idle, and many such pairs are quicker with a warp a row.  Measured, us with tiles and with warps: 8 heads of 64 over 8: 16
+// requests (128 pairs) 64 keys 14.9 and 9.2, 128 keys 14.9 and 16.5, 200 keys 21.7 and 25.4; 32 requests 200 keys 34.2 and 25.6, 1,000
+// keys 111 and 201; 64 requests 400 keys 85 and 84, 1,000 keys 195 and 202; 128 requests 1,000 keys 382 and 243; 32 heads of 128 over
+// 32: 8 requests 200 keys 49.5 and 34.1, 400 keys 85 and 109; 16 requests 1,000 keys 363 and 278; 16 heads of 64 over 8: 64 requests 200
+// keys 49.8 and 44.9, 1,000 keys 195 and 245; 128 requests 1,000 keys 378 and 308.  From three heads a kv head on only the first few
+// keys are quicker that way (12 heads of 128 over 2, 64 requests: 3 keys 9.5 and 5.1, 20 keys 10.0 and 9.3, 64 keys 16.4 and 21.8).
 SHRIKE_API int shrike_attention_fp32_single_form(int num_seqs, int num_heads, int num_kv_heads, int keys) {
   if (keys <= 8) return 2;
-  if (num_kv_heads <= 0 || num_heads / num_kv_heads > 2) return 1;
+  const int share = num_kv_heads > 0 ? num_heads / num_kv_heads : 0;
+  if (share < 1 || share > 2) return 1;
   const long long pairs = static_cast<long long>(num_seqs) * num_kv_heads;
-  return pairs >= 1024 || (pairs >= 256 && keys <= 128) ? 2 : 1;
+  return pairs >= 512 * share || (pairs >= 256 && keys <= 256) || (pairs >= 128 && keys <= 128) ? 2 : 1;
 }
 // A CTA takes its tokens' sequences one after another: with entries of few rows, several of them to a tile of sixteen (us with tiles and
-// with warps: 8 heads of 64 over 8: 8 entries of 2 tokens 26.8 and 4.1, 32 of 4 tokens over 60 keys 23.1 and 14.2, of 8 tokens over
-// 200 keys 44.7 and 73.9; 16 heads over 8: 100 entries of 3 tokens 55.9 and 26.7 [6 rows], 32 of 4 over 60 keys 15.3 and 24.4 [8 rows]).
+// with warps: 8 heads of 64 over 8: 8 entries of 2 tokens 26.8 and 3.5, 32 of 4 tokens over 60 keys 23.1 and 14.7, of 8 tokens over
+// 200 keys 44.2 and 60.9; 16 heads over 8: 100 entries of 3 tokens 55.8 and 26.1 [6 rows], 32 of 4 over 60 keys 15.4 and 21.9 [8 rows]).
 SHRIKE_API int shrike_attention_fp32_portion_form(int num_tokens, int num_seqs, int num_heads, int num_kv_heads) {
   if (num_kv_heads <= 0) return 1;
   return num_seqs > 1 && static_cast<long long>(num_tokens) * (num_heads / num_kv_heads) <= 6LL * num_seqs ? 2 : 1;

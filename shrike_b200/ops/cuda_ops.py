@@ -729,7 +729,9 @@ class CudaOps:
             # 0: none, 1: tiles of rows, 2: a warp a row, with the same bits
             has_single = has_portions = 0
             if max_q_len == 1 or (max_q_len > 1 and min_q_len == 1):
-                reach = max_ctx_len if 0 < max_ctx_len <= self.FEW_KEYS else max_blocks * page_size
+                reach = max_ctx_len if 0 < max_ctx_len <= self.FEW_KEYS else max_blocks * page_size   # the most keys that a row can see
+                if window:
+                    reach = min(reach, abs(window) + keep_first)
                 has_single = self.fp32_attention_form or lib.shrike_attention_fp32_single_form(num_seqs, num_heads, num_kv_heads, reach)
             if max_q_len != 1:   # lengths that are not known among them: that kernel takes entries of any length
                 longer = [length for length in q_lens if length > 1 or not has_single] if q_lens is not None else None

@@ -141,7 +141,8 @@ def test_fp32_attention_of_more_sequences_than_a_grid_has_places():
 
 # the batches that a rule sends to a warp a row, beside ones just short of it: many pairs of one or two heads, few keys, many short entries
 @pytest.mark.parametrize("heads,kv_heads,q_lens,ctx_lens", [
-    (32, 32, [1] * 32, list(range(1, 33))), (32, 32, [1] * 7, [5, 128, 33, 64, 65, 1, 127]), (32, 32, [1] * 8, [5, 128, 33, 64, 65, 1, 127, 31]),
+    (32, 32, [1] * 32, list(range(1, 33))), (32, 32, [1] * 3, [5, 128, 33]), (32, 32, [1] * 4, [5, 128, 33, 64]), (32, 32, [1] * 7, [5, 256, 33, 64, 65, 1, 127]),
+    (32, 32, [1] * 8, [5, 256, 33, 64, 65, 1, 127, 31]), (16, 8, [1] * 128, [300 - i for i in range(128)]),
     (6, 2, [1] * 3, [8, 3, 1]), (6, 2, [1] * 3, [9, 3, 1]), (4, 4, [2, 5, 1, 3], [70, 5, 1, 33]), (4, 2, [3, 3], [40, 3]), (4, 2, [3, 4], [40, 4])])
 def test_fp32_attention_by_either_form_gives_the_same_bits(heads, kv_heads, q_lens, ctx_lens):
     ops = cuda_ops(torch.float32)
