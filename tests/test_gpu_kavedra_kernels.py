@@ -144,6 +144,25 @@ def test_scans_in_a_row_on_one_state_without_anything_between_them(heads, dim, v
     close(state[0, :, : dim * vdim].view(heads, dim, vdim) / big, final / big, 1e-5, "the state left behind")
 
 
+@pytest.mark.parametrize("heads,dim,vdim,n", [(4, 32, 48, 2390), (4, 128, 128, 2500), (5, 64, 40, 3500)])
+def test_scans_of_more_runs_than_sms_equal_the_walk(heads, dim, vdim, n):
+    """156 and 328 CTAs of the runs on a B200's 148 SMs: three an SM; 280: two, for they are one full round."""
+    ops = cuda_ops(torch.float32)
+    decays = [0.9, 0.999, 0.5, 1.0, 0.97][:heads]
+    fused = rnd(n, 2 * heads * dim + heads * vdim, seed=heads + n)
+    d = torch.tensor(decays, dtype=torch.float32, device=DEV)
+    rows, outs, states = fused.to(DEV), [], []
+    for longest in (n, 0):   # in runs, and walked
+        out = torch.full((n, heads * vdim), float("nan"), dtype=torch.float32, device=DEV)
+        state = torch.zeros(1, heads, dim * vdim, dtype=torch.float32, device=DEV)
+        ops.decay_scan(rows, d, state, torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.tensor([0], dtype=torch.int32, device=DEV), out, 1,
+                       heads, dim, vdim, longest=longest)
+        outs.append(out), states.append(state)
+    # either is within 2e-5 of the recurrence in 64 bits
+    close(outs[0] / outs[1].abs().max(), outs[1].cpu() / outs[1].abs().max().cpu(), 4e-5, "outputs")
+    close(states[0] / states[1].abs().max(), states[1].cpu() / states[1].abs().max().cpu(), 4e-5, "the state left behind")
+
+
 def test_a_decay_of_one_keeps_a_token_for_ever_and_a_small_one_forgets_it():
     """One large key and value at the first token, the matching query 900 tokens later: the head with decay 1 returns
     the value in full, the head with decay 0.98 a share of 0.98^900 of it, in the chunked form and walking."""
@@ -349,7 +368,8 @@ def test_every_head_has_its_own_product(dtype, n, heads, padded, vdim):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("n,width,terms,partials", [(1, 64, 0, 1), (9, 96, 1, 1), (40, 72, 2, 3), (3, 128, 5, 2)])
+@pytest.mark.parametrize("n,width,terms,partials", [(1, 64, 0, 1), (9, 96, 1, 1), (40, 72, 2, 3), (3, 128, 5, 2),
+                                                    (1, 1024, 1, 2), (1, 1028, 1, 8), (3, 3584, 2, 4), (2, 3586, 1, 1), (900, 1028, 1, 2)])
 def test_pending_sums_are_added_and_the_rows_joined(dtype, n, width, terms, partials):
     ops = cuda_ops(dtype)
     resid, other = rnd(n, width, seed=1), rnd(n, width, seed=2)

@@ -58,3 +58,28 @@ def test_nucleus_of_tokens_that_hold_all_of_the_mass(vocab):
         ops.sample(logits, torch.tensor(temperature, device=DEV), torch.tensor(top_p, device=DEV), seeds, out)
         ops.check_status()
         assert out[:5].tolist() == [best] * 5 and int(out[5]) in (1, best)
+
+
+# around the vocabularies and batches from which a row is a cluster's and not a block's: a row's token does not depend on which
+@pytest.mark.parametrize("vocab,sizes", [(1535, (1, 8)), (1536, (1, 8, 9)), (2049, (8, 9)), (4095, (8, 9)), (4096, (8, 128, 129)), (11999, (128, 129)),
+                                         (12000, (1, 129))])
+def test_nucleus_sampling_by_a_cluster_or_a_block_draws_the_same_token(vocab, sizes):
+    ops = cuda_ops(torch.float32)
+    rows = max(sizes) + 1
+    logits = rnd(rows, vocab, seed=vocab) * 2.0
+    temperature = 0.5 + torch.rand(rows, generator=torch.Generator().manual_seed(1)).to(DEV)
+    top_p = torch.rand(rows, generator=torch.Generator().manual_seed(2)).clamp(0.05, 0.99).to(DEV)
+    seeds = torch.arange(rows, dtype=torch.int64, device=DEV) * 1000003 + 7
+    outs = []
+    for count in sizes:
+        out = torch.full((count,), -1, dtype=torch.int32, device=DEV)
+        ops.sample(logits[:count].contiguous(), temperature[:count].contiguous(), top_p[:count].contiguous(), seeds[:count].contiguous(), out)
+        outs.append(out)
+    ops.check_status()
+    probs = torch.softmax(logits.double() / temperature.double()[:, None], -1)
+    for out in outs:
+        assert torch.equal(out[: min(sizes)], outs[0][: min(sizes)]) and torch.equal(out, outs[-1][: len(out)])
+        # a kept token: the mass above it is less than top_p (float32 sums: 1e-5)
+        mine = probs[: len(out)].gather(1, out.long()[:, None])
+        above = torch.where(probs[: len(out)] > mine, probs[: len(out)], torch.zeros((), dtype=torch.float64, device=DEV)).sum(1)
+        assert (above < top_p[: len(out)].double() + 1e-5).all()
