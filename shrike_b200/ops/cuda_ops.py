@@ -826,8 +826,9 @@ class CudaOps:
                 self._arrivals = torch.zeros(max(groups, 4096), dtype=torch.int32, device=self.device)
                 self.generation += 1
             scratch, arrivals = self._scratch, self._arrivals
-        short = self.short_portions(max_q_len, max_blocks * page_size, max_ctx_len, head_dim,
-                                    num_heads * (sum(q > 1 or not has_single for q in q_lens) if q_lens is not None else num_seqs))
+        short = has_portions and self.short_portions(
+            max_q_len, max_blocks * page_size, max_ctx_len, head_dim,
+            num_heads * (sum(q > 1 or not has_single for q in q_lens) if q_lens is not None else num_seqs))
         tc_portions = bool(has_portions and self.tensor_core_attention and lib.shrike_attention_tc_available() and not short
                            and page_size in (8, 16, 32, 64) and (own_values or not lib.shrike_attention_tc_own_values()))
         portion_splits, portion_scratch = 1, None
