@@ -116,6 +116,10 @@ class DecoderModel:
         self.head = cls(spec, local_tensors, ops, runtime)
         parts += [self.final_norm, self.head]
         self.capture_safe = all(getattr(part, "capture_safe", False) for part in parts)
+        # decode steps of few sequences may run as one kernel where the kernels offer that for these layers
+        offer = getattr(ops, "decode_step", None)
+        plain = self.pass_entry is None and self.side_table is None and self.residual is None
+        self._whole_step = offer(runtime, self.blocks, config.order) if offer is not None and plain else None
 
     def cache_needs(self):
         """cache id -> KVNeed, and cache id -> StateNeed, over the run order."""
@@ -167,7 +171,10 @@ class DecoderModel:
             self.pass_entry.begin(resid, ctx)   # it keeps what it needs of the embedding's output
         if self.residual is not None:
             resid = self.residual.begin(resid, ctx)   # the residual in its own form (several streams a token)
-        for run in self.config.order:
+        whole = self._whole_step is not None and self._whole_step.takes(ctx)
+        if whole:
+            resid = self._whole_step.run(resid, ctx)
+        for run in () if whole else self.config.order:
             if run.enter is not None:
                 resid, delta = self.pass_entry.forward(resid, delta, ctx, run.enter)
             resid, delta = self.blocks[run.layer].forward(resid, delta, ctx, run)

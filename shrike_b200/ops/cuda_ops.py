@@ -146,6 +146,7 @@ class CudaOps:
         self._held_stream = None
         self._layer_program = None   # the native per-layer issue, built on first use
         self.native_layers = True    # whole layers are issued by one native call where the parts allow it
+        self.whole_steps = dtype == torch.bfloat16   # decode steps of few sequences as one kernel where the model allows it
         self.launches = 0        # launches of this package's own kernels
         self.library_calls = 0   # matrix products handed to cuBLAS
         # library matrix products keep float32 accumulation end to end: no TF32 for float32
@@ -326,6 +327,13 @@ class CudaOps:
 
             self._layer_program = LayerProgram(self)
         return self._layer_program
+
+    def decode_step(self, runtime, blocks, order):
+        """The program that runs all layers of a decode step as one kernel (`ops/decode_step.py`), or None where the model is
+        not one that it serves."""
+        from .decode_step import DecodeStep
+
+        return DecodeStep.of(self, runtime, blocks, order)
 
     # ---- kernels ------------------------------------------------------------
     def embed(self, ids, table, out, previous=None, position_table=None, positions=None, scale=1.0, keep=None):
@@ -635,6 +643,10 @@ class CudaOps:
             42: "gemm_fp32 (tiles): the wait for a free stage ran out",
             43: "gemm_fp32 (tiles): the wait for a loaded stage ran out",
             44: "gemm_fp32: copies still in flight after an aborted wait",
+            51: "decode_step: the weight stream's wait for a free stage ran out",
+            52: "decode_step: a warp's wait for a loaded stage ran out",
+            53: "decode_step: the wait for another CTA's values ran out",
+            54: "decode_step: copies still in flight after an aborted wait",
             31: "sampling: a row of logits had no finite element (NaN logits); token 0 was returned for it",
         }
         return roles.get(code, f"unknown status code {code}")

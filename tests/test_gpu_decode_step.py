@@ -1,0 +1,95 @@
+"""All layers of a decode step as one kernel, against the layer-by-layer path and the plain implementation."""
+
+import numpy as np
+import pytest
+import torch
+
+from shrike_b200.config import parse_config
+from shrike_b200.engine.batch import StepEntry
+from shrike_b200.engine.runner import ModelRunner
+from shrike_b200.weights.random_init import random_tensors
+from tests.gpu_common import TOL, cuda_ops
+from tests.helpers import random_tokens
+from tests.plain import plain_model as pm
+
+pytestmark = pytest.mark.gpu
+
+
+def shape(width, heads, kv_heads, dim, inter, layers=2):
+    return dict(architectures=["Qwen2ForCausalLM"], hidden_size=width, intermediate_size=inter, num_hidden_layers=layers,
+                num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=dim, vocab_size=777, rms_norm_eps=1e-6,
+                rope_theta=1000000.0, tie_word_embeddings=True, max_position_embeddings=32768, eos_token_id=776)
+
+
+# rows of a CTA of one and two tiles of 16, ring stages that end short, rows of the activation that do not fit and come in halves
+SHAPES = {
+    "d64": shape(896, 14, 2, 64, 4864),
+    "d64 one kv head": shape(384, 8, 1, 64, 1280, layers=3),
+    "d64 sixteen to a kv head": shape(256, 16, 1, 64, 1408),
+    "d128": shape(1536, 12, 2, 128, 8960),
+    "d128 every head its own": shape(512, 4, 4, 128, 1280),
+    "d128 wide": shape(3584, 28, 4, 128, 18944, layers=1),
+}
+
+
+def decode(raw, lengths, page_size, whole, steps=3):
+    """Logits of `steps` decode steps of sequences that hold `lengths` tokens, the pools after them, launches of the last step."""
+    config = parse_config(raw)
+    weights = {k: (v.to(torch.bfloat16) if v.dim() >= 2 else v) for k, v in random_tensors(config, 3, "cuda", torch.float32).items()}
+    ops = cuda_ops(torch.bfloat16)
+    pages = sum(-(-(n + steps) // page_size) for n in lengths)
+    runner = ModelRunner(config, weights, ops, "cuda", "bfloat16", page_size=page_size, num_pages=pages, max_slots=len(lengths))
+    sequences = [random_tokens(raw["vocab_size"], n + steps, 50 + i) for i, n in enumerate(lengths)]
+    caches = [runner.cache.open() for _ in lengths]
+    for cache, ids, n in zip(caches, sequences, lengths):
+        if n:
+            runner.cache.append(cache, 0, n)
+            runner.step([StepEntry(cache, ids[:n], 0, [])])
+    ops.whole_steps = whole
+    rows = []
+    for step in range(steps):   # eager, captured, replayed
+        for cache, n in zip(caches, lengths):
+            runner.cache.append(cache, n + step, 1)
+        before = ops.launches
+        out = runner.step([StepEntry(cache, [ids[n + step]], n + step, [0]) for cache, ids, n in zip(caches, sequences, lengths)])
+        launches = ops.launches - before
+        rows.append(out.float().cpu().numpy().copy())
+    ops.check_status()
+    return np.stack(rows), [pool.float().cpu() for pool in runner.storage.kv], launches, weights, sequences
+
+
+# runs of one, two and more tiles of keys (64 or 128), the new key first, last and alone in its tile, lengths that share no page border
+@pytest.mark.parametrize("page_size", [16, 5])
+@pytest.mark.parametrize("key,lengths", [
+    ("d64", (97,)), ("d64", (127, 128, 129, 0)), ("d64", (1, 255, 511, 30, 2)), ("d64 one kv head", (63, 700, 5, 64, 128, 256, 17, 1)),
+    ("d64 sixteen to a kv head", (40, 2600)), ("d128", (0,)), ("d128", (63, 64, 65)), ("d128", (517, 127)), ("d128 every head its own", (3, 700, 128)),
+    ("d128 wide", (77, 1300))])
+def test_a_step_as_one_kernel_gives_the_logits_and_cache_rows_of_the_layers_one_by_one(key, lengths, page_size):
+    raw = SHAPES[key]
+    got, got_pools, launches, weights, sequences = decode(raw, lengths, page_size, True)
+    want, want_pools, one_by_one, _, _ = decode(raw, lengths, page_size, False)
+    assert launches < 6 < one_by_one, "the step was meant to run as one kernel"
+    scale = max(1.0, float(np.abs(want).max()))
+    assert np.isfinite(got).all() and np.abs(got - want).max() <= TOL["bfloat16"] * scale
+    for a, b in zip(got_pools, want_pools):   # rows of earlier tokens the same, the steps' own within bfloat16's rounding of like sums
+        assert (a - b).abs().max() <= TOL["bfloat16"] * max(1.0, float(b.abs().max()))
+    for i, (ids, n) in enumerate(zip(sequences, lengths)):
+        plain = pm.forward(raw, weights, ids, dtype=torch.float64, rounding=pm.ROUNDING_POINTS).cpu().numpy()[n:]
+        assert np.abs(got[:, i] - plain).max() <= TOL["bfloat16"] * max(1.0, float(np.abs(plain).max())), i
+
+
+def test_other_sizes_and_more_sequences_keep_the_layers_one_by_one():
+    ops = cuda_ops(torch.bfloat16)
+    for raw, tokens, served in (("d64", 4, True), ("d64", 8, False), ("d128", 4, True), ("d128", 5, False), ("d128 wide", 2, True),
+                                ("d128 wide", 3, False), ("d64 one kv head", 8, True)):
+        config = parse_config(SHAPES[raw])
+        mixer, ffn = config.layers[0].mixer, config.layers[0].feed_forward
+        from shrike_b200.ops.build import decode_step_library
+        assert bool(decode_step_library().shrike_decode_step_serves(tokens, len(config.layers), mixer.width, mixer.num_heads, mixer.num_kv_heads,
+                                                                    mixer.head_dim, ffn.intermediate)) == served
+    for raw in (shape(448, 7, 1, 64, 1280), shape(512, 4, 2, 128, 1376), shape(512, 32, 16, 32, 1280), dict(SHAPES["d64"], use_sliding_window=True,
+                sliding_window=64, max_window_layers=0)):
+        config = parse_config(raw)
+        weights = {k: (v.to(torch.bfloat16) if v.dim() >= 2 else v) for k, v in random_tensors(config, 3, "cuda", torch.float32).items()}
+        runner = ModelRunner(config, weights, ops, "cuda", "bfloat16", page_size=16, num_pages=8, max_slots=2)
+        assert runner.model._whole_step is None
