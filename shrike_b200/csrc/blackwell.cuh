@@ -96,14 +96,27 @@ __device__ __forceinline__ unsigned instruction_descriptor(int m, int n, bool b_
   return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | (static_cast<unsigned>(n >> 3) << 17) |
          (static_cast<unsigned>(m >> 4) << 24);
 }
-__device__ __forceinline__ void umma(unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+// Products and commits are issued by a whole warp in step, of which one lane's count (`leader`, from elect_one()): behind a
+// branch that one lane takes, the operands are formed and moved per instruction and a product takes about 100 clocks to
+// issue; predicated, with operands that the compiler sees to be the same in all lanes (the warp's number and the tensor
+// memory's address through __shfl_sync), 25.
+__device__ __forceinline__ unsigned elect_one() {
+  unsigned leader;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
+  return leader;
 }
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void umma(unsigned leader, unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc,
+                                     unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void umma_commit(unsigned leader, unsigned long long* bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(smem_u32(bar)), "r"(leader) : "memory");
 }
 // 32 lanes x 32 columns of 32-bit: thread i of the warp gets lane (quarter * 32 + i), columns c .. c + 31.
 __device__ __forceinline__ void tmem_load32(unsigned taddr, unsigned (&r)[32]) {
