@@ -44,7 +44,7 @@ constexpr int BM = 128;        // weight rows per CTA = MMA M
 constexpr int BK = 64;         // k elements per stage: 128 bytes of bf16
 constexpr int UMMA_K = 16;
 constexpr int THREADS = 192;
-constexpr int MAX_STAGES = 8;
+constexpr int MAX_STAGES = 12;
 constexpr size_t A_BYTES = BM * BK * 2;
 
 enum : int { ERR_NONE = 0, ERR_PRODUCER = 1, ERR_MMA = 2, ERR_EPILOGUE = 3, ERR_DRAIN = 4 };
@@ -250,26 +250,34 @@ gemm_swap_ab_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
 }  // namespace tc
 
-// How K is split for a product with `tokens` rows.  Two CTAs live on an SM, and as long as
-// all CTAs of the product are resident together, more of them stream faster: measured at the
-// projection shapes of three model sizes, the time falls with every further split until the
-// grid exceeds the resident places (2 x 148), and jumps by a third right after.  So: the most
-// splits that keep the grid resident, at least three k-blocks each, none empty; at most 8 (what
-// the norm kernel adds in one round trip: a ninth slice costs it what the product gains), or 16
-// where eight would not even give every SM a CTA.  The same function sizes the partial stack.
+// How K is split for a product with `tokens` rows.  Short runs: as often as leaves every CTA an SM of its own, whose whole
+// shared memory is then its ring (below), ten times at most.  So many CTAs with deep rings read about as fast as twice
+// as many with half of it each, and what consumes the product has fewer runs to add (us, 8 tokens, two an SM | one an SM:
+// 5,120 x 5,120 in 7 | 3 runs 9.8 | 10.3, 2,048 x 11,008 in 16 | 9 8.9 | 8.6, 6,144 x 4,096 in 6 | 3 9.5 | 9.6; 43 tokens,
+// 896 x 4,864 in 16 | 10 | 8 4.7 | 4.3 | 4.5).
+// Long runs (beyond 40 k-blocks), and tiles that would leave more than a quarter of the SMs without a CTA (75 to 110
+// tiles; 50 to 55 in two runs): the most runs, eight at most (sixteen where eight would not give every SM a
+// CTA), that keep two CTAs an SM resident together; the time jumps by a third where the grid exceeds that
+// (3,584 x 18,944 in 8 | 5 runs 23.3 | 23.8 us, 10,240 x 5,120 in 3 | 1 18.5 | 20.2).
+// At least three k-blocks a run, none empty.  The same function sizes the stack.
 SHRIKE_API int shrike_gemm_tc_splits(int tokens, int n, int k) {
   (void)tokens;
   const int tiles = (n + tc::BM - 1) / tc::BM;
   const int kblocks = (k + tc::BK - 1) / tc::BK;
-  const int resident = 2 * shrike_device().sm_count;
-  const int most = tiles * 8 < resident / 2 ? 16 : 8;
-  int best = 1;
-  for (int splits = 2; splits <= most && tiles * splits <= resident; ++splits) {
-    const int per = (kblocks + splits - 1) / splits;
-    if (per < 3) break;
-    if ((kblocks + per - 1) / per == splits) best = splits;   // else the last split would be empty
-  }
-  return best;
+  const int sms = shrike_device().sm_count;
+  auto most_runs = [&](int most, int resident) {
+    int best = 1;
+    for (int splits = 2; splits <= most && tiles * splits <= resident; ++splits) {
+      const int per = (kblocks + splits - 1) / splits;
+      if (per < 3) break;
+      if ((kblocks + per - 1) / per == splits) best = splits;   // else the last split would be empty
+    }
+    return best;
+  };
+  const int alone = most_runs(10, sms);
+  const bool busy = tiles * 10 <= sms || sms / tiles * tiles >= sms - sms / 4;
+  if (busy && (kblocks + alone - 1) / alone <= 40) return alone;
+  return most_runs(tiles * 8 < sms ? 16 : 8, 2 * sms);
 }
 
 // x [tokens, k] and w [n, k] bfloat16 row-major, k a multiple of 8 (TMA wants 16-byte row
@@ -296,13 +304,15 @@ static int launch_gemm_tc(const void* x, const void* w, const float* bias, void*
   if ((kblocks + per_split - 1) / per_split != splits) return SHRIKE_BAD_ARGUMENT;
   const size_t stage_bytes = A_BYTES + static_cast<size_t>(tn) * BK * 2;
   const long long ctas = static_cast<long long>((n + BM - 1) / BM) * splits * token_tiles;
-  // Shared memory one CTA may take for its stages.  Half an SM's worth lets two CTAs live on
-  // an SM, so that one streams weights while the other starts up or stores its result, and
-  // still gives each a pipeline deep enough to cover the memory latency alone (three CTAs of
+  // Shared memory one CTA may take for its stages.  A product that gives no SM two CTAs takes nearly the whole of one: what
+  // an SM has in flight and has fetched before the kernel ahead is done then does not shrink for the want of a second CTA
+  // (17,920 x 1,536, 140 CTAs, 37 tokens: 14.3 us with 4 stages, 11.7 with 9; 9,728 x 896, 76 CTAs, 43 tokens: 8.6 and
+  // 6.5).  Half an SM's worth lets two CTAs live on an SM, so that one streams weights while the other starts up or
+  // stores its result, and still gives each a pipeline deep enough to cover the memory latency alone (three CTAs of
   // three stages each measured 7% slower over a whole decode step).  A product of many waves
   // (an output head) does better with four shallower CTAs per SM.
   const ShrikeDevice& device = shrike_device();
-  const int budget = tn <= 16 && ctas >= 6LL * device.sm_count ? 48 * 1024 : 100 * 1024;
+  const int budget = (ctas <= device.sm_count ? 208 : tn <= 16 && ctas >= 6LL * device.sm_count ? 48 : 100) * 1024;
   int stages = static_cast<int>(budget / stage_bytes);
   if (stages < 2) stages = 2;
   stages = stages > MAX_STAGES ? MAX_STAGES : stages;
