@@ -178,18 +178,33 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
 // the bisection's lower end can never count again and is dropped from its thread's list, in place, now and then.  The sums are those of one block of 1,024 threads that walk the row with a
 // stride of 1,024, to the bit: thread t of CTA r is that block's thread 128 r + t, dropped entries add nothing, and the 32
 // warps' sums meet in one warp in the same order.
-// Measured (one B200): 64 rows of 152,064 logits with top_p 0.95: 221 us, and 1,391 with a block a row that reads the row
-// from memory thirty times.
-constexpr int ROW_CTAS = 8, ROW_THREADS = SAMPLE_THREADS / ROW_CTAS;
+// Two CTAs fill an SM's shared memory, so the time is that of their few warps: HELP threads share what a place's entries cost
+// one by one (copies, exponentials, the draw's noise).
+// Measured (one B200): 64 rows of 152,064 logits with top_p 0.95: 180 us (220 with one thread a place and the row read
+// through registers, 191 with four, which also slow rows of a few thousand down: 64 rows of 5,000 47 and 73), one row 69 (90);
+// and 1,391 with a block a row that reads the row from memory thirty times.
+constexpr int ROW_CTAS = 8, ROW_THREADS = SAMPLE_THREADS / ROW_CTAS, HELP = 2;
 
 struct RowShare {
   float warps[2][4][32];   // up to four values per warp of the cluster, two buffers: one barrier a sum
   Best best[ROW_CTAS];
 };
 
+// Every HELP-th of the row's entries x[0], x[SAMPLE_THREADS], ... that belong to a place, from the `which`-th on, into
+// shared memory.  All copies are under way together: read through registers, eight at a time and eight warps an SM, a row
+// came at a sixth of the memory's rate.
+__device__ __forceinline__ void fetch_entries(float* place, const float* x, int which, int count) {
+  const unsigned to = static_cast<unsigned>(__cvta_generic_to_shared(place));
+#pragma unroll 4
+  for (int j = which; j < count; j += HELP)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to + j * static_cast<unsigned>(ROW_THREADS * sizeof(float))),
+                 "l"(x + static_cast<size_t>(j) * SAMPLE_THREADS) : "memory");
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 __device__ __forceinline__ void row_publish(float4 mine, RowShare& share, int buffer, cooperative_groups::cluster_group& cluster) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane < ROW_CTAS) {
+  if (lane < ROW_CTAS && warp < ROW_THREADS / 32) {
     RowShare* to = cluster.map_shared_rank(&share, lane);
     const int at = cluster.block_rank() * (ROW_THREADS / 32) + warp;
     to->warps[buffer][0][at] = mine.x;
@@ -200,7 +215,7 @@ __device__ __forceinline__ void row_publish(float4 mine, RowShare& share, int bu
   cluster.sync();
 }
 
-__global__ void __launch_bounds__(ROW_THREADS)
+__global__ void __launch_bounds__(ROW_THREADS * HELP)
 sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
                       const float* __restrict__ top_p, const long long* __restrict__ seeds, int* __restrict__ out,
                       const float* __restrict__ partial_value, const int* __restrict__ partial_index, int vocab,
@@ -217,7 +232,7 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
   if (temp == 0.f || nucleus >= 1.0f) {
     if (rank != 0) return;
     Best mine{-INFINITY, 0x7fffffff};
-    for (int i = threadIdx.x; i < chunks; i += ROW_THREADS)
+    for (int i = threadIdx.x; i < chunks; i += ROW_THREADS * HELP)
       mine = better(mine, Best{partial_value[static_cast<size_t>(row) * chunks + i],
                                partial_index[static_cast<size_t>(row) * chunks + i]});
     const Best top = block_best(mine, best_scratch);
@@ -226,31 +241,33 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
   }
   cluster.sync();   // every CTA of the cluster runs: its shared memory may be written from the others
   const float* x = logits + static_cast<size_t>(row) * vocab;
-  float* own = held + threadIdx.x;
-  const int first = rank * ROW_THREADS + threadIdx.x;
-  int count = first < vocab ? (vocab - first + SAMPLE_THREADS - 1) / SAMPLE_THREADS : 0;
+  // A place's entries are shared out among HELP threads wherever each stands for itself; what is added up in order, and the
+  // list of the bisection, is the first's alone (the others go along with a list of none).
+  const int place = threadIdx.x % ROW_THREADS, which = threadIdx.x / ROW_THREADS;
+  float* own = held + place;
+  const int first = rank * ROW_THREADS + place;
+  const int all = first < vocab ? (vocab - first + SAMPLE_THREADS - 1) / SAMPLE_THREADS : 0;
+  int count = which == 0 ? all : 0;
   const float inv_temp = 1.0f / temp;
   float local_max = -INFINITY;
+  fetch_entries(own, x + first, which, all);
+  __syncthreads();
 #pragma unroll 8
-  for (int j = 0; j < count; ++j) {
-    const float v = x[first + j * SAMPLE_THREADS];
-    own[j * ROW_THREADS] = v;
-    local_max = fmaxf(local_max, v);
-  }
+  for (int j = 0; j < count; ++j) local_max = fmaxf(local_max, own[j * ROW_THREADS]);
   row_publish(make_float4(warp_max(local_max), 0.f, 0.f, 0.f), share, 0, cluster);
   const float row_max = warp_max(share.warps[0][0][lane]);
-  float local_sum = 0.f;
 #pragma unroll 4
-  for (int j = 0; j < count; ++j) {
-    const float e = expf((own[j * ROW_THREADS] - row_max) * inv_temp);
-    own[j * ROW_THREADS] = e;
-    local_sum += e;
-  }
+  for (int j = which; j < all; j += HELP) own[j * ROW_THREADS] = expf((own[j * ROW_THREADS] - row_max) * inv_temp);
+  __syncthreads();
+  float local_sum = 0.f;
+#pragma unroll 8
+  for (int j = 0; j < count; ++j) local_sum += own[j * ROW_THREADS];
   row_publish(make_float4(warp_sum(local_sum), 0.f, 0.f, 0.f), share, 1, cluster);
   const float total = warp_sum(share.warps[1][0][lane]);
   const float inv_total = 1.0f / total;
 #pragma unroll 4
-  for (int j = 0; j < count; ++j) own[j * ROW_THREADS] *= inv_total;
+  for (int j = which; j < all; j += HELP) own[j * ROW_THREADS] *= inv_total;
+  __syncthreads();
   // Bisection on the bit pattern of a positive float: mass_above(lo) >= top_p and
   // mass_above(hi) < top_p hold throughout; at the end no probability lies
   // strictly between lo and hi, and the kept set is {p > lo}.
@@ -305,16 +322,13 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
   const float threshold = lo == 0u ? -1.f : __uint_as_float(lo);
   Best mine{-INFINITY, 0x7fffffff};
   const unsigned long long seed = static_cast<unsigned long long>(seeds[row]);
-  for (int i0 = first; i0 < vocab; i0 += 8 * SAMPLE_THREADS) {
-    float v[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = i0 + e * SAMPLE_THREADS < vocab ? x[i0 + e * SAMPLE_THREADS] : -INFINITY;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int i = i0 + e * SAMPLE_THREADS;
-      const float p = expf((v[e] - row_max) * inv_temp) * inv_total;
-      if (i < vocab && p > threshold) mine = better(mine, Best{v[e] * inv_temp + gumbel(seed, i), i});
-    }
+  __syncthreads();   // the logits once more, over what the bisection left of their probabilities
+  fetch_entries(own, x + first, which, all);
+#pragma unroll 4
+  for (int j = which; j < all; j += HELP) {
+    const int i = first + j * SAMPLE_THREADS;
+    const float v = own[j * ROW_THREADS], p = expf((v - row_max) * inv_temp) * inv_total;
+    if (p > threshold) mine = better(mine, Best{v * inv_temp + gumbel(seed, i), i});
   }
   const Best top = block_best(mine, best_scratch);
   if (threadIdx.x == 0) cluster.map_shared_rank(&share, 0)->best[rank] = top;
@@ -350,7 +364,7 @@ int launch_sample(const float* logits, const float* temperature, const float* to
     static PerDevice raised;
     const int rc = shrike_raise_smem(raised, sample_cluster_kernel, MOST);
     if (rc != 0) return rc;
-    err = launch_dependent_clusters(sample_cluster_kernel, dim3(rows * ROW_CTAS), dim3(ROW_THREADS), smem, stream, ROW_CTAS, logits,
+    err = launch_dependent_clusters(sample_cluster_kernel, dim3(rows * ROW_CTAS), dim3(ROW_THREADS * HELP), smem, stream, ROW_CTAS, logits,
                                     temperature, top_p, seeds, out, static_cast<const float*>(scratch_value),
                                     static_cast<const int*>(scratch_index), vocab, chunks, status);
   } else {
