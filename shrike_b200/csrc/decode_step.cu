@@ -22,10 +22,18 @@
 // How CTAs hand values on.  Every value that crosses CTAs travels as one 64-bit word with the number of the exchange beside it:
 // a reader polls the very words it needs until they carry the number it expects.  That takes one trip to L2 to write
 // and one to read, where stores, a fence, a counter, a poll and the loads took 1.5 us (fence and counter 0.7, poll 0.4, loads 0.4).
-// The numbers grow with every layer and launch, so nothing is ever cleared.  One buffer an exchange suffices: whoever writes it
-// again has read, directly or through others, what every reader of the old content wrote after reading it.  (Output rows need
-// all heads, every gated unit needs all output rows, down rows need all units, the next q/k/v rows need all down rows; a
-// pair's queries need rows of CTAs that have all of that behind them.)
+// The numbers grow with every layer and launch, so nothing is ever cleared.  A reader wants the very number it expects, so a
+// word may be written again only when all its readers have it.  One buffer an exchange suffices, because every reader publishes
+// something after it has read, and whoever writes the words again has read that, directly or through others:
+//   residual, part 0  read by the CTAs with q/k/v rows; the output rows that replace it need all heads, those need all q/k/v rows.
+//                     A CTA without such rows must not read it: nothing that waits for that CTA lies between the two.
+//   q/k/v             read by the CTAs with a pair; the next layer's rows need all down rows, those all gated units, of which
+//                     every CTA has one, and it comes to that behind its attention.
+//   runs' sums        read by the CTAs with a pair, replaced by them behind the next q/k/v rows: as above.
+//   heads             read by all CTAs in part 1; replaced behind the next q/k/v rows, which need every CTA's gated units.
+//   residual, part 2  read by all CTAs; the down rows that replace it need all gated units.
+//   activation        read by the CTAs with down rows; the next units need all output rows, those all heads, those the q/k/v rows,
+//                     and each of those needs all down rows.
 //
 // Rounding points are those of the separate kernels: normed rows, rotated q and k, v, probabilities, attention output,
 // gate, up and their product in bfloat16, all sums in float32.
@@ -196,8 +204,12 @@ __device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
 }
 
+// Whether CTA `cta` has rows of a product other than the gated one.
+__host__ __device__ inline bool has_rows(const Product& g, int cta) { return cta * g.rows < g.n; }
+// Whether it reads the residual words in part 0 (see above: those it writes q/k/v rows with, and no others).
+__host__ __device__ inline bool reads_residual(const Product* products, int cta) { return has_rows(products[0], cta); }
 // The gated product's units of 8 features that CTA `cta` of `ctas` takes: [first, end).
-__device__ __forceinline__ void units_of(int inter, int cta, int ctas, int& first, int& end) {
+__host__ __device__ __forceinline__ void units_of(int inter, int cta, int ctas, int& first, int& end) {
   const long long units = inter / 8;
   first = static_cast<int>(units * cta / ctas);
   end = static_cast<int>(units * (cta + 1) / ctas);
@@ -222,7 +234,7 @@ __device__ __forceinline__ void stream_weights(const Args& a, Shared* sh, unsign
       const CUtensorMap* map = &a.layers[l].maps[p];
       if (FETCH) prefetch_map(map);
       const int row = blockIdx.x * g.rows;
-      const int first = p == 2 ? first_unit : 0, end = p == 2 ? end_unit : (row < g.n ? 1 : 0);
+      const int first = p == 2 ? first_unit : 0, end = p == 2 ? end_unit : (has_rows(g, blockIdx.x) ? 1 : 0);
       const unsigned bytes = static_cast<unsigned>(g.rows * g.depth * 128);
 #pragma unroll 1
       for (int u = first; u < end && ok; ++u) {
@@ -390,7 +402,12 @@ struct Compute {
       }
     }
   }
-  __device__ __forceinline__ void norm(float eps) {
+  __device__ __forceinline__ void norm(float eps, bool reads) {
+    if (!reads) {
+      copy_wait<0>();   // the gains and the tile: their places are written again
+      compute_sync();
+      return;
+    }
     const int pitch = a.width * 2 + 16, pairs = a.width / 2;
     int spread = a.tokens == 1 ? 3 : (a.tokens == 2 ? 2 : (a.tokens <= 4 ? 1 : 0));   // few rows: several warps each
     while (spread < 3 && pairs > (16 * 32 << spread)) ++spread;
@@ -552,7 +569,7 @@ struct Compute {
   __device__ __forceinline__ void rows_product(int p, float bias, bool last) {
     const Product g = a.products[p];
     const int row0 = blockIdx.x * g.rows;
-    if (row0 >= g.n) return;
+    if (!has_rows(g, blockIdx.x)) return;
     float acc[2 * MT][4] = {};   // two chains: a product waits for the one before it on the same sums
     // the input's rows: whole, or (the activation's, where they do not fit) columns a half of x at a time
     const bool whole = p != 3 || a.tokens * (g.chunks * 128 + 16) <= X_BYTES;
@@ -937,7 +954,7 @@ struct Compute {
         // out and hold all parts' addresses over the layers
         int p = at;
         asm volatile("" : "+r"(p), "+r"(tid), "+r"(warp), "+r"(lane));
-        if (p == 0 || p == 2) norm(p == 0 ? layer.eps_mixer : layer.eps_ffn);
+        if (p == 0 || p == 2) norm(p == 0 ? layer.eps_mixer : layer.eps_ffn, p == 2 || reads_residual(a.products, blockIdx.x));
         else if (p == 1 || !last) bring_gain(p == 1 ? layer.norm_ffn : fields[l + 1].norm_mixer);
         if (p == 1) {
           rows_in(a.x_attn, a.heads * D, x_mem, a.heads * D * 2 + 16, 0, a.heads * D);
@@ -1107,6 +1124,22 @@ struct ShrikeStepArgs {
 SHRIKE_API int shrike_decode_step_serves(int tokens, int layers, int width, int heads, int kv_heads, int head_dim, int inter) {
   step::Cuts cuts;
   return step::cuts_of(tokens, layers, width, heads, kv_heads, head_dim, inter, &cuts) ? 1 : 0;
+}
+// What each of `ctas` CTAs does in a layer, on the host: bit p of roles[cta] says that it has rows (units) of product p, bit 4
+// that it reads the residual words in part 0.
+SHRIKE_API int shrike_decode_step_roles(int ctas, int width, int heads, int kv_heads, int head_dim, int inter, int* roles) {
+  using namespace step;
+  Product p[4];
+  if (!cut((heads + 2 * kv_heads) * head_dim, width, ctas, false, &p[0]) || !cut(width, heads * head_dim, ctas, false, &p[1]) ||
+      !cut(2 * inter, width, ctas, true, &p[2]) || !cut(width, inter, ctas, false, &p[3]))
+    return SHRIKE_BAD_ARGUMENT;
+  for (int cta = 0; cta < ctas; ++cta) {
+    int first, end;
+    units_of(inter, cta, ctas, first, end);
+    roles[cta] = (has_rows(p[0], cta) ? 1 : 0) | (has_rows(p[1], cta) ? 2 : 0) | (first < end ? 4 : 0) | (has_rows(p[3], cta) ? 8 : 0) |
+                 (reads_residual(p, cta) ? 16 : 0);
+  }
+  return SHRIKE_OK;
 }
 SHRIKE_API int shrike_decode_step_layer_bytes() { return static_cast<int>(sizeof(step::Layer)); }
 // 64-bit words that the exchanges of a step of up to `tokens` tokens take.

@@ -1,0 +1,131 @@
+"""The one-kernel decode step's exchanges, walked through on the host: CTAs hand values on as words that carry the number of the
+exchange, and a reader that comes after its words were written again would wait for a number that is gone."""
+
+import ctypes
+
+import pytest
+
+from shrike_b200.ops import build
+
+CTAS = 148
+WIDTHS = {   # width, heads, kv heads, head size, intermediate
+    "0.5b": (896, 14, 2, 64, 4864), "1.5b": (1536, 12, 2, 128, 8960), "3b": (2048, 16, 2, 128, 11008), "7b": (3584, 28, 4, 128, 18944),
+    "one kv head": (384, 8, 1, 64, 1280), "every head its own": (512, 4, 4, 128, 1280),
+}
+ROWS = (1, 2, 4, 8)   # bits of a CTA's role: it has rows (units) of q/k/v, output, gate/up, down
+READS = 16            # it reads the residual words in part 0
+
+
+def roles_of(sizes, ctas=CTAS):
+    roles = (ctypes.c_int * ctas)()
+    assert build.decode_step_library().shrike_decode_step_roles(ctas, *sizes, roles) == 0
+    return list(roles)
+
+
+def cta_of_row(sizes, ctas=CTAS):
+    """Which CTA writes a row of q/k/v: equal shares, rounded up to four."""
+    _width, heads, kv_heads, dim, _inter = sizes
+    each = -(-(-(-(heads + 2 * kv_heads) * dim // ctas)) // 4) * 4
+    return lambda row: row // each
+
+
+def walk(sizes, roles, tokens, runs, slow, layers=3):
+    """Runs the layers' exchanges with CTA `slow` held up: it goes one step on only when no other can.  Returns the CTAs that
+    found a word already written again, and whether all came to the end."""
+    _width, heads, kv_heads, dim, _inter = sizes
+    ctas, group, owner = len(roles), heads // kv_heads, cta_of_row(sizes)
+    pairs = [(t, h, r) for t in range(tokens) for h in range(kv_heads) for r in range(runs)]
+    assert len(pairs) <= ctas
+    words = {name: [-1] * ctas for name in ("residual", "qkv", "sums", "heads", "activation")}
+    has = [[c for c in range(ctas) if roles[c] & bit] for bit in ROWS]
+
+    def qkv_owners(h, last):
+        rows = list(range(h * group * dim, (h + 1) * group * dim))
+        if last:   # the run that holds the step's own key and value
+            for plane in (0, 1):
+                first = (heads + plane * kv_heads + h) * dim
+                rows += range(first, first + dim)
+        return sorted({owner(row) for row in rows})
+
+    def cta(c):
+        def put(name, number):
+            words[name][c] = number
+
+        if roles[c] & 2:
+            put("residual", 0)
+        for layer in range(layers):
+            number = 2 * layer
+            if roles[c] & READS:
+                yield "residual", has[1], number
+            if roles[c] & 1:
+                put("qkv", number)
+            if c < len(pairs):
+                _t, h, r = pairs[c]
+                yield "qkv", qkv_owners(h, r == runs - 1), number
+                if runs > 1:
+                    put("sums", number)
+                    yield "sums", range(c - r, c - r + runs), number
+                put("heads", number)
+            yield "heads", range(len(pairs)), number
+            if roles[c] & 2:
+                put("residual", number + 1)
+            yield "residual", has[1], number + 1
+            put("activation", number + 1)
+            if roles[c] & 8:
+                yield "activation", range(ctas), number + 1
+                put("residual", number + 2)
+        return
+
+    agents = {c: cta(c) for c in range(ctas)}
+    waits = {}
+    for c in range(ctas):
+        if c != slow:
+            waits[c] = next(agents[c], None)
+    missed, held = [], True   # `held`: the slow one has not begun
+    while waits and not missed:
+        moved = False
+        for c in sorted(waits):
+            if c == slow:
+                continue
+            while waits[c] is not None and all(words[waits[c][0]][o] == waits[c][2] for o in waits[c][1]):
+                moved = True
+                waits[c] = next(agents[c], None)
+            if waits[c] is None:
+                del waits[c]
+            elif any(words[waits[c][0]][o] > waits[c][2] for o in waits[c][1]):
+                missed.append(c)
+        if moved:
+            continue
+        if held:
+            held = False
+            waits[slow] = next(agents[slow], None)
+        elif slow in waits and all(words[waits[slow][0]][o] == waits[slow][2] for o in waits[slow][1]):
+            waits[slow] = next(agents[slow], None)
+        elif slow in waits and any(words[waits[slow][0]][o] > waits[slow][2] for o in waits[slow][1]):
+            missed.append(slow)
+        else:
+            break
+        if slow in waits and waits[slow] is None:
+            del waits[slow]
+    return missed, not waits
+
+
+@pytest.mark.parametrize("tokens,runs", [(1, 1), (1, 16), (2, 3)])
+@pytest.mark.parametrize("key", list(WIDTHS))
+def test_no_cta_finds_its_words_written_again_whichever_is_held_up(key, tokens, runs):
+    sizes = WIDTHS[key]
+    roles = roles_of(sizes)
+    pairs = tokens * runs * sizes[2]
+    without = [c for c in range(CTAS) if not roles[c] & 1]
+    assert all(role & 4 for role in roles)   # every CTA has a gated unit: most of the order rests on it
+    for slow in sorted({0, pairs - 1, pairs, CTAS // 2, CTAS - 1, *without[:1], *without[-1:]}):
+        assert walk(sizes, roles, tokens, runs, slow) == ([], True), slow
+
+
+def test_a_reader_of_the_residual_that_writes_no_rows_would_miss_it():
+    """What the roles are for: with every CTA reading the residual in part 0, one without q/k/v rows and without a pair finds the
+    next number there when it is held up."""
+    sizes = WIDTHS["0.5b"]
+    roles = [role | READS for role in roles_of(sizes)]
+    idle = [c for c in range(CTAS) if not roles[c] & 1]
+    assert idle and walk(sizes, roles, 1, 1, idle[0]) == ([idle[0]], False)
