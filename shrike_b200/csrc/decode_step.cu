@@ -200,6 +200,12 @@ __device__ __forceinline__ void fetch_box5(const CUtensorMap* map, int half, int
   asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global [%0, {%1, %2, %3, %4, %5}];" ::"l"(reinterpret_cast<unsigned long long>(map)),
                "r"(0), "r"(half), "r"(0), "r"(run), "r"(chunk) : "memory");
 }
+// Before a map in global memory is used: what the host's copy wrote there, and not an earlier table's map at this address that a
+// descriptor cache may still hold.  The streaming warpgroup does it for all layers at once and meets (24 layers: no time that
+// shows; map by map in the two threads that use them 0.7 us each, 65 us a step).
+__device__ __forceinline__ void acquire_map(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
+}
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
 }
@@ -1003,6 +1009,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_step_kernel(const __grid_co
   __syncthreads();
   if (threadIdx.x >= COMPUTE) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(STREAM_REGISTERS));
+    for (int i = threadIdx.x - COMPUTE; i < 4 * a.num_layers; i += THREADS - COMPUTE) acquire_map(&a.layers[i >> 2].maps[i & 3]);
+    asm volatile("bar.sync 2, %0;" ::"n"(THREADS - COMPUTE) : "memory");
     if (threadIdx.x == COMPUTE) stream_weights<false>(a, sh, smem_u32(ring));
     if (threadIdx.x == COMPUTE + 32) stream_weights<true>(a, sh, smem_u32(ring));
     __syncwarp();
