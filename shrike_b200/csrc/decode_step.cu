@@ -679,7 +679,9 @@ struct Compute {
   // The pool's row of key `key`, or -1: only keys of earlier positions (the step's own comes from `rotate`).
   __device__ __forceinline__ int pool_row(int key) const {
     if (key >= min(key_end, context - 1)) return -1;
-    const int page = __ldg(a.block_table + static_cast<size_t>(pair_token) * a.max_blocks + key / a.page_size);
+    const int block = key / a.page_size;
+    if (block >= a.max_blocks) return -1;   // never read beyond the sequence's own row of the table
+    const int page = __ldg(a.block_table + static_cast<size_t>(pair_token) * a.max_blocks + block);
     return page >= 0 && page < a.num_pages ? page * a.page_size + key % a.page_size : -1;
   }
   // Where tile `j` of the run lies: keys, then values.

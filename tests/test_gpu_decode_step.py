@@ -93,3 +93,42 @@ def test_other_sizes_and_more_sequences_keep_the_layers_one_by_one():
         weights = {k: (v.to(torch.bfloat16) if v.dim() >= 2 else v) for k, v in random_tensors(config, 3, "cuda", torch.float32).items()}
         runner = ModelRunner(config, weights, ops, "cuda", "bfloat16", page_size=16, num_pages=8, max_slots=2)
         assert runner.model._whole_step is None
+
+
+def runner_of(raw, requests, page_size=16, tokens=700, ops=None):
+    config = parse_config(raw)
+    weights = {k: (v.to(torch.bfloat16) if v.dim() >= 2 else v) for k, v in random_tensors(config, 3, "cuda", torch.float32).items()}
+    return ModelRunner(config, weights, ops or cuda_ops(torch.bfloat16), "cuda", "bfloat16", page_size=page_size,
+                       num_pages=requests * -(-tokens // page_size), max_slots=requests)
+
+
+def opened(runner, ids, count):
+    """A request whose cache holds the first `count` of `ids` and has room for one token more."""
+    cache = runner.cache.open()
+    if count:
+        runner.cache.append(cache, 0, count)
+        runner.step([StepEntry(cache, ids[:count], 0, [])])
+    runner.cache.append(cache, count, 1)
+    return cache
+
+
+def test_nothing_is_read_beyond_a_sequences_row_of_the_block_table():
+    """A context longer than the row: keys beyond it count as zeros, whatever stands in the next sequence's row."""
+    raw, lengths = SHAPES["d64"], (230, 90, 150)
+    runner = runner_of(raw, 3, page_size=5)
+    sequences = [random_tokens(raw["vocab_size"], n + 1, 50 + i) for i, n in enumerate(lengths)]
+    caches = [opened(runner, ids, n) for ids, n in zip(sequences, lengths)]
+    seen = []
+    with torch.inference_mode():
+        for other in (1, 2):   # the row behind the first one's
+            entries = [StepEntry(caches[i], [sequences[i][-1]], lengths[i], [0]) for i in (0, other)]
+            ctx = runner.builder.build(entries)
+            view = ctx.groups[0]
+            view.max_blocks = 32   # of the 47 blocks that the first one's context spans
+            view.block_table = view.block_table[:, :32].contiguous()
+            before = runner.ops.launches
+            logits, _ = runner._run(ctx, False)
+            assert runner.ops.launches - before < 6
+            seen.append(logits[0].float().cpu().numpy().copy())
+    runner.ops.check_status()
+    assert np.isfinite(seen[0]).all() and np.array_equal(seen[0], seen[1])
