@@ -19,6 +19,7 @@ import numpy as np
 import torch
 
 
+FEW_ENTRIES = 8    # up to so many single tokens a batch knows whether its entries keep out of one another's pages
 FIRST_GROUP = 11   # index of the first per-group part of the packed block (see BatchBuilder.stage)
 
 
@@ -60,6 +61,7 @@ class StepContext:
     starts: list[int]
     slots: list[int]  # host copy of state_slot
     all_single: bool = False  # every entry brings exactly one token
+    apart: bool = False  # up to FEW_ENTRIES single tokens, none of which goes to a page that another entry holds
     sample_temperature: torch.Tensor | None = None  # float32 [R], when every wanted row is sampled
     sample_top_p: torch.Tensor | None = None  # float32 [R]
     sample_seed: torch.Tensor | None = None  # int64 [R]
@@ -87,6 +89,7 @@ class Staged:
     host: object = None        # the pinned buffer that holds the block until `commit` copies it
     turn: int = 0
     committed: bool = False
+    apart: bool = False        # as StepContext.apart
 
 
 class BatchBuilder:
@@ -185,7 +188,9 @@ class BatchBuilder:
         if pad > 0:
             start_arr[real:] = 0
 
+        apart = False
         if max(q_lens) == 1:
+            apart = s <= FEW_ENTRIES
             # the steady state of decoding: one token per entry, filled without per-token work
             ids[:real] = [e.tokens[0] for e in entries]
             pos[:real] = starts
@@ -231,6 +236,9 @@ class BatchBuilder:
                 if pad:
                     slots[real:] = -1
                     table2d[real:, 0] = 0
+                if apart and real > 1:   # two tokens of one request, or of two that share a page: the later one reads the other's key
+                    reached = table2d[:real, [start // page for start in starts]] == slots[:real] // page
+                    apart = int(np.count_nonzero(reached)) == real   # each reaches its own
         else:
             self._fill_general(entries, q_lens, parts, max_blocks, sampled, page, s)
 
@@ -238,7 +246,7 @@ class BatchBuilder:
             q_lens, starts = q_lens + [1] * pad, starts + [0] * pad
             ctx_lens, slots_host = ctx_lens + [1] * pad, slots_host + [-1] * pad
         staged = Staged(n, s, r, max_blocks, sizes, offsets, total, sampled, q_lens, starts, ctx_lens, slots_host,
-                        rows=r - pad, host=host, turn=self._turn)
+                        rows=r - pad, host=host, turn=self._turn, apart=apart)
         if not defer:
             self.commit(staged)
         return staged
@@ -278,7 +286,7 @@ class BatchBuilder:
             ctx_len=views[7], state_slot=views[8], seq_start=views[10], out_rows=views[9], groups=groups,
             storage=self.storage, max_q_len=max(staged.q_lens), min_q_len=min(staged.q_lens),
             max_ctx_len=max(staged.ctx_lens), q_lens=staged.q_lens, starts=staged.starts, slots=staged.slots,
-            all_single=max(staged.q_lens) == 1,
+            all_single=max(staged.q_lens) == 1, apart=staged.apart,
             sample_temperature=views[1].view(torch.float32) if sampled else None,
             sample_top_p=views[2].view(torch.float32) if sampled else None,
             sample_seed=views[0].view(torch.int64) if sampled else None,

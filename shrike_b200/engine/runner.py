@@ -180,9 +180,9 @@ class ModelRunner:
                      and (decode or self.capture_portions))
         # what a captured launch sequence has baked in: the number of entries, every entry's
         # length (grids and shapes follow from them), the number of wanted rows, the table widths, and whether the
-        # contexts are of those for which other kernels run
+        # contexts, or entries that share pages, are of those for which other kernels run
         contexts = self.ops.context_class(decode, max(staged.ctx_lens)) if hasattr(self.ops, "context_class") else 0
-        key = (staged.s if decode else tuple(staged.q_lens), staged.r, tuple(staged.max_blocks), sample, contexts)
+        key = (staged.s if decode else tuple(staged.q_lens), staged.r, tuple(staged.max_blocks), sample, contexts, staged.apart)
         return Prepared(staged, sample, graphable, key, decode)
 
     def fetch(self, tokens: torch.Tensor):

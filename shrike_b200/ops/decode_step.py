@@ -102,7 +102,8 @@ class DecodeStep:
         return held
 
     def takes(self, ctx) -> bool:
-        return (ctx.all_single and ctx.num_tokens <= self.MAX_TOKENS and getattr(self.ops, "whole_steps", False)
+        # keys of earlier positions are read while this step's are still being written: no entry may bring another's
+        return (ctx.all_single and ctx.apart and ctx.num_tokens <= self.MAX_TOKENS and getattr(self.ops, "whole_steps", False)
                 and self._serves(ctx.num_tokens))
 
     def _tables(self, storage) -> None:

@@ -2,10 +2,15 @@
 exchange, and a reader that comes after its words were written again would wait for a number that is gone."""
 
 import ctypes
+from types import SimpleNamespace
 
 import pytest
+import torch
 
+from shrike_b200.cache.manager import CacheManager, KVGroupSpec
+from shrike_b200.engine.batch import BatchBuilder, StepEntry
 from shrike_b200.ops import build
+from shrike_b200.ops.decode_step import DecodeStep
 
 CTAS = 148
 WIDTHS = {   # width, heads, kv heads, head size, intermediate
@@ -129,3 +134,38 @@ def test_a_reader_of_the_residual_that_writes_no_rows_would_miss_it():
     roles = [role | READS for role in roles_of(sizes)]
     idle = [c for c in range(CTAS) if not roles[c] & 1]
     assert idle and walk(sizes, roles, 1, 1, idle[0]) == ([idle[0]], False)
+
+
+def held(manager, count):
+    cache = manager.open()
+    manager.append(cache, 0, count)
+    return cache
+
+
+@pytest.mark.parametrize("groups", [1, 2])
+def test_entries_that_share_a_page_with_a_new_token_are_left_to_the_layers_one_by_one(groups):
+    """Such an entry may read the key that another of the same step stores: the layers one by one store all keys first."""
+    manager = CacheManager([KVGroupSpec((g,), 2, 64, None) for g in range(groups)], 4, 64, 16)
+    builder = BatchBuilder(4, groups, "cpu", None)
+    step = object.__new__(DecodeStep)
+    step.ops = SimpleNamespace(whole_steps=True)
+    step._served = {n: True for n in range(1, 9)}
+    a, b, c = held(manager, 12), held(manager, 9), held(manager, 12)
+
+    def taken(*entries, pad_to=0):
+        staged = builder.stage([StepEntry(cache, [1] * count, start, [0]) for cache, start, count in entries], pad_to=pad_to)
+        return step.takes(builder.context(staged))
+
+    assert taken((a, 11, 1)) and taken((a, 11, 1), (b, 8, 1), (c, 11, 1)) and taken((a, 11, 1), (b, 8, 1), pad_to=8)
+    assert not taken((a, 10, 1), (a, 11, 1))                    # neighbours on one page
+    assert not taken((a, 8, 1), (a, 7, 1))                      # across a page's border
+    assert not taken((a, 3, 1), (b, 8, 1), (a, 11, 1))          # pages apart, which the later one reads all the same
+    assert not taken((a, 11, 1), (a, 11, 1))
+    assert not taken((a, 10, 2), (b, 8, 1))                     # no step of single tokens
+    shared = held(manager, 4)                                   # another request, whose first page is a's
+    for table, other in zip(shared.tables, a.tables):
+        table.pages[0] = other.pages[0]
+    assert taken((a, 11, 1), (shared, 3, 1)) is False and taken((b, 8, 1), (shared, 3, 1))
+    many = [(held(manager, 1), 0, 1) for _ in range(9)]
+    assert taken(*many[:8]) and not taken(*many)
+    assert torch.equal(builder.build([StepEntry(a, [1], 11, [0])]).ctx_len, torch.tensor([12], dtype=torch.int32))
