@@ -72,6 +72,7 @@ constexpr int MAX_ROWS = 32;                   // weight rows of a CTA in a prod
 constexpr int MAX_LAYERS = 96;
 constexpr unsigned POLL_LIMIT = 4000000u;      // looks at a word before it is given up: seconds
 
+constexpr int NOT_TOGETHER = -2;   // the launcher's answer where the device will not run all CTAs at once: nothing has run
 enum : int { ERR_PRODUCER = 51, ERR_STAGE = 52, ERR_WORD = 53, ERR_DRAIN = 54 };
 
 // A product: `n` rows of weights, K = 64 * chunks, `rows` of them a CTA (gated: a unit's 16), `depth` chunks to a ring stage.
@@ -1224,7 +1225,8 @@ SHRIKE_API int shrike_decode_step(const ShrikeStepArgs* in, cudaStream_t stream)
   config.dynamicSmemBytes = cuts.smem;
   config.stream = stream;
   cudaLaunchAttribute attribute;
-  attribute.id = cudaLaunchAttributeCooperative;   // all CTAs live at once, or none starts: they wait for one another
+  // all CTAs live at once, or none starts: they wait for one another (a process may be held to a part of the SMs)
+  attribute.id = cudaLaunchAttributeCooperative;
   attribute.val.cooperative = 1;
   config.attrs = &attribute;
   config.numAttrs = 1;
@@ -1234,6 +1236,10 @@ SHRIKE_API int shrike_decode_step(const ShrikeStepArgs* in, cudaStream_t stream)
     const int rc = shrike_raise_smem(raised, decode_step_kernel<D>, device.max_smem);           \
     if (rc != 0) return rc;                                                                     \
     const cudaError_t err = cudaLaunchKernelEx(&config, decode_step_kernel<D>, a);              \
+    if (err == cudaErrorCooperativeLaunchTooLarge || err == cudaErrorNotSupported) {            \
+      cudaGetLastError();                                                                       \
+      return NOT_TOGETHER;                                                                      \
+    }                                                                                           \
     if (err != cudaSuccess) return static_cast<int>(err);                                       \
     return shrike_launch_status();                                                              \
   }

@@ -171,9 +171,7 @@ class DecoderModel:
             self.pass_entry.begin(resid, ctx)   # it keeps what it needs of the embedding's output
         if self.residual is not None:
             resid = self.residual.begin(resid, ctx)   # the residual in its own form (several streams a token)
-        whole = self._whole_step is not None and self._whole_step.takes(ctx)
-        if whole:
-            resid = self._whole_step.run(resid, ctx)
+        whole = self._whole_step is not None and self._whole_step.takes(ctx) and self._whole_step.run(resid, ctx)
         for run in () if whole else self.config.order:
             if run.enter is not None:
                 resid, delta = self.pass_entry.forward(resid, delta, ctx, run.enter)

@@ -41,6 +41,7 @@ class StepArgs(_c.Structure):
 
 class DecodeStep:
     MAX_TOKENS = 8
+    NOT_TOGETHER = -2   # the launcher's answer where the device will not run all CTAs at once
 
     def __init__(self, ops, runtime, blocks, order):
         self.ops, self.runtime, self.blocks, self.order = ops, runtime, blocks, order
@@ -58,6 +59,7 @@ class DecodeStep:
         self._storage = None   # weakly: the pool the table's addresses belong to
         self._table = self._words = self._sync = None
         self._served: dict[int, bool] = {}
+        self._refused = False   # by the device, at a launch
 
     @classmethod
     def of(cls, ops, runtime, blocks, order):
@@ -103,7 +105,7 @@ class DecodeStep:
 
     def takes(self, ctx) -> bool:
         # keys of earlier positions are read while this step's are still being written: no entry may bring another's
-        return (ctx.all_single and ctx.apart and ctx.num_tokens <= self.MAX_TOKENS and getattr(self.ops, "whole_steps", False)
+        return (not self._refused and ctx.all_single and ctx.apart and ctx.num_tokens <= self.MAX_TOKENS and getattr(self.ops, "whole_steps", False)
                 and self._serves(ctx.num_tokens))
 
     def _tables(self, storage) -> None:
@@ -143,7 +145,8 @@ class DecodeStep:
             raise KernelError(f"decode_step: launcher returned {rc}")
 
     def run(self, resid, ctx):
-        """Runs the layers on `resid` [N, W] float32, in place: nothing is left pending."""
+        """Runs the layers on `resid` [N, W] float32, in place: nothing is left pending.  False where the device will not run the
+        kernel's CTAs together: nothing has run then, and no step is taken any more."""
         self._tables(ctx.storage)
         width, heads, kv_heads, dim, inter = self.sizes
         mixer = self.blocks[self.order[0].layer].mixer
@@ -157,6 +160,10 @@ class DecodeStep:
             sync=self._sync.data_ptr(), status=self.ops.status.data_ptr(), num_slots=keys.shape[0] * keys.shape[1],
             num_layers=len(self.order), tokens=ctx.num_tokens, width=width, heads=heads, kv_heads=kv_heads, head_dim=dim, inter=inter,
             max_blocks=view.max_blocks, page_size=keys.shape[1], num_pages=keys.shape[0], scale=mixer.spec.scale)
-        self._check(self.lib.shrike_decode_step(_c.byref(args), self.ops._stream()))
+        rc = self.lib.shrike_decode_step(_c.byref(args), self.ops._stream())
+        self._refused = rc == self.NOT_TOGETHER
+        if self._refused:
+            return False
+        self._check(rc)
         self.ops.launches += 1
-        return resid
+        return True

@@ -149,7 +149,7 @@ def test_entries_that_share_a_page_with_a_new_token_are_left_to_the_layers_one_b
     builder = BatchBuilder(4, groups, "cpu", None)
     step = object.__new__(DecodeStep)
     step.ops = SimpleNamespace(whole_steps=True)
-    step._served = {n: True for n in range(1, 9)}
+    step._served, step._refused = {n: True for n in range(1, 9)}, False
     a, b, c = held(manager, 12), held(manager, 9), held(manager, 12)
 
     def taken(*entries, pad_to=0):

@@ -132,3 +132,23 @@ def test_nothing_is_read_beyond_a_sequences_row_of_the_block_table():
             seen.append(logits[0].float().cpu().numpy().copy())
     runner.ops.check_status()
     assert np.isfinite(seen[0]).all() and np.array_equal(seen[0], seen[1])
+
+
+def test_where_the_device_will_not_run_all_ctas_together_the_layers_run_one_by_one():
+    raw, n = SHAPES["d64"], 40
+    ids = random_tokens(raw["vocab_size"], n + 1, 9)
+    seen = []
+    for refused in (False, True):
+        runner = runner_of(raw, 1)
+        program = runner.model._whole_step
+        if refused:
+            runner.ops.whole_steps = True
+            program.lib = type("Refuses", (), {"__getattr__": lambda _, name, real=program.lib: getattr(real, name),
+                                               "shrike_decode_step": staticmethod(lambda args, stream: program.NOT_TOGETHER)})()
+        else:
+            runner.ops.whole_steps = False
+        cache = opened(runner, ids, n)
+        for _ in range(3):   # eager, captured, replayed
+            seen.append(runner.step([StepEntry(cache, [ids[n]], n, [0])]).float().cpu().numpy().copy())
+        runner.ops.check_status()
+    assert all(np.array_equal(seen[0], other) for other in seen[1:])
