@@ -1064,11 +1064,10 @@ static bool cuts_of(int tokens, int layers, int width, int heads, int kv_heads, 
   if (!cut((heads + 2 * kv_heads) * dim, width, ctas, false, &p[0]) || !cut(width, q_width, ctas, false, &p[1]) ||
       !cut(2 * inter, width, ctas, true, &p[2]) || !cut(width, inter, ctas, false, &p[3]))
     return false;
-  // What a CTA reads of the others' words in a layer: beyond it the launches one by one are quicker.  Measured at 500 keys, us a
-  // step as launches and as one kernel: up to four sequences it wins to some 350 KB (width 2,048, 4 sequences, 340 KB: 1,873 and
-  // 1,739; 3,584, 2, 294 KB: 2,772 and 2,596; 3, 441 KB: 2,751 and 2,817); more take the norm two rounds of rows, and win to some
-  // 200 KB (896, 5, 190 KB: 820 and 687; 7, 266 KB: 840 and 884).  Longer contexts change it little (1,536, 1 sequence, 12,000 keys:
-  // 1,715 and 1,413).
+  // What a CTA reads of the others' words in a layer: beyond it the launches one by one are quicker.  Measured at 600 to 1,024
+  // keys, us a step as launches and as one kernel: up to four sequences it wins to some 350 KB (width 2,048, 3 sequences, 255 KB:
+  // 1,740 and 1,600; 4, 340 KB: 1,766 and 1,761; 3,584, 2, 294 KB: 2,712 and 2,620; 3, 441 KB, 500 keys: 2,751 and 2,817); more take
+  // the norm two rounds of rows, and win to some 200 KB (896, 5, 190 KB: 720 and 699; 7, 266 KB, 500 keys: 840 and 884).
   const long long read = 4LL * tokens * (4LL * width + q_width + inter);
   if (read > (tokens <= 4 ? 352 : 200) * 1024LL) return false;
   const int wide = width > q_width ? width : q_width;
@@ -1081,6 +1080,37 @@ static bool cuts_of(int tokens, int layers, int width, int heads, int kv_heads, 
   if (out->ring > MAX_SLOTS) out->ring = MAX_SLOTS;
   out->smem = fixed + static_cast<size_t>(out->ring) * SLOT;
   return true;
+}
+
+// The longest context with which a step that is served is at least as quick as the launches one by one: this kernel's attention
+// has one CTA an SM and two tiles of keys in it, the launches' two CTAs and three tiles.
+// In us a layer, fitted to both ways in turn at 100 to 32,000 keys, 1 to 8 sequences and 1 to 14 kv heads:
+//   here      2 for each tile of a run (64 keys of heads of 128, 128 of 64)
+//   launches  1.35 for each tile of 64 keys that one of two CTAs an SM walks, or, where pairs are few and their splits meet in
+//             global memory, 2.3 and up to 10 (7) for that
+//   the rest  what this kernel saves in products and norms: 11 or 12 less what is read of others' words
+// Measured, keys at which both are equal (and what this says), sequences in turn.  2 kv heads of 128: 1,536 wide, 1 to 4: 13,700
+// (12,300), 13,400 (11,900), 11,800 (11,400), 11,000 (11,500); 2,048 wide, 1 to 4: 13,000 (11,900), 12,800 (11,000), 11,900 (9,600),
+// 9,500 (10,200).  3,584 wide, 4 kv heads, 1 and 2: 11,000 (11,600), 12,000 (10,400).  1,536 wide, 12 kv heads, 1 to 4: 14,500 (16,400),
+// 3,000 (2,700), 1,500 (1,300), 200 (620).  896 wide, 2 kv heads of 64, 1, 2 and 5: 25,300 (23,400), 31,000 (30,000), 12,500 (14,200);
+// 14 kv heads, 1 to 4: 16,700 (18,100), 6,900 (7,700), 3,500 (3,300), 1,600 (1,500).  512 wide, 8 kv heads of 64, 5 and 8: 3,300
+// (3,200), 1,700 (1,700).  Beyond it the loss grows: 1,536 wide and 32,000 keys 1,601 us a step as launches and 2,412 here; 14
+// layers with 12 kv heads, 4 sequences of 16,384 keys 1,349 and 2,839.
+static int most_keys(int tokens, int width, int heads, int kv_heads, int dim, int inter) {
+  const int ctas = shrike_device().sm_count, pairs = tokens * kv_heads;
+  int runs = ctas / pairs;
+  runs = runs > MAX_SPLITS ? MAX_SPLITS : runs;
+  const bool narrow = dim == 64, few = pairs <= (narrow ? 10 : 16);
+  const double kilobytes = 4.0 * tokens * (4.0 * width + heads * dim + inter) / 1024;
+  const double here = 2.0 / (runs * (narrow ? 128 : 64));   // a key
+  const double launches = (few && tokens <= 4 ? 2.3 : 1.35) * pairs / (64.0 * 2 * ctas);
+  double ahead = tokens <= 4 ? 11.7 - 0.04 * kilobytes : 11 - 0.045 * kilobytes;
+  if (ahead < 0) ahead = 0;
+  if (!narrow) ahead += few ? 2 : 3;   // a run's first tile, which the shortest context has too
+  if (few) ahead += narrow ? 8 - 0.5 * pairs : (pairs < 6 ? 11 - 0.5 * pairs : 8);
+  constexpr int FAR = 65536;   // where the two grow alike (896 wide, 4 sequences): no further than twice what was measured
+  const double keys = here > launches ? ahead / (here - launches) : FAR;
+  return static_cast<int>(keys < FAR ? keys : FAR);
 }
 
 // A product's weights as ring stages: rows of 64 columns, `depth` of them side by side.
@@ -1151,6 +1181,12 @@ SHRIKE_API int shrike_decode_step_roles(int ctas, int width, int heads, int kv_h
                  (reads_residual(p, cta) ? 16 : 0);
   }
   return SHRIKE_OK;
+}
+// The longest context for which it is also the quicker way; 0 where it is not served.
+SHRIKE_API int shrike_decode_step_keys(int tokens, int layers, int width, int heads, int kv_heads, int head_dim, int inter) {
+  step::Cuts cuts;
+  if (!step::cuts_of(tokens, layers, width, heads, kv_heads, head_dim, inter, &cuts)) return 0;
+  return step::most_keys(tokens, width, heads, kv_heads, head_dim, inter);
 }
 SHRIKE_API int shrike_decode_step_layer_bytes() { return static_cast<int>(sizeof(step::Layer)); }
 // 64-bit words that the exchanges of a step of up to `tokens` tokens take.

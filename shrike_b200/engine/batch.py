@@ -91,6 +91,18 @@ class Staged:
     committed: bool = False
     apart: bool = False        # as StepContext.apart
 
+    @property
+    def all_single(self) -> bool:
+        return max(self.q_lens) == 1
+
+    @property
+    def num_tokens(self) -> int:
+        return self.n
+
+    @property
+    def max_ctx_len(self) -> int:
+        return max(self.ctx_lens)
+
 
 class BatchBuilder:
     """Packs entries into pinned host memory and copies them in one transfer."""
@@ -285,8 +297,8 @@ class BatchBuilder:
             token_ids=views[3], positions=views[4], seq_of_token=views[5], q_start=views[6],
             ctx_len=views[7], state_slot=views[8], seq_start=views[10], out_rows=views[9], groups=groups,
             storage=self.storage, max_q_len=max(staged.q_lens), min_q_len=min(staged.q_lens),
-            max_ctx_len=max(staged.ctx_lens), q_lens=staged.q_lens, starts=staged.starts, slots=staged.slots,
-            all_single=max(staged.q_lens) == 1, apart=staged.apart,
+            max_ctx_len=staged.max_ctx_len, q_lens=staged.q_lens, starts=staged.starts, slots=staged.slots,
+            all_single=staged.all_single, apart=staged.apart,
             sample_temperature=views[1].view(torch.float32) if sampled else None,
             sample_top_p=views[2].view(torch.float32) if sampled else None,
             sample_seed=views[0].view(torch.int64) if sampled else None,

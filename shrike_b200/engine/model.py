@@ -158,6 +158,10 @@ class DecoderModel:
             visit(part)
         return total
 
+    def one_kernel(self, step) -> bool:
+        """Whether all layers of a step run as one kernel."""
+        return self._whole_step is not None and self._whole_step.takes(step)
+
     def forward(self, ctx) -> torch.Tensor:
         """float32 logits [R, vocab] at `ctx.out_rows`."""
         ctx.carried.clear()   # nothing is carried from one forward pass to the next
@@ -171,7 +175,7 @@ class DecoderModel:
             self.pass_entry.begin(resid, ctx)   # it keeps what it needs of the embedding's output
         if self.residual is not None:
             resid = self.residual.begin(resid, ctx)   # the residual in its own form (several streams a token)
-        whole = self._whole_step is not None and self._whole_step.takes(ctx) and self._whole_step.run(resid, ctx)
+        whole = self.one_kernel(ctx) and self._whole_step.run(resid, ctx)
         for run in () if whole else self.config.order:
             if run.enter is not None:
                 resid, delta = self.pass_entry.forward(resid, delta, ctx, run.enter)

@@ -179,10 +179,10 @@ class ModelRunner:
         graphable = (self.use_graphs and self.device.type == "cuda" and self.capture_safe
                      and (decode or self.capture_portions))
         # what a captured launch sequence has baked in: the number of entries, every entry's
-        # length (grids and shapes follow from them), the number of wanted rows, the table widths, and whether the
-        # contexts, or entries that share pages, are of those for which other kernels run
-        contexts = self.ops.context_class(decode, max(staged.ctx_lens)) if hasattr(self.ops, "context_class") else 0
-        key = (staged.s if decode else tuple(staged.q_lens), staged.r, tuple(staged.max_blocks), sample, contexts, staged.apart)
+        # length (grids and shapes follow from them), the number of wanted rows, the table widths, whether the
+        # contexts are of those for which other kernels run, and whether all layers run as one kernel
+        contexts = self.ops.context_class(decode, staged.max_ctx_len) if hasattr(self.ops, "context_class") else 0
+        key = (staged.s if decode else tuple(staged.q_lens), staged.r, tuple(staged.max_blocks), sample, contexts, self.model.one_kernel(staged))
         return Prepared(staged, sample, graphable, key, decode)
 
     def fetch(self, tokens: torch.Tensor):

@@ -46,11 +46,11 @@ class DecodeStep:
     def __init__(self, ops, runtime, blocks, order):
         self.ops, self.runtime, self.blocks, self.order = ops, runtime, blocks, order
         self.lib = build.decode_step_library()
-        self.lib.shrike_decode_step_serves.argtypes = [_I] * 7
+        self.lib.shrike_decode_step_keys.argtypes = [_I] * 7
         self.lib.shrike_decode_step_words.argtypes = [_I] * 6
         self.lib.shrike_decode_step_table.argtypes = [_P, _I, _I, _I, _I, _I, _I, _P]
         self.lib.shrike_decode_step.argtypes = [_P, _P]
-        for name in ("serves", "table", "layer_bytes"):
+        for name in ("keys", "table", "layer_bytes"):
             getattr(self.lib, f"shrike_decode_step_{name}").restype = _I
         self.lib.shrike_decode_step_words.restype = _LL
         self.lib.shrike_decode_step.restype = _I
@@ -58,7 +58,7 @@ class DecodeStep:
         self.sizes = (mixer.width, mixer.num_heads, mixer.num_kv_heads, mixer.head_dim, ffn.intermediate)
         self._storage = None   # weakly: the pool the table's addresses belong to
         self._table = self._words = self._sync = None
-        self._served: dict[int, bool] = {}
+        self._most_keys: dict[int, int] = {}   # sequences -> the longest context served
         self._refused = False   # by the device, at a launch
 
     @classmethod
@@ -95,18 +95,20 @@ class DecodeStep:
         if any((t is None) != (first is None) or (t is not None and t is not first and not torch.equal(t, first)) for t in turns):
             return None
         program = cls(ops, runtime, blocks, order)
-        return program if program._serves(1) else None
+        return program if program.most_keys(1) > 0 else None
 
-    def _serves(self, tokens: int) -> bool:
-        held = self._served.get(tokens)
+    def most_keys(self, tokens: int) -> int:
+        """The longest context of a step of `tokens` sequences that is served (0: none)."""
+        held = self._most_keys.get(tokens)
         if held is None:
-            held = self._served[tokens] = bool(self.lib.shrike_decode_step_serves(tokens, len(self.order), *self.sizes))
+            held = self._most_keys[tokens] = self.lib.shrike_decode_step_keys(tokens, len(self.order), *self.sizes)
         return held
 
-    def takes(self, ctx) -> bool:
+    def takes(self, step) -> bool:
+        """Whether a step is run here; `step` is a `StepContext`, or a `Staged` step whose captured form is looked for."""
         # keys of earlier positions are read while this step's are still being written: no entry may bring another's
-        return (not self._refused and ctx.all_single and ctx.apart and ctx.num_tokens <= self.MAX_TOKENS and getattr(self.ops, "whole_steps", False)
-                and self._serves(ctx.num_tokens))
+        return (not self._refused and step.all_single and step.apart and step.num_tokens <= self.MAX_TOKENS
+                and getattr(self.ops, "whole_steps", False) and step.max_ctx_len <= self.most_keys(step.num_tokens))
 
     def _tables(self, storage) -> None:
         """The layers' addresses on the device, written once per cache pool."""

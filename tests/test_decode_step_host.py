@@ -149,12 +149,13 @@ def test_entries_that_share_a_page_with_a_new_token_are_left_to_the_layers_one_b
     builder = BatchBuilder(4, groups, "cpu", None)
     step = object.__new__(DecodeStep)
     step.ops = SimpleNamespace(whole_steps=True)
-    step._served, step._refused = {n: True for n in range(1, 9)}, False
+    step._most_keys, step._refused = {n: 1000 for n in range(1, 9)}, False
     a, b, c = held(manager, 12), held(manager, 9), held(manager, 12)
 
     def taken(*entries, pad_to=0):
         staged = builder.stage([StepEntry(cache, [1] * count, start, [0]) for cache, start, count in entries], pad_to=pad_to)
-        return step.takes(builder.context(staged))
+        assert step.takes(staged) == step.takes(builder.context(staged))   # what a captured step goes by, and the step
+        return step.takes(staged)
 
     assert taken((a, 11, 1)) and taken((a, 11, 1), (b, 8, 1), (c, 11, 1)) and taken((a, 11, 1), (b, 8, 1), pad_to=8)
     assert not taken((a, 10, 1), (a, 11, 1))                    # neighbours on one page
@@ -169,3 +170,31 @@ def test_entries_that_share_a_page_with_a_new_token_are_left_to_the_layers_one_b
     many = [(held(manager, 1), 0, 1) for _ in range(9)]
     assert taken(*many[:8]) and not taken(*many)
     assert torch.equal(builder.build([StepEntry(a, [1], 11, [0])]).ctx_len, torch.tensor([12], dtype=torch.int32))
+
+
+def test_the_longest_context_a_step_is_served_with_follows_the_sizes():
+    """Within a quarter of where the two ways were measured to be equal (at 148 SMs), fewer keys with more sequences where kv heads
+    are many, and none where the sizes themselves are not served."""
+    keys = build.decode_step_library().shrike_decode_step_keys
+    for sizes, measured in ((WIDTHS["1.5b"], {1: 13700, 2: 13400, 3: 11800, 4: 11000}), (WIDTHS["3b"], {1: 13000, 2: 12800, 3: 11900, 4: 9500}),
+                            (WIDTHS["7b"], {1: 11000, 2: 12000}), (WIDTHS["0.5b"], {1: 25300, 2: 31000}),
+                            ((896, 14, 14, 64, 4864), {1: 16700, 2: 6900, 3: 3460, 4: 1580}), ((512, 8, 8, 64, 1280), {5: 3260, 8: 1720}),
+                            ((1536, 12, 12, 128, 8960), {1: 14500, 2: 3050, 3: 1480})):
+        for tokens, equal in measured.items():
+            assert 0.75 * equal <= keys(tokens, 28, *sizes) <= 1.15 * equal, (sizes, tokens, keys(tokens, 28, *sizes))
+    for heads in (6, 12):
+        line = [keys(tokens, 28, 1536, 12, heads, 128, 8960) for tokens in (1, 2, 3, 4)]
+        assert line == sorted(line, reverse=True) and 4 * line[3] < line[0], line
+    assert all(0 <= keys(tokens, 2, width, heads, heads, 64, 1280) <= 65536 for tokens in range(1, 9)
+               for width, heads in ((256, 4), (384, 6), (512, 2)))
+    assert keys(5, 28, *WIDTHS["1.5b"]) == keys(3, 28, *WIDTHS["7b"]) == keys(9, 24, *WIDTHS["0.5b"]) == keys(1, 200, *WIDTHS["0.5b"]) == 0
+
+
+def test_a_context_beyond_that_is_left_to_the_layers_one_by_one():
+    manager = CacheManager([KVGroupSpec((0,), 2, 64, None)], 4, 64, 16)
+    builder = BatchBuilder(4, 1, "cpu", None)
+    step = object.__new__(DecodeStep)
+    step.ops, step._refused, step._most_keys = SimpleNamespace(whole_steps=True), False, {1: 30, 2: 20}
+    a, b = held(manager, 40), held(manager, 9)
+    taken = lambda *starts: step.takes(builder.stage([StepEntry(c, [1], start, [0]) for c, start in zip((a, b), starts)]))
+    assert taken(29) and not taken(30) and taken(19, 8) and not taken(20, 8)
