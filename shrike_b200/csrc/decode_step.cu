@@ -70,7 +70,10 @@ constexpr int MAX_TOKENS = 8;
 constexpr int MAX_SPLITS = 16;                 // runs of a pair's keys
 constexpr int MAX_ROWS = 32;                   // weight rows of a CTA in a product
 constexpr int MAX_LAYERS = 96;
-constexpr unsigned POLL_LIMIT = 4000000u;      // looks at a word before it is given up: seconds
+#ifndef SHRIKE_STEP_POLL_LIMIT
+#define SHRIKE_STEP_POLL_LIMIT 4000000u
+#endif
+constexpr unsigned POLL_LIMIT = SHRIKE_STEP_POLL_LIMIT;   // looks at a word before it is given up: seconds
 
 constexpr int NOT_TOGETHER = -2;   // the launcher's answer where the device will not run all CTAs at once: nothing has run
 enum : int { ERR_PRODUCER = 51, ERR_STAGE = 52, ERR_WORD = 53, ERR_DRAIN = 54 };
@@ -278,7 +281,7 @@ __device__ __forceinline__ void stream_weights(const Args& a, Shared* sh, unsign
       }
     }
   }
-  if (!FETCH && !ok) {   // copies may still be in flight: wait for them before leaving
+  if (!FETCH) {   // where a wait ran out, here or later in the other warps, nobody waits for the copies still in flight: not to leave before
     const int left = stage < a.ring ? stage : a.ring;
 #pragma unroll 1
     for (int i = 0; i < left; ++i) {

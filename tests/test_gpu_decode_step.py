@@ -1,5 +1,7 @@
 """All layers of a decode step as one kernel, against the layer-by-layer path and the plain implementation."""
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -7,6 +9,8 @@ import torch
 from shrike_b200.config import parse_config
 from shrike_b200.engine.batch import StepEntry
 from shrike_b200.engine.runner import ModelRunner
+from shrike_b200.ops import build
+from shrike_b200.ops.cuda_ops import KernelError
 from shrike_b200.weights.random_init import random_tensors
 from tests.gpu_common import TOL, cuda_ops
 from tests.helpers import random_tokens
@@ -152,3 +156,36 @@ def test_where_the_device_will_not_run_all_ctas_together_the_layers_run_one_by_o
             seen.append(runner.step([StepEntry(cache, [ids[n]], n, [0])]).float().cpu().numpy().copy())
         runner.ops.check_status()
     assert all(np.array_equal(seen[0], other) for other in seen[1:])
+
+
+def test_a_wait_that_runs_out_ends_the_step_with_its_code_and_the_next_step_is_right():
+    """A build whose waits for other CTAs' words give up at the first look that finds them missing: the kernel runs to its end,
+    says so in the status word, and leaves the exchanges fit for the next launch."""
+    raw, n = SHAPES["d64"], 300
+    ids = random_tokens(raw["vocab_size"], n + 1, 9)
+    runner = runner_of(raw, 1)
+    runner.use_graphs = False
+    program = runner.model._whole_step
+    cache = opened(runner, ids, n)
+    patient, impatient = program.lib, build.load_library("shrike_decode_step_impatient", ["decode_step.cu"], {"SHRIKE_STEP_POLL_LIMIT": 1})
+    impatient.shrike_decode_step.argtypes, impatient.shrike_decode_step.restype = patient.shrike_decode_step.argtypes, ctypes.c_int
+
+    class Impatient:
+        shrike_decode_step = staticmethod(impatient.shrike_decode_step)
+
+        def __getattr__(self, name):
+            return getattr(patient, name)
+
+    def step():
+        return runner.step([StepEntry(cache, [ids[n]], n, [0])]).float().cpu().numpy().copy()
+
+    want = step()
+    runner.ops.check_status()
+    for _ in range(2):
+        program.lib = Impatient()
+        step()
+        with pytest.raises(KernelError, match="wait for another CTA's values ran out"):
+            runner.ops.check_status()
+        program.lib = patient
+        assert np.array_equal(step(), want)
+        runner.ops.check_status()
