@@ -189,3 +189,70 @@ def test_a_wait_that_runs_out_ends_the_step_with_its_code_and_the_next_step_is_r
         program.lib = patient
         assert np.array_equal(step(), want)
         runner.ops.check_status()
+
+
+def follow(raw, seed, whole, script, lengths):
+    """Logits of a script's steps on one runner, and the launches of each.  A step is a list of (request, its count of tokens);
+    None: the cache pool is replaced by a copy."""
+    config = parse_config(raw)
+    weights = {k: (v.to(torch.bfloat16) if v.dim() >= 2 else v) for k, v in random_tensors(config, seed, "cuda", torch.float32).items()}
+    ops = cuda_ops(torch.bfloat16)
+    room = [n + 200 for n in lengths]
+    runner = ModelRunner(config, weights, ops, "cuda", "bfloat16", page_size=16, num_pages=sum(-(-n // 16) for n in room), max_slots=len(lengths))
+    ids = [random_tokens(raw["vocab_size"], n, 70 + i) for i, n in enumerate(room)]
+    ops.whole_steps = whole
+    caches, at, rows, launches = [], list(lengths), [], []
+    for i, n in enumerate(lengths):
+        caches.append(runner.cache.open())
+        runner.cache.append(caches[i], 0, room[i])
+        runner.step([StepEntry(caches[i], ids[i][:n], 0, [])])
+    for step in script:
+        if step is None:
+            held = runner.storage
+            pages = [group.shape[2] for group in held.kv]
+            runner.storage = runner.builder.storage = type(held)(held.groups, 16, pages, {}, len(lengths), torch.bfloat16, runner.device)
+            for new, old in zip(runner.storage.kv, held.kv):
+                new.copy_(old)
+                old.fill_(float("nan"))
+            runner._graphs.clear()   # a captured step belongs to the pool it was captured with
+            continue
+        before = ops.launches
+        out = runner.step([StepEntry(caches[i], ids[i][at[i]: at[i] + count], at[i], [count - 1]) for i, count in step])
+        launches.append(ops.launches - before)
+        rows.append(out.float().cpu().numpy().copy())
+        for i, count in step:
+            at[i] += count
+    ops.check_status()
+    return rows, launches
+
+
+def singles(*requests):
+    return [(i, 1) for i in requests]
+
+
+@pytest.mark.parametrize("seed", [3, 4])   # the second engine of a process finds what the first has freed
+def test_steps_of_different_counts_and_kinds_in_one_engine(seed):
+    """The words that CTAs exchange lie elsewhere for every count of sequences, and the numbers in them go on through captured
+    launches, prompts, steps that the layers take one by one and a new cache pool."""
+    raw, lengths = SHAPES["d64"], (40, 333, 90, 1, 700, 128, 127, 64, 500, 12)
+    script = [singles(0)] * 3 + [singles(0, 1, 2, 3)] * 3 + [singles(2, 3)] * 2 + [[(4, 70), (0, 1), (1, 1)]]
+    script += [singles(*range(9))] * 2 + [singles(0, 1, 2, 3), singles(5), singles(8, 9, 0), singles(4, 5, 6, 7, 8)] * 2
+    script += [singles(6), None] + [singles(0), singles(3, 2, 1, 0), singles(4, 9)] * 3 + [[(7, 33)], singles(7), singles(4)]
+    got, launches = follow(raw, seed, True, script, lengths)
+    want, _ = follow(raw, seed, False, script, lengths)
+    steps = [step for step in script if step is not None]
+    for step, a, b, count in zip(steps, got, want, launches):
+        assert np.isfinite(a).all() and np.abs(a - b).max() <= TOL["bfloat16"] * max(1.0, float(np.abs(b).max())), step
+        assert (count < 6) == (len(step) <= 5 and max(n for _, n in step) == 1), (step, count)
+
+
+@pytest.mark.parametrize("lengths", [(9000,), (20000, 130), (3, 12000, 700, 64)])
+def test_long_contexts(lengths):
+    """Runs of many tiles of keys, up to the contexts that are left to the layers one by one."""
+    raw = SHAPES["d64"]
+    script = [singles(*range(len(lengths)))] * 3
+    got, launches = follow(raw, 3, True, script, lengths)
+    want, _ = follow(raw, 3, False, script, lengths)
+    assert max(launches) < 6
+    for a, b in zip(got, want):
+        assert np.isfinite(a).all() and np.abs(a - b).max() <= TOL["bfloat16"] * max(1.0, float(np.abs(b).max()))
