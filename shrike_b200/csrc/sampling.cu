@@ -178,12 +178,12 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
 // the bisection's lower end can never count again and is dropped from its thread's list, in place, now and then.  The sums are those of one block of 1,024 threads that walk the row with a
 // stride of 1,024, to the bit: thread t of CTA r is that block's thread 128 r + t, dropped entries add nothing, and the 32
 // warps' sums meet in one warp in the same order.
-// Two CTAs fill an SM's shared memory, so the time is that of their few warps: HELP threads share what a place's entries cost
-// one by one (copies, exponentials, the draw's noise).
-// Measured (one B200): 64 rows of 152,064 logits with top_p 0.95: 180 us (220 with one thread a place and the row read
-// through registers, 191 with four, which also slow rows of a few thousand down: 64 rows of 5,000 47 and 73), one row 69 (90);
-// and 1,391 with a block a row that reads the row from memory thirty times.
-constexpr int ROW_CTAS = 8, ROW_THREADS = SAMPLE_THREADS / ROW_CTAS, HELP = 2;
+// HELP threads share what a place's entries cost one by one (copies, exponentials, the draw's noise), one or two.  Where two
+// CTAs fill an SM's shared memory, or rows are few, the time is that of their few warps, and two threads pay; where an SM holds
+// many CTAs the second thread only takes another CTA's place.  Measured (one B200, top_p 0.95), us with one and two threads a
+// place: 64 rows of 152,064 logits 177 and 148, one row 72 and 58; 64 rows of 5,000 39 and 46, 128 rows of 12,000 58 and 89; and
+// 1,391 for the first with a block a row that reads the row from memory thirty times.  Four threads: 191 where two took 180.
+constexpr int ROW_CTAS = 8, ROW_THREADS = SAMPLE_THREADS / ROW_CTAS;
 
 struct RowShare {
   float warps[2][4][32];   // up to four values per warp of the cluster, two buffers: one barrier a sum
@@ -193,6 +193,7 @@ struct RowShare {
 // Every HELP-th of the row's entries x[0], x[SAMPLE_THREADS], ... that belong to a place, from the `which`-th on, into
 // shared memory.  All copies are under way together: read through registers, eight at a time and eight warps an SM, a row
 // came at a sixth of the memory's rate.
+template <int HELP>
 __device__ __forceinline__ void fetch_entries(float* place, const float* x, int which, int count) {
   const unsigned to = static_cast<unsigned>(__cvta_generic_to_shared(place));
 #pragma unroll 4
@@ -215,6 +216,7 @@ __device__ __forceinline__ void row_publish(float4 mine, RowShare& share, int bu
   cluster.sync();
 }
 
+template <int HELP>
 __global__ void __launch_bounds__(ROW_THREADS * HELP)
 sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
                       const float* __restrict__ top_p, const long long* __restrict__ seeds, int* __restrict__ out,
@@ -250,7 +252,7 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
   int count = which == 0 ? all : 0;
   const float inv_temp = 1.0f / temp;
   float local_max = -INFINITY;
-  fetch_entries(own, x + first, which, all);
+  fetch_entries<HELP>(own, x + first, which, all);
   __syncthreads();
 #pragma unroll 8
   for (int j = 0; j < count; ++j) local_max = fmaxf(local_max, own[j * ROW_THREADS]);
@@ -323,7 +325,7 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
   Best mine{-INFINITY, 0x7fffffff};
   const unsigned long long seed = static_cast<unsigned long long>(seeds[row]);
   __syncthreads();   // the logits once more, over what the bisection left of their probabilities
-  fetch_entries(own, x + first, which, all);
+  fetch_entries<HELP>(own, x + first, which, all);
 #pragma unroll 4
   for (int j = which; j < all; j += HELP) {
     const int i = first + j * SAMPLE_THREADS;
@@ -357,16 +359,24 @@ int launch_sample(const float* logits, const float* temperature, const float* to
   constexpr size_t MOST = 200 * 1024;
   // The cluster form costs 0.3 us a cluster to start, whatever a row holds; a block a row costs a scan of the row at every step of
   // the bisection.  Measured, us with clusters and with blocks: 1,000 tokens 20 and 19 (1 row), 37 and 23 (64), 96 and 29 (256);
-  // 2,000 tokens 22 and 23 (8), 30 and 23 (32); 5,000 tokens 40 and 52 (64), 54 and 57 (128), 103 and 59 (256); 12,000 tokens 109
-  // and 112 (256), 206 and 217 (512); 152,000 tokens 183 and 1,117 (64).  Both give the same tokens.
+  // 2,000 tokens 22 and 23 (8), 30 and 23 (32); 5,000 tokens 39 and 52 (64), 53 and 57 (128), 103 and 59 (256); 12,000 tokens 107
+  // and 112 (256), 206 and 217 (512); 152,000 tokens 148 and 1,117 (64).  Both give the same tokens.
   const bool clusters = vocab >= 12000 || (vocab >= 4096 && rows <= 128) || (vocab >= 1536 && rows <= 8);
   if (clusters && smem <= MOST) {
-    static PerDevice raised;
-    const int rc = shrike_raise_smem(raised, sample_cluster_kernel, MOST);
-    if (rc != 0) return rc;
-    err = launch_dependent_clusters(sample_cluster_kernel, dim3(rows * ROW_CTAS), dim3(ROW_THREADS * HELP), smem, stream, ROW_CTAS, logits,
-                                    temperature, top_p, seeds, out, static_cast<const float*>(scratch_value),
-                                    static_cast<const int*>(scratch_index), vocab, chunks, status);
+    auto launch = [&](auto kernel, int help, PerDevice& raised) {
+      const int rc = shrike_raise_smem(raised, kernel, MOST);
+      if (rc != 0) return static_cast<cudaError_t>(rc);
+      return launch_dependent_clusters(kernel, dim3(rows * ROW_CTAS), dim3(ROW_THREADS * help), smem, stream, ROW_CTAS, logits, temperature,
+                                       top_p, seeds, out, static_cast<const float*>(scratch_value),
+                                       static_cast<const int*>(scratch_index), vocab, chunks, status);
+    };
+    // Two threads a place (above) for few rows, or for rows that leave an SM few CTAs.  Measured, us with one and two: 4,096 tokens
+    // 24 and 25 (16 rows), 51 and 79 (128); 8,000 25 and 24 (12), 39 and 46 (64); 20,000 30 and 28 (12), 38 and 41 (24), 61 and 85
+    // (128); 32,000 49 and 40 (24), 70 and 64 (64), 72 and 93 (128); 64,000 68 and 68 (64), 160 and 171 (192); 100,000 90 and 91
+    // (64), 321 and 311 (256).
+    const bool pairs = vocab >= 90000 || (vocab >= 30000 && rows <= 64) || (vocab >= 6000 && rows <= 12);
+    static PerDevice raised_alone, raised_pairs;
+    err = pairs ? launch(sample_cluster_kernel<2>, 2, raised_pairs) : launch(sample_cluster_kernel<1>, 1, raised_alone);
   } else {
     err = launch_dependent(sample_kernel, rows, SAMPLE_THREADS, 0, stream, logits, temperature, top_p, seeds, out,
                            static_cast<const float*>(scratch_value), static_cast<const int*>(scratch_index), vocab, chunks, status);

@@ -83,3 +83,9 @@ def test_nucleus_sampling_by_a_cluster_or_a_block_draws_the_same_token(vocab, si
         mine = probs[: len(out)].gather(1, out.long()[:, None])
         above = torch.where(probs[: len(out)] > mine, probs[: len(out)], torch.zeros((), dtype=torch.float64, device=DEV)).sum(1)
         assert (above < top_p[: len(out)].double() + 1e-5).all()
+
+
+# around those from which two threads share a place's entries
+@pytest.mark.parametrize("vocab,sizes", [(5999, (12, 13)), (6000, (12, 13)), (29999, (12, 13, 64)), (30000, (1, 64, 65)), (89999, (64, 65)), (90000, (12, 65))])
+def test_nucleus_sampling_by_one_or_two_threads_a_place_draws_the_same_token(vocab, sizes):
+    test_nucleus_sampling_by_a_cluster_or_a_block_draws_the_same_token(vocab, sizes)
