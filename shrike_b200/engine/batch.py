@@ -19,7 +19,7 @@ import numpy as np
 import torch
 
 
-FEW_ENTRIES = 8    # up to so many single tokens a batch knows whether its entries keep out of one another's pages
+FEW_ENTRIES = 8    # up to so many single tokens a batch may tell whether its entries keep out of one another's pages
 FIRST_GROUP = 11   # index of the first per-group part of the packed block (see BatchBuilder.stage)
 
 
@@ -61,7 +61,7 @@ class StepContext:
     starts: list[int]
     slots: list[int]  # host copy of state_slot
     all_single: bool = False  # every entry brings exactly one token
-    apart: bool = False  # up to FEW_ENTRIES single tokens, none of which goes to a page that another entry holds
+    apart: bool = False  # up to FEW_ENTRIES single tokens, of which each is known to go to a page that no other entry holds
     sample_temperature: torch.Tensor | None = None  # float32 [R], when every wanted row is sampled
     sample_top_p: torch.Tensor | None = None  # float32 [R]
     sample_seed: torch.Tensor | None = None  # int64 [R]
@@ -117,6 +117,7 @@ class BatchBuilder:
         self._turn = 0
         self._dev = None
         self._range = None
+        self.watches_pages = False   # whether batches of two and more tell if their entries keep apart (some microseconds a step)
         self.generation = 0  # grows when the device buffer moves: captured launch sequences are stale then
         self.copied_bytes = 0  # host-to-device bytes of all steps so far
 
@@ -202,7 +203,7 @@ class BatchBuilder:
 
         apart = False
         if max(q_lens) == 1:
-            apart = s <= FEW_ENTRIES
+            apart = s == 1 or (self.watches_pages and s <= FEW_ENTRIES)
             # the steady state of decoding: one token per entry, filled without per-token work
             ids[:real] = [e.tokens[0] for e in entries]
             pos[:real] = starts

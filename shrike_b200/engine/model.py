@@ -158,6 +158,11 @@ class DecoderModel:
             visit(part)
         return total
 
+    @property
+    def has_one_kernel(self) -> bool:
+        """Whether there are steps whose layers run as one kernel."""
+        return self._whole_step is not None
+
     def one_kernel(self, step) -> bool:
         """Whether all layers of a step run as one kernel."""
         return self._whole_step is not None and self._whole_step.takes(step)

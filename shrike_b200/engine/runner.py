@@ -86,6 +86,7 @@ class ModelRunner:
             self.groups, page_size, num_pages, state_needs, max_slots, self.dtype, self.device
         )
         self.builder = BatchBuilder(page_size, len(self.groups), self.device, self.storage)
+        self.builder.watches_pages = self.model.has_one_kernel
         self.use_graphs = True
         # steps are recorded as CUDA graphs (decode batches at once, batches with portions once their
         # shape repeats) only if every part says that its forward() depends on the batch's shape alone

@@ -147,6 +147,7 @@ def test_entries_that_share_a_page_with_a_new_token_are_left_to_the_layers_one_b
     """Such an entry may read the key that another of the same step stores: the layers one by one store all keys first."""
     manager = CacheManager([KVGroupSpec((g,), 2, 64, None) for g in range(groups)], 4, 64, 16)
     builder = BatchBuilder(4, groups, "cpu", None)
+    builder.watches_pages = True
     step = object.__new__(DecodeStep)
     step.ops = SimpleNamespace(whole_steps=True)
     step._most_keys, step._refused = {n: 1000 for n in range(1, 9)}, False
@@ -167,6 +168,9 @@ def test_entries_that_share_a_page_with_a_new_token_are_left_to_the_layers_one_b
     for table, other in zip(shared.tables, a.tables):
         table.pages[0] = other.pages[0]
     assert taken((a, 11, 1), (shared, 3, 1)) is False and taken((b, 8, 1), (shared, 3, 1))
+    builder.watches_pages = False                               # a runner asks only where it matters
+    assert taken((a, 11, 1)) and not taken((a, 11, 1), (b, 8, 1))
+    builder.watches_pages = True
     many = [(held(manager, 1), 0, 1) for _ in range(9)]
     assert taken(*many[:8]) and not taken(*many)
     assert torch.equal(builder.build([StepEntry(a, [1], 11, [0])]).ctx_len, torch.tensor([12], dtype=torch.int32))
@@ -193,6 +197,7 @@ def test_the_longest_context_a_step_is_served_with_follows_the_sizes():
 def test_a_context_beyond_that_is_left_to_the_layers_one_by_one():
     manager = CacheManager([KVGroupSpec((0,), 2, 64, None)], 4, 64, 16)
     builder = BatchBuilder(4, 1, "cpu", None)
+    builder.watches_pages = True
     step = object.__new__(DecodeStep)
     step.ops, step._refused, step._most_keys = SimpleNamespace(whole_steps=True), False, {1: 30, 2: 20}
     a, b = held(manager, 40), held(manager, 9)
