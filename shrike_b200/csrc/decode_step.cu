@@ -7,9 +7,10 @@
 // CTA's share of all weights, layer after layer, through a ring in shared memory and runs ahead of the arithmetic by the depth
 // of that ring (it needs nothing but the layer table), so that HBM keeps busy while the other warps wait for one another.
 //
-// Measured (500 keys, us a step as separate launches and as one kernel): 0.5B widths 1 sequence 766 and 446, 4 sequences 799
-// and 536; 1.5B 1,159 and 772, 1,176 and 1,051; 3B 1,770 and 1,332; 7B 2,727 and 2,513.  A layer takes 13 us at 0.5B widths (the
-// five exchanges 0.7 each, attention 2.3, gated and down products 2.6 and 3.2) and 24 at 1.5B.
+// Measured (500 keys, us a step as separate launches and as one kernel, in turn): 0.5B widths 1 sequence 654 and 440, 4 sequences
+// 670 and 533; 1.5B 1,058 and 773, 1,099 and 1,055; 3B 1,673 and 1,332; 7B 2,694 and 2,538.  A layer takes 14.8 us at 0.5B widths
+// and 23.5 at 1.5B (12 against 24 layers, 14 against 28); one of 256 columns, which has next to no weights, 13.2: that is what the
+// five exchanges, the norms and the attention take by themselves.
 //
 // A layer:  norm + q/k/v product | rotation, store, attention | output product + residual | norm + gate/up product +
 // activation | down product + residual.  A product gives every CTA the same number of weight rows (the gated one units of 8 gate rows
@@ -56,7 +57,8 @@ typedef unsigned long long Word;               // a value below, the exchange's 
 constexpr int WARPS = 8;                       // warps that compute
 constexpr int COMPUTE = WARPS * 32;
 // The ninth streams weights, the tenth fetches to L2; two more, idle, make them a warpgroup, whose registers go to the computing
-// ones: what these held beyond 168 registers lay in local memory (657 us a step of the 0.5B widths with such spills, 546 without).
+// ones: what these held beyond 168 registers lay in local memory (0.5B widths, in an early
+// state of this kernel: 657 us a step with such spills, 546 without).
 constexpr int THREADS = COMPUTE + 128;
 constexpr int COMPUTE_REGISTERS = 232, STREAM_REGISTERS = 40;
 static_assert(COMPUTE * COMPUTE_REGISTERS + 128 * STREAM_REGISTERS <= THREADS * 168, "no more than the launch brings");
@@ -1069,8 +1071,8 @@ static bool cuts_of(int tokens, int layers, int width, int heads, int kv_heads, 
     return false;
   // What a CTA reads of the others' words in a layer: beyond it the launches one by one are quicker.  Measured at 600 to 1,024
   // keys, us a step as launches and as one kernel: up to four sequences it wins to some 350 KB (width 2,048, 3 sequences, 255 KB:
-  // 1,740 and 1,600; 4, 340 KB: 1,766 and 1,761; 3,584, 2, 294 KB: 2,712 and 2,620; 3, 441 KB, 500 keys: 2,751 and 2,817); more take
-  // the norm two rounds of rows, and win to some 200 KB (896, 5, 190 KB: 720 and 699; 7, 266 KB, 500 keys: 840 and 884).
+  // 1,740 and 1,600; 4, 340 KB: 1,766 and 1,761, at 100 keys 1,711 and 1,733; 3,584, 2, 294 KB: 2,712 and 2,620; 3, 441 KB, 500 keys: 2,751 and 2,817); more take
+  // the norm two rounds of rows, and win to some 200 KB (896, 5, 190 KB: 704 and 699, at 500 keys 673 and 693; 7, 266 KB, 500 keys: 840 and 884).
   const long long read = 4LL * tokens * (4LL * width + q_width + inter);
   if (read > (tokens <= 4 ? 352 : 200) * 1024LL) return false;
   const int wide = width > q_width ? width : q_width;

@@ -254,7 +254,10 @@ gemm_swap_ab_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // shared memory is then its ring (below), ten times at most.  So many CTAs with deep rings read about as fast as twice
 // as many with half of it each, and what consumes the product has fewer runs to add (us, 8 tokens, two an SM | one an SM:
 // 5,120 x 5,120 in 7 | 3 runs 9.8 | 10.3, 2,048 x 11,008 in 16 | 9 8.9 | 8.6, 6,144 x 4,096 in 6 | 3 9.5 | 9.6; 43 tokens,
-// 896 x 4,864 in 16 | 10 | 8 4.7 | 4.3 | 4.5).
+// 896 x 4,864 in 16 | 10 | 8 4.7 | 4.3 | 4.5).  With the norm that adds the runs behind it, 8 tokens: 4,096 x 4,096 in 8 | 4 runs
+// 9.7 | 9.1, 3,584 x 3,584 in 8 | 5 8.0 | 7.3, 1,024 x 4,096 in 16 | 10 6.0 | 5.0, 9,216 x 4,608 in 4 | 2 26.5 | 24.6; the other way
+// 6,144 x 4,096 in 6 | 3 12.7 | 13.1, 5,120 x 5,120 in 7 | 3 12.4 | 12.9, 2,560 x 2,560 in 8 | 7 5.8 | 6.4, and at 40 tokens 2,560 x 2,048
+// in 8 | 7 6.6 | 7.4.  Steps of 3 to 64 tokens at widths of 2,048 to 5,120 are 2 to 15% quicker by this line with these rings.
 // Long runs (beyond 40 k-blocks), and tiles that would leave more than a quarter of the SMs without a CTA (75 to 110
 // tiles; 50 to 55 in two runs): the most runs, eight at most (sixteen where eight would not give every SM a
 // CTA), that keep two CTAs an SM resident together; the time jumps by a third where the grid exceeds that
