@@ -256,3 +256,16 @@ def test_long_contexts(lengths):
     assert max(launches) < 6
     for a, b in zip(got, want):
         assert np.isfinite(a).all() and np.abs(a - b).max() <= TOL["bfloat16"] * max(1.0, float(np.abs(b).max()))
+
+
+def test_a_batch_that_grows_beyond_the_longest_context_goes_on_layer_by_layer():
+    """Eight kv heads, eight sequences: the line lies low.  Captured launches of one way are not replayed for the other."""
+    raw = shape(512, 8, 8, 64, 1280)
+    line = build.decode_step_library().shrike_decode_step_keys(8, 2, 512, 8, 8, 64, 1280)
+    lengths = (line - 4, 300, 20, 1, 130, 64, 800, 500)
+    script = [singles(*range(8))] * 8
+    got, launches = follow(raw, 3, True, script, lengths)
+    want, _ = follow(raw, 3, False, script, lengths)
+    assert 500 < line < 5000 and [count < 6 for count in launches] == [True] * 4 + [False] * 4
+    for a, b in zip(got, want):
+        assert np.isfinite(a).all() and np.abs(a - b).max() <= TOL["bfloat16"] * max(1.0, float(np.abs(b).max()))
